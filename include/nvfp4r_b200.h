@@ -198,6 +198,25 @@ NVFP4R_API int nvfp4r_linear_packed(const void* x, int64_t x_row_stride, int M, 
                                     const float* global_scale_inv, const void* packed, int N,
                                     float alpha, void* out, int out_dtype, int rcp_mode,
                                     void* workspace, size_t workspace_bytes, void* stream);
+/* The same linear for more tokens than one decode launch takes, given scratch for the quantized
+ * tokens: the tokens are quantized once into `scratch` and one launch multiplies all of them, the weight
+ * tile re-used for up to 256 tokens (gemm_large.cu), instead of one pass over the weight per 32 rows.
+ *   nvfp4r_linear_packed_scratch_bytes   bytes of scratch, or 0 where nvfp4r_linear_packed is the
+ *                                        faster kernel (few tokens) or the shape is unsupported:
+ *                                        call that one then
+ *   nvfp4r_linear_packed_scratch         scratch >= that many bytes, 16-byte aligned, any contents; not
+ *                                        kept after the launch
+ * Same operands, arithmetic and rcp_mode meaning; the weight must be final before the preceding
+ * kernel of the stream is launched. */
+NVFP4R_API size_t nvfp4r_linear_packed_scratch_bytes(int M, int N, int K);
+NVFP4R_API int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride, int M, int K,
+                                            const float* global_scale_inv, const void* packed, int N,
+                                            float alpha, void* out, int out_dtype, int rcp_mode,
+                                            void* scratch, size_t scratch_bytes, void* stream);
+/* Debug/tuning of that kernel: fewest tokens it takes (0 = automatic), tokens per tile (a multiple
+ * of 16 up to 256, 0 = automatic), schedule (0 whole tiles, 1 stream-K, -1 automatic). */
+NVFP4R_API int nvfp4r_set_gemm_large_tuning(int min_m, int tile_tokens, int stream_k);
+
 /* The same linear with the operator that PRODUCES its input fused into the prologue, so
  * that the bf16 activation never makes a round trip through HBM and one launch
  * disappears per fusion. The reference names this as its own end goal

@@ -295,9 +295,11 @@ int nvfp4r_gemm(const void* A, const void* B, const void* SFA, const void* SFB, 
     g.w = B; g.wsf_swizzled = SFB;
     g.a_codes = A; g.a_sf_swizzled = SFA;
     g.out = C; g.out_dtype = out_dtype; g.c_n_major = (c_layout == NVFP4R_C_N_MAJOR);
-    g.M = M; g.N = N; g.K = K; g.alpha = alpha; g.workspace = workspace;
+    g.M = M; g.N = N; g.K = K; g.alpha = alpha; g.workspace = workspace; g.workspace_bytes = workspace_bytes;
     const char* why = nullptr;
-    cudaError_t e = nvfp4r::launch_linear_tc(g, as_stream(stream), &why);
+    bool taken = false;
+    cudaError_t e = nvfp4r::launch_gemm_large(g, as_stream(stream), &taken);
+    if (e == cudaSuccess && !taken) e = nvfp4r::launch_linear_tc(g, as_stream(stream), &why);
     if (why != nullptr) return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, why);
     return e == cudaSuccess ? NVFP4R_OK : cuda_fail(e, "gemm launch");
 }
@@ -320,7 +322,7 @@ int nvfp4r_linear_tc(const void* x, int64_t x_row_stride, int M, int K, const fl
     g.w = weight; g.wsf_swizzled = weight_scale_swizzled;
     g.xb = x; g.xb_stride = x_row_stride; g.gs = gs; g.rcp_mode = rcp_mode;
     g.out = out; g.out_dtype = out_dtype; g.c_n_major = false;
-    g.M = M; g.N = N; g.K = K; g.alpha = alpha; g.workspace = workspace;
+    g.M = M; g.N = N; g.K = K; g.alpha = alpha; g.workspace = workspace; g.workspace_bytes = workspace_bytes;
     const char* why = nullptr;
     cudaError_t e = nvfp4r::launch_linear_tc(g, as_stream(stream), &why);
     if (why != nullptr) return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, why);
@@ -383,6 +385,39 @@ int nvfp4r_linear_packed(const void* x, int64_t x_row_stride, int M, int K, cons
     cudaError_t e = nvfp4r::launch_linear_packed(g, as_stream(stream), &why);
     if (why != nullptr) return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, why);
     return e == cudaSuccess ? NVFP4R_OK : cuda_fail(e, "linear_packed launch");
+}
+
+size_t nvfp4r_linear_packed_scratch_bytes(int M, int N, int K) { return nvfp4r::large_scratch_bytes(M, N, K); }
+
+int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride, int M, int K, const float* gs,
+                                 const void* packed, int N, float alpha, void* out, int out_dtype, int rcp_mode,
+                                 void* scratch, size_t scratch_bytes, void* stream) {
+    NVFP4R_RANGE("nvfp4r_linear_packed_scratch");
+    if (!x || !gs || !packed || !out || !scratch) return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: null pointer");
+    if (rcp_mode != NVFP4R_RCP_EXACT && rcp_mode != NVFP4R_RCP_APPROX)
+        return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: bad rcp_mode");
+    if (out_dtype < NVFP4R_BF16 || out_dtype > NVFP4R_F32)
+        return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: bad out_dtype");
+    const size_t need = nvfp4r::large_scratch_bytes(M, N, K);
+    if (need == 0)
+        return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, "linear_packed_scratch: shape belongs to nvfp4r_linear_packed");
+    if (scratch_bytes < need || !aligned(scratch, 16))
+        return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: scratch too small or misaligned");
+    if (!aligned(x, 16) || (x_row_stride % 8) || !aligned(packed, 16) || !aligned(out, out_dtype == NVFP4R_F32 ? 4 : 2))
+        return fail(NVFP4R_ERR_ALIGNMENT, "linear_packed_scratch: x and packed weight need 16-byte alignment");
+    if (x_row_stride < K) return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: row stride < K");
+    nvfp4r::PackedLinearArgs g = {};
+    g.packed = packed; g.xb = x; g.xb_stride = x_row_stride; g.gs = gs; g.rcp_mode = rcp_mode;
+    g.out = out; g.out_dtype = out_dtype; g.M = M; g.N = N; g.K = K; g.alpha = alpha;
+    cudaError_t e = nvfp4r::launch_linear_large(g, scratch, as_stream(stream));
+    return e == cudaSuccess ? NVFP4R_OK : cuda_fail(e, "linear_packed_scratch launch");
+}
+
+int nvfp4r_set_gemm_large_tuning(int min_m, int tile_tokens, int stream_k) {
+    if (min_m < 0 || tile_tokens < 0 || tile_tokens > 256 || tile_tokens % 16 || stream_k < -1 || stream_k > 1)
+        return fail(NVFP4R_ERR_INVALID_ARGUMENT, "gemm large tuning: min_m >= 0, tile_tokens 0..256 in 16s, stream_k -1..1");
+    nvfp4r::set_large_tuning(min_m, tile_tokens, stream_k);
+    return NVFP4R_OK;
 }
 
 int nvfp4r_linear_packed_ex(const nvfp4r_prologue* pro, const void* x, int64_t x_row_stride, int M, int K,
@@ -709,6 +744,7 @@ int nvfp4r_status_mirror(volatile int** host_word) {
         if (e == cudaSuccess) e = nvfp4r::set_status_mirror_peer(d);
         if (e == cudaSuccess) e = nvfp4r::set_status_mirror_reset(d);
         if (e == cudaSuccess) e = nvfp4r::set_status_mirror_head(d);
+        if (e == cudaSuccess) e = nvfp4r::set_status_mirror_large(d);
         if (e != cudaSuccess) { cudaFreeHost(h); return cuda_fail(e, "status_mirror: set-up"); }
         host_ptr[dev] = h;
     }
@@ -727,7 +763,9 @@ int nvfp4r_check_device_status(void) {
     if (e == cudaSuccess) e = nvfp4r::read_and_clear_reset_status(&flag5);
     int flag6 = 0;
     if (e == cudaSuccess) e = nvfp4r::read_and_clear_head_status(&flag6);
-    flag4 |= flag5 | flag6;
+    int flag7 = 0;
+    if (e == cudaSuccess) e = nvfp4r::read_and_clear_large_status(&flag7);
+    flag4 |= flag5 | flag6 | flag7;
     if (e != cudaSuccess) return cuda_fail(e, "device status");
     flag |= flag2 | flag3 | flag4;
     return flag ? fail(NVFP4R_ERR_DEVICE_TIMEOUT, "a bounded device-side wait gave up") : NVFP4R_OK;

@@ -79,6 +79,9 @@ struct GemvTuning {
 GemvTuning& gemv_tuning();
 
 // ---- gemm_tcgen05.cu ------------------------------------------------------
+// Front part of a gemm workspace that only ever holds tile tickets (zero between launches), wherever
+// the workspace is large enough to keep the partial sums of every shape behind it.
+constexpr size_t kGemmTicketArea = 4096;
 // One NVFP4 weight [N,K/2] (+ swizzled scales) against M activation rows, either
 // bf16 rows quantized on the fly (xb) or pre-quantized codes + swizzled scales.
 struct TcLinearArgs {
@@ -96,6 +99,7 @@ struct TcLinearArgs {
     int M, N, K;
     float alpha;
     void* workspace;
+    size_t workspace_bytes;
 };
 size_t gemm_workspace_bytes(int M, int N, int K);
 // `*why` is set (and cudaSuccess returned) when the shape is outside what the
@@ -138,6 +142,16 @@ void set_packed_tuning(int splits);
 #ifdef NVFP4R_TRACE
 cudaError_t read_packed_trace(unsigned long long* out16);
 #endif
+
+// ---- gemm_large.cu --------------------------------------------------------
+// Scratch of the many-token linear over a packed weight; 0: launch_linear_packed is to be used.
+size_t large_scratch_bytes(int M, int N, int K);
+cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaStream_t stream);
+// *taken = false: nothing was launched, launch_linear_tc is to be used.
+cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* taken);
+void set_large_tuning(int min_m, int bn, int stream_k);
+cudaError_t set_status_mirror_large(int* device_ptr);
+cudaError_t read_and_clear_large_status(int* flag);
 
 // Synchronises the device, returns the time-out flag set by bounded waits
 // inside the kernels and clears it.

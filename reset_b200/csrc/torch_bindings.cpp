@@ -254,6 +254,20 @@ at::Tensor linear_packed_op(const at::Tensor& x, const at::Tensor& global_scale_
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     const auto dt = out_dtype_int == 0 ? at::kBFloat16 : out_dtype_int == 1 ? at::kHalf : at::kFloat;
     auto out = at::empty({M, N}, x.options().dtype(dt));
+    // many tokens: quantized once into scratch of this call (the caching allocator's, so capture and
+    // streams are its business), one launch for all of them
+    const size_t scratch_bytes = nvfp4r_linear_packed_scratch_bytes(static_cast<int>(M), static_cast<int>(N),
+                                                                    static_cast<int>(K));
+    if (scratch_bytes > 0) {
+        auto scratch = at::empty({static_cast<int64_t>(scratch_bytes)}, x.options().dtype(at::kByte));
+        check_status(nvfp4r_linear_packed_scratch(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),
+                                                  global_scale_inv.data_ptr<float>(), packed.data_ptr(),
+                                                  static_cast<int>(N), static_cast<float>(alpha), out.data_ptr(),
+                                                  static_cast<int>(out_dtype_int), static_cast<int>(rcp_mode),
+                                                  scratch.data_ptr(), scratch_bytes, current_stream()),
+                     "linear_packed");
+        return out;
+    }
     at::Tensor& ws = fixed_workspace(1, x.device(),
                                      nvfp4r_linear_packed_workspace_bytes(static_cast<int>(M), static_cast<int>(N),
                                                                           static_cast<int>(K)), "linear_packed");

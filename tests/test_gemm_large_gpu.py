@@ -1,0 +1,149 @@
+"""GPU parity of the many-token tensor-core kernel (``gemm_large.cu``) against the CPU oracle: tile edges
+and remainders in tokens and K, both schedules (whole tiles, stream-K), both operand forms (packed
+weight through ``torch.ops.nvfp4r.linear_packed``, row-major operands through ``nvfp4r_gemm``), every
+output type and layout. Products of e2m1 codes and e4m3 scales are exact and sums are fp32: rel-L2 <=
+1e-5 against the float64 dequantise-matmul, the bound of the other tensor-core kernels; 16-bit outputs
+add half a unit in the last place per element (2^-8 of it for the 8 significant bits of bf16, 2^-11 for
+the 11 of fp16)."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import nvfp4 as onv
+from helpers import cuda, make_activation, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+F32 = 2
+
+
+@pytest.fixture(scope="module")
+def capi():
+    import reset_b200.nvfp4r  # noqa: F401  (registers the operators)
+    from reset_b200 import capi as c
+    return c
+
+
+@pytest.fixture(autouse=True)
+def _tuning():
+    from reset_b200 import _lib
+    yield
+    _lib.lib().nvfp4r_set_gemm_large_tuning(0, 0, -1)
+
+
+def _tune(min_m, bn, sk):
+    from reset_b200 import _lib
+    _lib.check(_lib.lib().nvfp4r_set_gemm_large_tuning(min_m, bn, sk), "tuning")
+
+
+def _case(M, N, K, seed):
+    w, ws = onv.random_nvfp4((N,), K, seed=seed)
+    xb = make_activation(M, K, seed=seed + 1)
+    xc, xsf = onv.quantize_nvfp4(xb.float().numpy(), 48.0)
+    return w, ws, xb, torch.tensor([48.0], device="cuda"), onv.linear_f64(w, ws, xc, xsf, alpha=0.5)
+
+
+def _packed(capi, w, ws, xb, gs, N, dtype=F32):
+    packed = capi.pack_weight(cuda(w), cuda(ws))
+    return torch.ops.nvfp4r.linear_packed(xb, gs, packed, N, 0.5, dtype, 0)
+
+
+@pytest.mark.parametrize("bn,sk", [(0, -1), (16, 0), (64, 1), (112, 0), (112, 1), (128, 0), (128, 1), (176, 0), (256, 0),
+                                   (256, 1)])
+@pytest.mark.parametrize("M,N,K", [(33, 128, 128), (45, 2560, 5120), (128, 384, 640), (129, 256, 1024), (257, 1920, 5760)])
+def test_packed_tiles_and_schedules(capi, M, N, K, bn, sk):
+    _tune(1, bn, sk if sk != 1 or (N // 128) * ((K + 255) // 256) >= 296 else -1)
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + K)
+    x = torch.empty(M, K + 24, dtype=torch.bfloat16, device="cuda")[:, :K]     # rows further apart than K
+    x.copy_(xb)
+    a = _packed(capi, w, ws, x, gs, N)
+    b = _packed(capi, w, ws, x, gs, N)
+    assert torch.equal(a, b)                                                   # does not depend on arrival order
+    assert rel_l2(a.cpu().numpy(), exact) <= 1e-5
+
+
+@pytest.mark.parametrize("M", [1, 2, 15, 16, 17, 31, 32, 47, 64, 65, 96, 127, 200, 255, 256, 300, 511, 513, 777])
+def test_packed_token_counts_stay_inside_the_output(capi, M):
+    from reset_b200 import _lib
+    _tune(1, 0, -1)
+    N, K = 256, 768
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M)
+    packed, x = capi.pack_weight(cuda(w), cuda(ws)), xb.cuda()
+    lib = _lib.lib()
+    n = lib.nvfp4r_linear_packed_scratch_bytes(M, N, K)
+    scratch = torch.full((n + 512,), 0x7F, dtype=torch.uint8, device="cuda")   # NaN scales wherever nothing is written
+    out = torch.full((M * N + 512,), 7.0, device="cuda")
+    st = lib.nvfp4r_linear_packed_scratch(x.data_ptr(), K, M, K, gs.data_ptr(), packed.data_ptr(), N, 0.5,
+                                          out.data_ptr() + 1024, F32, 0, scratch.data_ptr() + 256, n,
+                                          torch.cuda.current_stream().cuda_stream)
+    _lib.check(st, "linear_packed_scratch")
+    got = out.cpu().numpy()
+    assert (got[:256] == 7.0).all() and (got[256 + M * N:] == 7.0).all()
+    s = scratch.cpu().numpy()
+    assert (s[:256] == 0x7F).all() and (s[256 + n:] == 0x7F).all()
+    assert rel_l2(got[256:256 + M * N].reshape(M, N), exact) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype,half_ulp", [(0, 2.0 ** -8), (1, 2.0 ** -11)])
+def test_packed_16_bit_outputs_round_once(capi, dtype, half_ulp):
+    M, N, K = 131, 384, 1024
+    w, ws, xb, gs, exact = _case(M, N, K, seed=5)
+    got = _packed(capi, w, ws, xb.cuda(), gs, N, dtype).double().cpu().numpy()
+    scale = np.abs(exact) + np.sqrt(np.mean(exact ** 2)) * 1e-3
+    assert np.max(np.abs(got - exact) / scale) <= half_ulp * 1.01
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n_major", [True, False])
+@pytest.mark.parametrize("M,N,K,bn,sk", [(33, 128, 256, 0, -1), (40, 2560, 4096, 0, 1), (64, 1280, 8192, 64, 1),
+                                         (130, 384, 1024, 128, 0), (300, 1280, 4096, 256, 1), (257, 256, 512, 256, 0)])
+def test_gemm_row_major(capi, M, N, K, bn, sk, n_major, dtype):
+    _tune(0, bn, sk)
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + N)
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    C = torch.full((M, N), float("nan"), dtype=dtype, device="cuda")
+    wksp = torch.zeros(16 << 20, dtype=torch.int64, device="cuda")
+    capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=n_major)
+    got = C.double().cpu().numpy()
+    got = got.reshape(N, M).T if n_major else got
+    assert rel_l2(got, exact) <= {torch.float32: 1e-5, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+
+
+def test_gemm_output_of_any_alignment(capi):
+    """A 2-byte aligned output takes the narrow stores."""
+    M, N, K = 48, 256, 512
+    w, ws, xb, gs, exact = _case(M, N, K, seed=9)
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    buf = torch.zeros(M * N + 1, dtype=torch.float16, device="cuda")
+    wksp = torch.zeros(16 << 20, dtype=torch.int64, device="cuda")
+    for n_major in (True, False):
+        C = buf[1:].view(M, N)
+        capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=n_major)
+        got = C.double().cpu().numpy()
+        assert rel_l2(got.reshape(N, M).T if n_major else got, exact) <= 2.0 ** -11
+
+
+def test_gemm_small_workspace_takes_the_other_kernel(capi):
+    """A workspace sized for 32 rows served any M before and still does."""
+    M, N, K = 70, 512, 4096
+    w, ws, xb, gs, exact = _case(M, N, K, seed=3)
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    C = torch.empty((M, N), device="cuda")
+    capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, capi.gemm_workspace(32, N, K, "cuda"), n_major=False)
+    assert rel_l2(C.cpu().numpy(), exact) <= 1e-5
+
+
+def test_linear_packed_under_capture(capi):
+    M, N, K = 160, 512, 1024
+    w, ws, xb, gs, exact = _case(M, N, K, seed=4)
+    packed, x = capi.pack_weight(cuda(w), cuda(ws)), xb.cuda()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = torch.ops.nvfp4r.linear_packed(x, gs, packed, N, 0.5, F32, 0)
+    for _ in range(3):
+        out.zero_()
+        g.replay()
+        assert rel_l2(out.cpu().numpy(), exact) <= 1e-5
