@@ -471,7 +471,12 @@ cudaError_t launch_linear_tc(const TcLinearArgs& g, cudaStream_t stream, const c
         p.splits = plan.splits;
         p.iters = g.K / kBK;
         p.stages = plan.stages;
-        const size_t tickets = (static_cast<size_t>(p.tiles) * sizeof(unsigned) + 255) / 256 * 256;
+        // Tickets of every shape share the front of the workspace and partial sums stay behind it: a
+        // workspace that serves shapes of different N would otherwise offer one shape's partial sums
+        // as another's tickets. A workspace too small for that keeps the tight layout.
+        size_t tickets = (static_cast<size_t>(p.tiles) * sizeof(unsigned) + 255) / 256 * 256;
+        const size_t partials = plan.splits > 1 ? static_cast<size_t>(p.tiles) * plan.splits * plan.bn * kTileRows * sizeof(float) : 0;
+        if (tickets < kGemmTicketArea && kGemmTicketArea + partials <= g.workspace_bytes) tickets = kGemmTicketArea;
         p.tickets = static_cast<unsigned*>(g.workspace);
         p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(g.workspace) + tickets);
 

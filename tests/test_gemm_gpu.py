@@ -162,3 +162,15 @@ def test_tc_rejects_bad_shapes(capi):
     w = torch.zeros((100, 128), dtype=torch.uint8, device="cuda")
     with pytest.raises(_lib.Nvfp4rError):
         capi.linear_tc(xb, gs, w, sf, 1.0, wk)                # N % 128
+
+
+def test_one_workspace_serves_every_shape(capi):
+    """The fixed scratch of the operator is shared by weights of every width: the partial sums that a
+    narrow weight leaves behind are not taken for the tile tickets of a wide one."""
+    wksp = torch.zeros(16 << 20, dtype=torch.int64, device="cuda")
+    for N, K in ((512, 8192), (24576, 2048), (512, 8192), (16384, 2048)):
+        w, ws, wd, wsd = _weights(N, K, seed=N % 97)
+        xc, xsf = onv.random_nvfp4((4,), K, seed=21)
+        C = torch.full((4, N), float("nan"), dtype=torch.float32, device="cuda")
+        capi.gemm(cuda(xc), wd, cuda(onv.swizzle_blockscale(xsf)), wsd, C, 1.0, wksp, n_major=False)
+        assert rel_l2(C.cpu().numpy(), onv.linear_f64(w, ws, xc, xsf)) <= 1e-5
