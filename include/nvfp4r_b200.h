@@ -610,8 +610,8 @@ NVFP4R_API int nvfp4r_sample(const float* logits, int64_t row_stride, int B, int
  * descent over order-preserving keys of the logits (three levels of 2048-bin histograms of count
  * and fixed-point probability mass, integer atomics: the result does not depend on the order of
  * the additions), then the Gumbel-max draw skips everything below the threshold key.
- *   workspace  >= nvfp4r_sample_workspace_bytes(B) bytes, 8-byte aligned, ALL ZERO before its first
- *              use; every call leaves the histograms zeroed. Calls that share it must be ordered.
+ *   workspace  >= nvfp4r_sample_workspace_bytes(B) bytes, 8-byte aligned. Checked and left untouched: one
+ *              launch of a thread-block cluster per row keeps the histograms in shared memory.
  * No counterpart in the reference (vLLM owns the sampler there, reset/README.md:87-88). */
 NVFP4R_API size_t nvfp4r_sample_workspace_bytes(int B);
 NVFP4R_API int nvfp4r_sample_top_k_top_p(const float* logits, int64_t row_stride, int B, int V,

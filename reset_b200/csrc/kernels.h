@@ -153,6 +153,12 @@ void set_large_tuning(int min_m, int bn, int stream_k);
 cudaError_t set_status_mirror_large(int* device_ptr);
 cudaError_t read_and_clear_large_status(int* flag);
 
+// ---- sample_truncated.cu --------------------------------------------------
+// top_k 0: no top-k; top_p >= 1: no top-p.
+cudaError_t launch_sample_truncated(const float* logits, int64_t row_stride, int B, int V, int top_k, float top_p,
+                                    unsigned long long seed, unsigned long long* draws, int* last_ids, int* out,
+                                    cudaStream_t stream);
+
 // Synchronises the device, returns the time-out flag set by bounded waits
 // inside the kernels and clears it.
 cudaError_t read_and_clear_device_status(int* flag);

@@ -337,6 +337,74 @@ def test_sample_top_k_top_p_support_and_frequencies(V, top_k, top_p):
     assert chi_ours < dof + 6 * (2 * dof) ** 0.5 + 10, (chi_ours, chi_ref, dof)
 
 
+def _gumbel_scores(row, seed, b, draw):
+    """The restated generator over a whole row at once (numpy, wrapping 64-bit integers)."""
+    def mix(z):
+        z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        return z ^ (z >> np.uint64(31))
+    key = np.uint64(_mix64((seed ^ _mix64(((b << 40) + draw) & _M64)) & _M64))
+    with np.errstate(over="ignore"):
+        r = mix(key + np.arange(row.size, dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15))
+    u = ((r >> np.uint64(41)).astype(np.float32) + np.float32(0.5)) * np.float32(1.0 / 8388608.0)
+    return row.astype(np.float64) - np.log(-np.log(u.astype(np.float64)))
+
+
+@pytest.mark.parametrize("V,stride,k", [
+    (1, 1, 0), (7, 8, 2), (8, 8, 7), (33, 36, 1), (33, 33, 16), (4095, 4096, 17), (4097, 4097, 512), (4100, 4100, 513),
+    (32000, 32000, 20), (151936, 151936, 20), (151936, 151939, 1024), (393216, 393216, 50), (393217, 393217, 50),
+])
+def test_sample_one_launch_draws_the_exact_set(V, stride, k):
+    """Slices with remainders, empty slices, unaligned rows, k on both sides of the bound's range and rows on both
+    sides of the shared-memory limit: the id is the restated generator's arg-max over the exact top-k / top-p set.
+    Scores are compared, not ids: the kernel's fp32 logf is within a few ulp of a noise of at most 20, so
+    the drawn id scores within 1e-4 of the best in float64 (5e-6 x 20)."""
+    from reset_b200 import capi
+    B, seed = 5, 21
+    g = torch.Generator().manual_seed(V + k)
+    x = torch.randn(B, stride, generator=g) * 3
+    rows = x[:, :V]
+    rows[1] = rows[1].round()                             # ties: all of the k-th value's equals stay
+    if V > 4:
+        rows[2, V // 2:] = float("-inf")
+        rows[2, 0] = float("nan")
+        rows[3, V // 3] = float("inf")                    # an infinite logit always wins
+        rows[4] = 1.25                                    # one value only
+    dev = x.cuda()[:, :V]
+    ws = capi.sample_workspace(B, "cuda")
+    for top_p in (1.0, 1e-6):
+        draws = torch.arange(B, dtype=torch.int64, device="cuda")
+        ids = capi.sample(dev, draws, seed=seed, top_k=k, top_p=top_p, workspace=ws).tolist()
+        assert draws.tolist() == [b + 1 for b in range(B)]
+        for b in range(B):
+            row = rows[b].numpy()
+            ok = row > -np.inf
+            if 0 < k < V and ok.sum() >= k:
+                ok &= row >= np.sort(row[ok])[-k]
+            if top_p < 1.0:                               # a vanishing nucleus: the largest value and its equals
+                ok &= row == row[ok].max()
+            score = np.where(ok, _gumbel_scores(np.where(ok, row, 0), seed, b, b), -np.inf)
+            assert ok[ids[b]] and (score[ids[b]] >= score.max() - 1e-4 or score.max() == np.inf), (b, top_p, ids[b])
+
+
+@pytest.mark.parametrize("V", [64, 151936, 400000])
+def test_sample_one_launch_nucleus_boundary(V):
+    """Halving masses 1/2, 1/4, ...: 0.9 needs four tokens, 0.9 of the top three renormalised needs all three."""
+    from reset_b200 import capi
+    B = 256
+    pos = torch.randperm(V, generator=torch.Generator().manual_seed(V))[:30]
+    row = torch.full((V,), -200.0)
+    row[pos] = 5.0 - 0.6931472 * torch.arange(30, dtype=torch.float32)
+    dev = row.repeat(B, 1).cuda()
+    ws = capi.sample_workspace(B, "cuda")
+    for k, p, n in ((0, 0.9, 4), (3, 0.9, 3), (3, 0.8, 2), (2, 1.0, 2), (0, 0.49, 1)):
+        seen = set()
+        draws = torch.zeros(B, dtype=torch.int64, device="cuda")
+        for _ in range(3):
+            seen |= set(capi.sample(dev, draws, seed=4, top_k=k, top_p=p, workspace=ws).tolist())
+        assert seen == set(pos[:n].tolist()), (k, p)
+
+
 def test_sample_truncation_edge_rows():
     """One-hot rows (what ReSET writes for temperature 0), rows with fewer finite entries than k,
     top_p so small that one token remains, and the untruncated call through the same entry."""
