@@ -411,12 +411,15 @@ void set_gemv_rows_tuning(int mode, int rows, int target_warps) {
 // L2-cold: 6144x4096 5.1 vs 5.3 us, 6400x5120 6.7 vs 6.3 us, 4096x12288 10.9 vs 7.8 us,
 // 5120x3200 11.1 (plain loads) vs 4.9 us), and for N where the ring kernel's groups of 4 rows
 // leave a second round to under a quarter of its warps (N = 5120: 5120x5120 7.3 us on the ring
-// kernel). More tokens: the ring kernel.
+// kernel). More tokens: the MMA kernel (gemv_mma.cu), faster on every shape measured (640x1024 to
+// 25600x12288, 2 to 8 tokens: 1.2 to 5 times), and the ring kernel where the tokens don't fit its shared memory
+// (8 tokens: K > 13440).
 cudaError_t launch_gemv_auto(const GemvArgs& a, cudaStream_t stream) {
     if (a.push_world > 1)        // the all-reduce inside the launch exists in the ring kernel only
         return (a.pro_kind == 0 && gemv_stream_supported(a)) ? launch_gemv_stream(a, stream) : cudaErrorNotSupported;
     if (a.pro_kind != 0)         // fused prologues exist in the register-resident kernel only
         return gemv_rows_supported(a) ? launch_gemv_rows(a, stream) : cudaErrorNotSupported;
+    if (!gemv_tuning().force_generic && gemv_mma_supported(a)) return launch_gemv_mma(a, stream);
     const bool ring = gemv_stream_supported(a);
     if (!gemv_tuning().force_generic && gemv_rows_supported(a)) {
         const int64_t wbytes = static_cast<int64_t>(a.N) * a.K * 9 / 16;

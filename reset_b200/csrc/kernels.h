@@ -62,6 +62,8 @@ cudaError_t launch_gemv_stream(const GemvArgs& a, cudaStream_t stream);
 cudaError_t launch_gemv_generic(const GemvArgs& a, cudaStream_t stream);
 
 // The register-resident kernel for one or two tokens (gemv_rows.cu).
+bool gemv_mma_supported(const GemvArgs& a);      // two to eight tokens (gemv_mma.cu)
+cudaError_t launch_gemv_mma(const GemvArgs& a, cudaStream_t stream);
 bool gemv_rows_supported(const GemvArgs& a);
 cudaError_t launch_gemv_rows(const GemvArgs& a, cudaStream_t stream);
 // mode: 0 automatic, 1 whenever supported, -1 never; rows per step 0 (automatic), 2 or 4;

@@ -186,3 +186,32 @@ def test_bad_arguments_are_rejected(capi):
     st = _lib.lib().nvfp4r_gemv(wd.data_ptr(), wd.data_ptr(), wd.data_ptr(), wd.data_ptr(),
                                 out.data_ptr(), 1, 8, 48, 0, 24, 0, 3, 24, 3, 1.0, 1, None)
     assert st == -2                                                           # K % 32
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 1, 32), (3, 15, 96), (8, 16, 128), (5, 17, 160), (2, 4737, 1024), (7, 4100, 2080),
+                                   (4, 300, 12288), (8, 33, 13440), (8, 33, 13568), (6, 2400, 992), (8, 40, 25600)])
+def test_gemv_of_several_tokens(capi, M, N, K):
+    """The MMA kernel at the edges of its tiles (16 rows, 128 elements, 8 warps), one and two CTAs per SM, more
+    tiles than CTAs, and past the largest K it can hold; quantized tokens and bf16 tokens, padded weight rows.
+    Products are exact and sums are fp32: 1e-5 as for the other kernels; bf16 adds 2^-8 per element."""
+    w, ws = onv.random_nvfp4((N,), K, seed=N + K)
+    x, xs = onv.random_nvfp4((M, 1), K, seed=M)
+    wd = torch.zeros(N, K // 2 + 32, dtype=torch.uint8, device="cuda")[:, :K // 2]
+    wd.copy_(cuda(w))
+    wsd = cuda(ws)
+    out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    again = torch.empty_like(out)
+    for o in (out, again):
+        capi.gemv_out(wd.unsqueeze(0).expand(M, -1, -1), wsd.unsqueeze(0).expand(M, -1, -1), cuda(x), cuda(xs), o, 0.5)
+    assert torch.equal(out, again)
+    assert rel_l2(out.cpu().numpy(), onv.linear_f64(w, ws, x[:, 0], xs[:, 0], alpha=0.5)) <= 1e-5
+    tok = (torch.randn(M, K + 8, generator=torch.Generator().manual_seed(K)).to(torch.bfloat16))[:, :K]
+    xc, xsf = onv.quantize_nvfp4(tok.float().numpy(), 48.0)
+    exact = onv.linear_f64(w, ws, xc, xsf, alpha=0.5)
+    dev = torch.empty(M, K + 8, dtype=torch.bfloat16, device="cuda")[:, :K]
+    dev.copy_(tok)
+    gs = torch.tensor([48.0], device="cuda")
+    for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 2.0 ** -8)):
+        got = torch.empty(M, N, dtype=dtype, device="cuda")
+        capi.linear(dev, gs, cuda(w), cuda(ws), 0.5, out=got, rcp_mode=0)
+        assert rel_l2(got.float().cpu().numpy(), exact) <= tol
