@@ -630,12 +630,27 @@ void fill_common(const LargePlan& plan, LargeParams* p, void* out, int M, int N,
 
 }  // namespace
 
-// Tokens from which this path is taken: up to 32 the decode kernels make one pass over the weight too.
+// Tokens from which the row-major operands of the raw gemm operator take this path.
 constexpr int kLargeMinM = 33;
+
+// Tokens from which the packed linear takes it, where the caller can give it scratch. Up to 16 tokens the decode kernel
+// makes one pass over the weight as well and needs no second launch; its CTAs each quantize the tokens of their
+// K part, which grows with the tokens, while this path pays a few us for partial sums where the weight has few
+// row tiles and long rows. Measured, us, decode kernel / this one:
+//   N >= 6 K       34816x5120: 12 tokens 22.0 / 21.8, 16 tokens 26.4 / 21.5; 12288x2048: 13 tokens 8.2 / 6.4;
+//                  but (N >= 16 K) 24576x1024: 13 tokens 6.1 / 6.8, 17 tokens 8.1 / 6.9
+//   N >= 1.5 K     24576x4096: 16 tokens 17.8 / 17.8, 17 tokens 27.0 / 18.0; 10240x5120: 17 tokens 15.9 / 11.6;
+//                  6144x4096: 17 tokens 10.0 / 9.7
+//   N >= K         4096x4096: 24 tokens 9.2 / 9.4, 32 tokens 11.3 / 9.5
+//   below          4096x12288: 24 tokens 13.2 / 15.7, 32 tokens 15.7 / 15.7; 1280x5120: 32 tokens 9.6 / 11.2
+int large_min_m(int N, int K) {
+    const int64_t n = N, k = K;
+    return n >= 6 * k && n < 16 * k ? 13 : 2 * n >= 3 * k ? 17 : n >= k ? 25 : kLargeMinM;
+}
 
 size_t large_scratch_bytes(int M, int N, int K) {
     LargePlan plan;
-    if (M < (g_large_min_m ? g_large_min_m : kLargeMinM) || N <= 0 || K <= 0 || N % kRows || K % 128) return 0;
+    if (M < (g_large_min_m ? g_large_min_m : large_min_m(N, K)) || N <= 0 || K <= 0 || N % kRows || K % 128) return 0;
     if (!plan_large(M, N, K, false, &plan)) return 0;
     return plan.token_bytes + plan.ticket_bytes + plan.partial_bytes;
 }

@@ -65,6 +65,16 @@ def test_packed_tiles_and_schedules(capi, M, N, K, bn, sk):
     assert rel_l2(a.cpu().numpy(), exact) <= 1e-5
 
 
+@pytest.mark.parametrize("N,K,first", [(1536, 256, 13), (4096, 256, 17), (384, 256, 17), (256, 256, 25), (256, 384, 33)])
+def test_first_token_count_follows_the_shape(capi, N, K, first):
+    """Both sides of the line between the decode kernel and this one, per shape class, give the same product."""
+    from reset_b200 import _lib
+    for M in (first - 1, first):
+        assert (_lib.lib().nvfp4r_linear_packed_scratch_bytes(M, N, K) > 0) == (M >= first)
+        w, ws, xb, gs, exact = _case(M, N, K, seed=M)
+        assert rel_l2(_packed(capi, w, ws, xb.cuda(), gs, N).cpu().numpy(), exact) <= 1e-5
+
+
 @pytest.mark.parametrize("M", [1, 2, 15, 16, 17, 31, 32, 47, 64, 65, 96, 127, 200, 255, 256, 300, 511, 513, 777])
 def test_packed_token_counts_stay_inside_the_output(capi, M):
     from reset_b200 import _lib
