@@ -2,28 +2,33 @@
 //
 // The row is read from memory once; each CTA keeps an eighth of it in shared memory and the eight exchange
 // histograms, totals and picks through distributed shared memory with cluster barriers. Phases:
-//   1. load, row maximum, and a lower bound of the k-th largest value;
-//   2. per truncation (top-k by count, then top-p by mass) a radix descent over the order-preserving keys,
+//   1. load, row maximum;
+//   2. top-k up to 128: the k-th largest of the 128 warps' maxima bounds the k-th largest value from below (k
+//      groups have an element at or above it). What reaches the bound goes to one CTA's list, a few more than k
+//      on unordered logits; with at most 512 entries that CTA settles the row by comparing all pairs, one
+//      entry per thread, and the launch ends;
+//   3. otherwise, per truncation (top-k by count, then top-p by mass) a radix descent over the order-preserving keys,
 //      11 + 11 + 10 bits: histogram of the keys that share the prefix found so far, each CTA sums 256 of the
 //      2048 bins over the eight histograms, and the CTA whose bins cross the goal announces the bin. After
 //      the last level the prefix is the key of the last token kept; equal keys are all kept;
-//   3. arg-max of logit + Gumbel noise among the keys at or above the threshold.
+//   4. arg-max of logit + Gumbel noise among the keys at or above the threshold.
 // Mass is exp(x - row max) scaled by 2^32 and truncated to an integer, so no result depends on the order of
 // the additions. Elements of mass 0 are left out of the top-p histograms: a bin of mass 0 is never the first
 // to reach the goal.
 //
 // Bound: latency (barriers and dependent passes over shared memory); the traffic is 0.6 MB per row.
 // Measured against 11 to 17 launches over a scratch in device memory, 151936 entries, us a call, before -> after:
-//   top-k 20 top-p 0.95   1 row 57.7 -> 35.1   8 rows 70.9 -> 37.6   32 rows 133 -> 47.2   256 rows 956 -> 373
-//   top-p 0.9             1 row 38.3 -> 35.5   8 rows 49.5 -> 41.0   32 rows 105 -> 55.5   256 rows 700 -> 407
+//   top-k 20 top-p 0.95   1 row 57.7 -> 7.4    8 rows 70.9 -> 8.4    32 rows 133 -> 10.1   256 rows 956 -> 90
+//   top-p 0.9             1 row 38.3 -> 35.3   8 rows 49.5 -> 41.4   32 rows 105 -> 55.4   256 rows 700 -> 410
+//   top-k 1000            1 row 37.1 -> 24.1   8 rows 45.1 -> 26.1   32 rows 96 -> 34.8    256 rows 657 -> 268
+// (the first line without phase 2: 35.1, 37.6, 47.2, 373)
 //
 //   * 8 CTAs of 512 threads: the largest cluster every device can place, and at 151936 entries two CTAs
 //     (76 KB of row each) fit an SM, so 32 rows run at once.
 //   * A shared-memory add on a 64-bit word is a compare-and-swap loop, and logits crowd into few of the
 //     first level's bins. So masses are added as two 32-bit halves (16 + 17 bits; a slice has fewer than
-//     65536 elements, so neither overflows), and top-k counts only what is at or above the bound of phase 1:
-//     of g >= k disjoint groups of a row's elements the smallest group maximum has at least k elements at or
-//     above it. Rows too long for shared memory are re-read from L2 and use 64-bit adds.
+//     65536 elements, so neither overflows), and top-k counts only what reaches the bound of phase 2. Rows too
+//     long for shared memory are re-read from L2 and use 64-bit adds.
 #include <cooperative_groups.h>
 
 #include "kernels.h"
@@ -45,12 +50,16 @@ constexpr int kMaxCached = 48 * 1024;          // elements of a slice kept in sh
 __host__ __device__ constexpr int level_shift(int level) { return level == 0 ? 21 : (level == 1 ? 10 : 0); }
 __host__ __device__ constexpr int level_bins(int level) { return level == 2 ? 1024 : 2048; }
 
-__device__ __forceinline__ uint32_t warp_max_u(uint32_t v, int width) {
-    for (int s = width / 2; s > 0; s >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, s));
-    return v;
+constexpr int kGroups = kCtas * kWarps;        // groups of a row: one per warp
+constexpr int kListMax = kThreads;                // candidates that one CTA settles, one per thread
+
+__device__ __forceinline__ unsigned long long mass_of(float x, float m) {
+    // the maximum itself weighs exactly 2^32, also when it is +inf
+    return x == m ? (1ull << 32) : __float2ull_rd(__expf(x - m) * 4294967296.0f);
 }
 
-template <bool kCached>
+// kFew: 0 < top_k <= kGroups (its own instance: the list's code costs the descent registers)
+template <bool kCached, bool kFew>
 __global__ void __launch_bounds__(kThreads, 2)
 sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int per, int top_k, float top_p,
                         unsigned long long seed, unsigned long long* __restrict__ draws,
@@ -60,11 +69,14 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
     __shared__ __align__(16) uint32_t s_hist[2 * kBins];
     __shared__ unsigned long long s_scan[kSeg / 32];
     __shared__ float s_f[kWarps];
-    __shared__ uint32_t s_u[kWarps];
     __shared__ int s_i[kWarps];
     // written by the CTAs of the cluster
     __shared__ float s_peer_max[kCtas];
-    __shared__ uint32_t s_peer_bound[kCtas];
+    __shared__ uint32_t s_group[kGroups];
+    __shared__ uint32_t s_bound;
+    __shared__ int s_count;                                   // rank 0: candidates of the row
+    __shared__ float s_list_x[kListMax];
+    __shared__ int s_list_i[kListMax];
     __shared__ unsigned long long s_peer_total[kCtas];
     __shared__ unsigned long long s_pick_above;
     __shared__ uint32_t s_pick_bin;
@@ -126,34 +138,119 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
         }
     };
 
-    // Bound of the k-th largest: groups of `width` threads, at least k of them in this CTA.
-    const uint32_t my_key = sortable_key(vmax);
-    int width = 32;
-    while (width > 1 && kThreads / width < top_k) width >>= 1;
-    uint32_t bound = 0u;
-    if (top_k > 0 && top_k <= kThreads) {
-        const uint32_t g = warp_max_u(my_key, width);
-        bound = ~warp_max_u(~g, 32);                          // smallest of the warp's group maxima
-    }
     float m = vmax;
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-    if (lane == 0) { s_f[warp] = m; s_u[warp] = bound; }
+    if (lane == 0) s_f[warp] = m;
+    if (tid == 0) s_count = 0;
     __syncthreads();
     cluster.barrier_wait();
+    if (kFew && tid < kGroups)                                // 16 group maxima to each of 8 CTAs
+        *cluster.map_shared_rank(&s_group[rank * kWarps + tid % kWarps], tid / kWarps) = sortable_key(s_f[tid % kWarps]);
     if (tid < kCtas) {
         float cm = s_f[0];
-        uint32_t cb = s_u[0];
 #pragma unroll
-        for (int w = 1; w < kWarps; ++w) { cm = fmaxf(cm, s_f[w]); cb = min(cb, s_u[w]); }
+        for (int w = 1; w < kWarps; ++w) cm = fmaxf(cm, s_f[w]);
         *cluster.map_shared_rank(&s_peer_max[rank], tid) = cm;
-        *cluster.map_shared_rank(&s_peer_bound[rank], tid) = cb;
     }
     cluster.sync();
     m = s_peer_max[0];
-    uint32_t floor_key = s_peer_bound[0];
 #pragma unroll
-    for (int q = 1; q < kCtas; ++q) { m = fmaxf(m, s_peer_max[q]); floor_key = max(floor_key, s_peer_bound[q]); }
+    for (int q = 1; q < kCtas; ++q) m = fmaxf(m, s_peer_max[q]);
+
+    // ---- few candidates: one CTA settles the row ---------------------------------------------------
+    uint32_t floor_key = 0u;
+    bool settled = false;
+    if (kFew) {
+        if (tid < kGroups) {
+            const uint32_t mine = s_group[tid];
+            int r = 0;
+            for (int j = 0; j < kGroups; ++j) r += s_group[j] > mine || (s_group[j] == mine && j < tid);
+            if (r == top_k - 1) s_bound = mine;
+        }
+        __syncthreads();
+        floor_key = s_bound;
+        int* count = cluster.map_shared_rank(&s_count, 0);
+        float* list_x = cluster.map_shared_rank(s_list_x, 0);
+        int* list_i = cluster.map_shared_rank(s_list_i, 0);
+        for_each([&](float x, int i) {
+            if (!(x > -INFINITY) || sortable_key(x) < floor_key) return;
+            const int at = atomicAdd(count, 1);
+            if (at < kListMax) { list_x[at] = x; list_i[at] = i; }
+        });
+        cluster.sync();
+        settled = *count <= kListMax;                            // same answer in every thread of the cluster
+    }
+    float best = -INFINITY;
+    int arg = 0x7fffffff;
+    auto take = [&](float ob, int oa) {
+        if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
+    };
+    auto block_best = [&] {                                   // thread 0 ends up with the CTA's
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, s);
+            take(ob, __shfl_xor_sync(0xffffffffu, arg, s));
+        }
+        if (lane == 0) { s_f[warp] = best; s_i[warp] = arg; }
+        __syncthreads();
+        if (tid == 0)
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) take(s_f[w], s_i[w]);
+    };
+    auto finish = [&] {
+        // a row without any finite candidate (all -inf or NaN) yields id 0, never the sentinel
+        if (arg == 0x7fffffff) arg = 0;
+        out[b] = arg;
+        draws[b] += 1ull;
+        if (last_ids != nullptr) {
+            last_ids[2 * b] = last_ids[2 * b + 1];
+            last_ids[2 * b + 1] = arg;
+        }
+    };
+    if (kFew && settled) {
+        if (rank == 0) {
+            // a candidate stays when fewer than k are larger, and when what is larger and stays by count has
+            // less than the goal's mass
+            const int n = s_count;
+            const bool have = tid < n;
+            const float x = have ? s_list_x[tid] : 0.0f;
+            const uint32_t mine = have ? sortable_key(x) : 0u;
+            uint32_t* keys = s_hist;                          // [kListMax]
+            unsigned long long* mass = reinterpret_cast<unsigned long long*>(s_hist + kListMax);      // [kListMax]
+            keys[tid] = mine;
+            __syncthreads();
+            bool keep = have;
+            if (have) {
+                int larger = 0;
+                for (int j = 0; j < n; ++j) larger += keys[j] > mine;
+                keep = larger < top_k;
+            }
+            if (top_p < 1.0f) {
+                mass[tid] = keep ? mass_of(x, m) : 0ull;
+                __syncthreads();
+                if (keep) {
+                    unsigned long long total = 0ull, above = 0ull;
+                    for (int j = 0; j < n; ++j) {
+                        const unsigned long long w = mass[j];
+                        total += w;
+                        if (keys[j] > mine) above += w;
+                    }
+                    unsigned long long goal =
+                        static_cast<unsigned long long>(ceil(static_cast<double>(top_p) * static_cast<double>(total)));
+                    if (goal < 1ull) goal = 1ull;
+                    keep = above < goal;
+                }
+            }
+            const unsigned long long key = gumbel_key(seed, b, draws[b]);
+            if (keep) { best = x + gumbel_noise(key, s_list_i[tid]); arg = s_list_i[tid]; }
+            if (best == -INFINITY) arg = 0x7fffffff;
+            block_best();
+            if (tid == 0) finish();
+        }
+        cluster.sync();                                       // rank 0's count has been read by all
+        return;
+    }
 
     // ---- truncation --------------------------------------------------------------------------------
     uint32_t min_key = 0u, thr_key = 0u;                      // candidates / final set: key >= ...
@@ -179,8 +276,7 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
                     atomicAdd(&s_hist[bin], 1u);
                     return;
                 }
-                // the maximum itself weighs exactly 2^32, also when it is +inf
-                const unsigned long long w = x == m ? (1ull << 32) : __float2ull_rd(__expf(x - m) * 4294967296.0f);
+                const unsigned long long w = mass_of(x, m);
                 if (kCached) {
                     const uint32_t w_lo = static_cast<uint32_t>(w) & 0xffffu, w_hi = static_cast<uint32_t>(w >> 16);
                     if (w_lo != 0u) atomicAdd(&s_hist[bin], w_lo);
@@ -255,26 +351,13 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
 
     // ---- Gumbel-max draw within the set --------------------------------------------------------------
     const unsigned long long key = gumbel_key(seed, b, draws[b]);
-    float best = -INFINITY;
-    int arg = 0x7fffffff;
     for_each([&](float x, int i) {
         if (!(x > -INFINITY) || sortable_key(x) < thr_key) return;
         const float s = x + gumbel_noise(key, i);
         if (s > best) { best = s; arg = i; }
     });
-    auto take = [&](float ob, int oa) {
-        if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
-    };
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, s);
-        take(ob, __shfl_xor_sync(0xffffffffu, arg, s));
-    }
-    if (lane == 0) { s_f[warp] = best; s_i[warp] = arg; }
-    __syncthreads();
+    block_best();
     if (tid == 0) {
-#pragma unroll
-        for (int w = 1; w < kWarps; ++w) take(s_f[w], s_i[w]);
         *cluster.map_shared_rank(&s_peer_best[rank], 0) = best;
         *cluster.map_shared_rank(&s_peer_arg[rank], 0) = arg;
     }
@@ -282,14 +365,7 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
     if (rank == 0 && tid == 0) {
 #pragma unroll
         for (int q = 0; q < kCtas; ++q) take(s_peer_best[q], s_peer_arg[q]);
-        // a row without any finite candidate (all -inf or NaN) yields id 0, never the sentinel
-        if (arg == 0x7fffffff) arg = 0;
-        out[b] = arg;
-        draws[b] += 1ull;
-        if (last_ids != nullptr) {
-            last_ids[2 * b] = last_ids[2 * b + 1];
-            last_ids[2 * b + 1] = arg;
-        }
+        finish();
     }
 }
 
@@ -300,15 +376,17 @@ cudaError_t launch_sample_truncated(const float* logits, int64_t row_stride, int
                                     cudaStream_t stream) {
     const int per = static_cast<int>(((static_cast<int64_t>(V) + kCtas - 1) / kCtas + 3) / 4 * 4);
     const bool cached = per <= kMaxCached;
-    static bool attr_done[64] = {};
+    const bool few = top_k > 0 && top_k <= kGroups;
+    const auto kern = cached ? (few ? sample_truncated_kernel<true, true> : sample_truncated_kernel<true, false>)
+                             : (few ? sample_truncated_kernel<false, true> : sample_truncated_kernel<false, false>);
+    static bool attr_done[2][64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (cached && (dev < 0 || dev >= 64 || !attr_done[dev])) {
-        e = cudaFuncSetAttribute(sample_truncated_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kMaxCached * static_cast<int>(sizeof(float)));
+    if (cached && (dev < 0 || dev >= 64 || !attr_done[few][dev])) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxCached * static_cast<int>(sizeof(float)));
         if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr_done[dev] = true;
+        if (dev >= 0 && dev < 64) attr_done[few][dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kCtas, static_cast<unsigned>(B));
@@ -324,8 +402,7 @@ cudaError_t launch_sample_truncated(const float* logits, int64_t row_stride, int
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = gemv_tuning().use_pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, cached ? sample_truncated_kernel<true> : sample_truncated_kernel<false>, logits,
-                              row_stride, V, per, top_k, top_p, seed, draws, last_ids, out);
+    return cudaLaunchKernelEx(&cfg, kern, logits, row_stride, V, per, top_k, top_p, seed, draws, last_ids, out);
 }
 
 }  // namespace nvfp4r
