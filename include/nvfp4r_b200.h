@@ -606,10 +606,10 @@ NVFP4R_API int nvfp4r_sample(const float* logits, int64_t row_stride, int B, int
  * sampler applies them behind the processor: top-k first (the k largest logits; keys equal to the
  * k-th are all kept), then top-p on the distribution renormalised over that set (the smallest set
  * of largest probabilities whose mass reaches top_p). top_k <= 0 or >= V and top_p >= 1 switch the
- * respective truncation off; with both off this is nvfp4r_sample. The sets are found by a radix
- * descent over order-preserving keys of the logits (three levels of 2048-bin histograms of count
- * and fixed-point probability mass, integer atomics: the result does not depend on the order of
- * the additions), then the Gumbel-max draw skips everything below the threshold key.
+ * respective truncation off; with both off this is nvfp4r_sample. The sets are exact: top-k up to 128
+ * by comparing the few candidates above a bound, else by a radix descent over order-preserving keys
+ * of count or fixed-point probability mass (integer sums: the result does not depend on the order of
+ * the additions); then the Gumbel-max draw skips everything below the threshold.
  *   workspace  >= nvfp4r_sample_workspace_bytes(B) bytes, 8-byte aligned. Checked and left untouched: one
  *              launch of a thread-block cluster per row keeps the histograms in shared memory.
  * No counterpart in the reference (vLLM owns the sampler there, reset/README.md:87-88). */
