@@ -16,8 +16,8 @@
 // bf16 tokens, quantized) once per CTA into shared memory, 16 bytes per lane and two MMAs without bank conflicts. The
 // warps' sums of a tile meet in shared memory and are added in warp order: results are bit-identical run to run.
 //
-// Bound: latency of the two loads per lane and chunk with 16 warps per SM (24576x4096: 3.7 TB/s), the launch and
-// the token prologue on small weights. Measured against the ring kernel (gemv.cu) and, for K % 256 != 0, the
+// Bound: instruction issue with 16 warps per SM (61 % of the slots, conversion and f16 pipes first; waits for loads
+// are 0.7 of 6.5 stall cycles an instruction; 24576x4096: 3.7 TB/s), the launch and the token prologue on small weights. Measured against the ring kernel (gemv.cu) and, for K % 256 != 0, the
 // plain-load fallback, fp16 out, weights cold in L2, us, before -> after:
 //   7168x5120     2 tokens 10.8 -> 8.2    4 tokens 15.4 -> 8.8    8 tokens 24.7 -> 10.0
 //   640x1024      2 tokens 2.26 -> 1.67                           8 tokens 4.3 -> 1.8
