@@ -137,14 +137,24 @@ NVFP4R_API int nvfp4r_linear(const void* x, int64_t x_row_stride, int M, int K,
  *             reference kernel writes (gemm_nvfp4.cu:581, ops.py:86-88);
  *             NVFP4R_C_M_MAJOR: element (m,n) at C[m*N + n].
  * Any M >= 1 (the reference needs M % 64 == 0), N % 128 == 0, K % 256 == 0, any
- * such K (the reference has a fixed table, gemm_nvfp4.cu:633-650). Rows are taken 32
- * at a time, each pass streaming the weight once: built for decode-sized M.
+ * such K (the reference has a fixed table, gemm_nvfp4.cu:633-650). Up to 32 rows one
+ * launch streams the weight once. More rows take one launch of the many-token kernel
+ * (gemm_large.cu) where the workspace holds its partial sums, else 32 rows per launch.
  * `workspace` (>= nvfp4r_gemm_workspace_bytes(M, N, K) bytes, 16-byte aligned) holds
- * split-K partial sums and tile tickets; its first use must find it zeroed, and
- * every call leaves it zeroed again. Calls sharing a workspace must be ordered
- * on the stream. The first call on a device builds TMA descriptors on the host
- * (cuTensorMapEncodeTiled) and caches them per (pointer, shape).
+ * tile tickets and split-K partial sums. Its first NVFP4R_GEMM_TICKET_BYTES bytes (all
+ * of it, if it is smaller) must be zero before the first use, and every call leaves
+ * them zero again; the rest may hold anything. So calls of any shapes may share one
+ * workspace, of either entry point; they must be ordered on the stream. A workspace of
+ * nvfp4r_gemm_workspace_bytes keeps the partial sums clear of the tickets; a smaller one
+ * that still holds both (sized for a build that asked for less) is accepted and costs a
+ * clearing launch per call. The size is that of 32 rows; partial sums of the many-token
+ * kernel take at most 2 x SM count x 256 x 512 bytes (39 MB on 148 SMs), and a workspace
+ * without room for them runs 32 rows per launch.
+ * nvfp4r_linear_tc and the 32-row path build a TMA descriptor on the host
+ * (cuTensorMapEncodeTiled) and cache it per (pointer, shape); the many-token kernel
+ * encodes two per call.
  * ------------------------------------------------------------------------- */
+#define NVFP4R_GEMM_TICKET_BYTES 16384
 typedef enum nvfp4r_c_layout { NVFP4R_C_M_MAJOR = 0, NVFP4R_C_N_MAJOR = 1 } nvfp4r_c_layout;
 NVFP4R_API size_t nvfp4r_gemm_workspace_bytes(int M, int N, int K);
 NVFP4R_API int nvfp4r_gemm(const void* A, const void* B, const void* SFA, const void* SFB,

@@ -103,7 +103,7 @@ def linear(x: torch.Tensor, global_scale_inv: torch.Tensor, weight: torch.Tensor
 
 
 def gemm_workspace(M: int, N: int, K: int, device) -> torch.Tensor:
-    """Zero-initialised scratch for the tensor-core kernel (it leaves it zeroed)."""
+    """Zero-initialised scratch for the tensor-core kernel (which leaves its ticket area zeroed)."""
     n = L.lib().nvfp4r_gemm_workspace_bytes(M, N, K)
     return torch.zeros((n + 15) // 16 * 2, dtype=torch.int64, device=device)
 

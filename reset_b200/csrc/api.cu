@@ -274,7 +274,7 @@ static int tc_common_checks(const char* who, int M, int N, int K, int out_dtype,
     if (N % 128 != 0) return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, "tensor-core path: N must be a multiple of 128");
     if (K % 256 != 0) return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, "tensor-core path: K must be a multiple of 256");
     if (M == 0 || N == 0) return NVFP4R_OK;
-    if (!workspace || workspace_bytes < nvfp4r_gemm_workspace_bytes(M, N, K) || !aligned(workspace, 16))
+    if (!workspace || workspace_bytes < nvfp4r::gemm_workspace_min_bytes(M, N, K) || !aligned(workspace, 16))
         return fail(NVFP4R_ERR_INVALID_ARGUMENT, "tensor-core path: workspace missing, too small or misaligned");
     (void)who;
     return NVFP4R_OK;

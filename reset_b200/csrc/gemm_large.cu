@@ -112,12 +112,6 @@ quant_pack_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, int
         *reinterpret_cast<uint32_t*>(base + bn * 128 + (r >> 7) * 2048 + (b >> 2) * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4) = s4;
 }
 
-__global__ void clear_tickets_kernel(unsigned* __restrict__ tickets, int n) {
-    pdl_launch_dependents();
-    pdl_wait_prior();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) tickets[i] = 0u;
-}
-
 // ---- work of one CTA -------------------------------------------------------------------------
 struct Segment { int tile, k0, k1; };
 
@@ -682,27 +676,26 @@ cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* 
     LargePlan plan;
     if (g.xb != nullptr || g.M < (g_large_min_m ? g_large_min_m : kLargeMinM) || !plan_large(g.M, g.N, g.K, true, &plan))
         return cudaSuccess;
-    const size_t need = plan.sk_ctas ? kGemmTicketArea + plan.ticket_bytes + plan.partial_bytes : 0;
-    if (need > g.workspace_bytes) return cudaSuccess;
     LargeParams p = {};
     fill_common(plan, &p, g.out, g.M, g.N, g.K, g.alpha, g.c_n_major);
     if (!code_map(g.w, g.N, g.K, kRows, &p.map_w) || !code_map(g.a_codes, g.M, g.K, plan.bn, &p.map_x)) return cudaSuccess;
     p.wsf = static_cast<const uint8_t*>(g.wsf_swizzled);
     p.xsf = static_cast<const uint8_t*>(g.a_sf_swizzled);
-    // The workspace is shared with the decode-sized kernel, which finds its tickets in the first
-    // kGemmTicketArea bytes zeroed and leaves partial sums behind them: this launch stays behind that area
-    // and clears its own tickets first.
-    uint8_t* ws = static_cast<uint8_t*>(g.workspace) + kGemmTicketArea;
-    p.tickets = reinterpret_cast<unsigned*>(ws);
-    p.partials = reinterpret_cast<float*>(ws + plan.ticket_bytes);
+    // The workspace, tickets included, is shared with the decode-sized kernel: both leave the tickets zero.
+    GemmScratch scratch = {};
     cudaError_t e = cudaSuccess;
-    if (plan.sk_ctas) e = launch_small(clear_tickets_kernel, dim3(1), 256, stream, p.tickets, plan.tiles - plan.sk_base);
+    if (plan.sk_ctas > 0 && !gemm_scratch(g.workspace, g.workspace_bytes, plan.ticket_bytes, plan.partial_bytes, stream,
+                                          &scratch, &e))
+        return cudaSuccess;
     if (e != cudaSuccess) return e;
+    p.tickets = scratch.tickets;
+    p.partials = scratch.partials;
     static const Kern table[2][3] = {
         {gemm_large_kernel<true, 0, false>, gemm_large_kernel<true, 1, false>, gemm_large_kernel<true, 2, false>},
         {gemm_large_kernel<true, 0, true>, gemm_large_kernel<true, 1, true>, gemm_large_kernel<true, 2, true>}};
     *taken = true;
-    return launch_with_pdl(table[g.c_n_major ? 1 : 0][g.out_dtype], plan, p, stream);
+    e = launch_with_pdl(table[g.c_n_major ? 1 : 0][g.out_dtype], plan, p, stream);
+    return e == cudaSuccess ? gemm_scratch_done(scratch, stream) : e;
 }
 
 void set_large_tuning(int min_m, int bn, int stream_k) {

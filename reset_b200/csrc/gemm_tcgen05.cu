@@ -428,14 +428,59 @@ bool make_plan(int M, int N, int K, Plan* plan) {
 
 }  // namespace
 
+namespace {
+
+size_t ticket_bytes_of(int tiles) { return (static_cast<size_t>(tiles) * sizeof(unsigned) + 255) / 256 * 256; }
+size_t partial_bytes_of(const Plan& plan, int tiles) {
+    return plan.splits > 1 ? static_cast<size_t>(tiles) * plan.splits * plan.bn * kTileRows * sizeof(float) : 0;
+}
+
+// Launched without programmatic serialization: it runs behind the whole kernel before it and ahead of the next.
+__global__ void clear_kernel(uint4* __restrict__ p, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = make_uint4(0, 0, 0, 0);
+}
+
+cudaError_t clear_front(void* p, size_t bytes, cudaStream_t stream) {
+    const int n = static_cast<int>(bytes / 16);
+    if (n > 0) clear_kernel<<<(n + 1023) / 1024, 1024, 0, stream>>>(static_cast<uint4*>(p), n);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+bool gemm_scratch(void* workspace, size_t bytes, size_t ticket_bytes, size_t partial_bytes, cudaStream_t stream,
+                  GemmScratch* out, cudaError_t* err) {
+    *err = cudaSuccess;
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    const bool apart = ticket_bytes <= kGemmTicketArea && kGemmTicketArea + partial_bytes <= bytes;
+    if (!apart && ticket_bytes + partial_bytes > bytes) return false;
+    out->tickets = reinterpret_cast<unsigned*>(ws);
+    out->partials = reinterpret_cast<float*>(ws + (apart ? kGemmTicketArea : ticket_bytes));
+    out->dirty = apart ? 0 : (bytes < kGemmTicketArea ? bytes : kGemmTicketArea);
+    if (ticket_bytes > kGemmTicketArea) *err = clear_front(ws, ticket_bytes, stream);
+    return true;
+}
+
+cudaError_t gemm_scratch_done(const GemmScratch& s, cudaStream_t stream) {
+    return s.dirty ? clear_front(s.tickets, s.dirty, stream) : cudaSuccess;
+}
+
+// What a workspace needed before it had a ticket area; still accepted, one launch more per 32 rows.
+size_t gemm_workspace_min_bytes(int M, int N, int K) {
+    if (M <= 0 || N <= 0 || K <= 0 || N % kTileRows || K % kBK) return 16;
+    Plan plan;
+    if (!make_plan(M < 32 ? M : 32, N, K, &plan)) return 16;
+    const int tiles = N / kTileRows;
+    return ticket_bytes_of(tiles) + partial_bytes_of(plan, tiles) + 256;
+}
+
 size_t gemm_workspace_bytes(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0 || N % kTileRows || K % kBK) return 16;
     Plan plan;
     if (!make_plan(M < 32 ? M : 32, N, K, &plan)) return 16;
-    const size_t tiles = N / kTileRows;
-    const size_t tickets = (tiles * sizeof(unsigned) + 255) / 256 * 256;
-    const size_t partials = plan.splits > 1 ? tiles * plan.splits * plan.bn * kTileRows * sizeof(float) : 0;
-    return tickets + partials + 256;
+    const int tiles = N / kTileRows;
+    const size_t tickets = ticket_bytes_of(tiles);
+    return (tickets > kGemmTicketArea ? tickets : kGemmTicketArea) + partial_bytes_of(plan, tiles) + 256;
 }
 
 cudaError_t launch_linear_tc(const TcLinearArgs& g, cudaStream_t stream, const char** why) {
@@ -471,19 +516,19 @@ cudaError_t launch_linear_tc(const TcLinearArgs& g, cudaStream_t stream, const c
         p.splits = plan.splits;
         p.iters = g.K / kBK;
         p.stages = plan.stages;
-        // Tickets of every shape share the front of the workspace and partial sums stay behind it: a
-        // workspace that serves shapes of different N would otherwise offer one shape's partial sums
-        // as another's tickets. A workspace too small for that keeps the tight layout.
-        size_t tickets = (static_cast<size_t>(p.tiles) * sizeof(unsigned) + 255) / 256 * 256;
-        const size_t partials = plan.splits > 1 ? static_cast<size_t>(p.tiles) * plan.splits * plan.bn * kTileRows * sizeof(float) : 0;
-        if (tickets < kGemmTicketArea && kGemmTicketArea + partials <= g.workspace_bytes) tickets = kGemmTicketArea;
-        p.tickets = static_cast<unsigned*>(g.workspace);
-        p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(g.workspace) + tickets);
+        GemmScratch scratch = {};
+        cudaError_t e = cudaSuccess;
+        if (plan.splits > 1 && !gemm_scratch(g.workspace, g.workspace_bytes, ticket_bytes_of(p.tiles),
+                                             partial_bytes_of(plan, p.tiles), stream, &scratch, &e))
+            return cudaErrorInvalidValue;
+        if (e != cudaSuccess) return e;
+        p.tickets = scratch.tickets;
+        p.partials = scratch.partials;
 
         void (*kern)(TcParams) = plan.bn == 16 ? linear_tc_kernel<16> : linear_tc_kernel<32>;
         static bool attr_done[2][64] = {};
         int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
+        e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
         const int ki = plan.bn == 16 ? 0 : 1;
         if (dev >= 0 && dev < 64 && !attr_done[ki][dev]) {
@@ -502,6 +547,7 @@ cudaError_t launch_linear_tc(const TcLinearArgs& g, cudaStream_t stream, const c
         cfg.attrs = attr;
         cfg.numAttrs = gemv_tuning().use_pdl ? 1 : 0;
         e = cudaLaunchKernelEx(&cfg, kern, p);
+        if (e == cudaSuccess) e = gemm_scratch_done(scratch, stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -81,9 +81,20 @@ struct GemvTuning {
 GemvTuning& gemv_tuning();
 
 // ---- gemm_tcgen05.cu ------------------------------------------------------
-// Front part of a gemm workspace that only ever holds tile tickets (zero between launches), wherever
-// the workspace is large enough to keep the partial sums of every shape behind it.
-constexpr size_t kGemmTicketArea = 4096;
+// Front part of a gemm workspace: the tile tickets of every launch, zero between launches. It covers 4096 row
+// tiles (N up to 524288, twice the widest vocabulary in use). Partial sums lie behind it; a launch that cannot
+// keep them there (smaller workspace, wider weight) clears the area again.
+constexpr size_t kGemmTicketArea = NVFP4R_GEMM_TICKET_BYTES;
+// Where the tickets and the partial sums of one launch lie in the caller's workspace.
+struct GemmScratch {
+    unsigned* tickets;
+    float* partials;
+    size_t dirty;        // bytes of the ticket area to be cleared behind the launch (0: partial sums stay clear of it)
+};
+// False: the workspace is too small. Clears the tickets first where they reach past the area.
+bool gemm_scratch(void* workspace, size_t bytes, size_t ticket_bytes, size_t partial_bytes, cudaStream_t stream,
+                  GemmScratch* out, cudaError_t* err);
+cudaError_t gemm_scratch_done(const GemmScratch& s, cudaStream_t stream);
 // One NVFP4 weight [N,K/2] (+ swizzled scales) against M activation rows, either
 // bf16 rows quantized on the fly (xb) or pre-quantized codes + swizzled scales.
 struct TcLinearArgs {
@@ -104,6 +115,7 @@ struct TcLinearArgs {
     size_t workspace_bytes;
 };
 size_t gemm_workspace_bytes(int M, int N, int K);
+size_t gemm_workspace_min_bytes(int M, int N, int K);     // the smallest that is accepted
 // `*why` is set (and cudaSuccess returned) when the shape is outside what the
 // kernel handles.
 cudaError_t launch_linear_tc(const TcLinearArgs& g, cudaStream_t stream, const char** why);

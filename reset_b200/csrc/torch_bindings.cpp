@@ -103,7 +103,8 @@ at::Tensor& fixed_workspace(int kind, const at::Device& dev, size_t bytes, const
         TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None, who,
                     ": the first call on a device allocates the operator's scratch; make it before "
                     "capturing a CUDA graph");
-        t = at::zeros({static_cast<int64_t>(workspace_capacity())},
+        // kind 0: the ticket area on top of the capacity, which counts partial sums
+        t = at::zeros({static_cast<int64_t>(workspace_capacity() + (kind == 0 ? NVFP4R_GEMM_TICKET_BYTES : 0))},
                       at::TensorOptions().device(dev).dtype(at::kByte));
     }
     TORCH_CHECK(bytes <= static_cast<size_t>(t.nbytes()), who, ": this shape needs ", bytes,

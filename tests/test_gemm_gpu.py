@@ -174,3 +174,74 @@ def test_one_workspace_serves_every_shape(capi):
         C = torch.full((4, N), float("nan"), dtype=torch.float32, device="cuda")
         capi.gemm(cuda(xc), wd, cuda(onv.swizzle_blockscale(xsf)), wsd, C, 1.0, wksp, n_major=False)
         assert rel_l2(C.cpu().numpy(), onv.linear_f64(w, ws, xc, xsf)) <= 1e-5
+
+
+_PERIOD = 4096
+
+
+@pytest.fixture(scope="module")
+def wide_weights(capi):
+    """{N: operands}: the rows of one 4096-row weight repeated down to N, so that the oracle computes 4096 of them."""
+    def tiled(t, N):
+        return t.repeat((N + _PERIOD - 1) // _PERIOD, 1)[:N].contiguous()
+    out = {}
+    for N, K in ((4096, 8192), (151936, 4096), (200064, 8192)):
+        w, ws = onv.random_nvfp4((_PERIOD,), K, seed=K)
+        wd, wsd = tiled(cuda(w), N), capi.swizzle_blockscale(tiled(cuda(ws), N))
+        xb = make_activation(64, K, seed=31)
+        xc, xsf = onv.quantize_nvfp4(xb.float().numpy(), 48.0)
+        out[N] = (K, wd, wsd, xb.cuda(), cuda(xc), xsf, cuda(onv.linear_f64(w, ws, xc, xsf)))
+    yield out
+    out.clear()
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("size", ["ample", "queried", "tight"])
+def test_one_workspace_many_and_few_tokens_wide_and_narrow(capi, wide_weights, size):
+    """Every order of a narrow weight, a 151936-row and a 200064-row vocabulary, 64 tokens and then 4, `gemm` and
+    `linear_tc`: whatever a call leaves behind, the next finds its tickets zero. Also on a workspace of exactly the
+    queried size, and on one of tickets + partial sums + 256 bytes, the least that is accepted."""
+    from itertools import permutations
+    from reset_b200 import _lib
+    need = max(_lib.lib().nvfp4r_gemm_workspace_bytes(M, N, wide_weights[N][0]) for N in wide_weights for M in (4, 64))
+    if size == "tight":
+        need -= 16384 - (max(wide_weights) // 128 * 4 + 255) // 256 * 256
+    wksp = torch.zeros({"ample": 128 << 20}.get(size, need), dtype=torch.uint8, device="cuda")
+    gs = torch.tensor([48.0], device="cuda")
+    for order in permutations(wide_weights):
+        for N in order:
+            K, wd, wsd, xb, xc, xsf, exact = wide_weights[N]
+            for M in (64, 4):
+                C = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+                capi.gemm(xc[:M], wd, cuda(onv.swizzle_blockscale(xsf[:M])), wsd, C, 1.0, wksp, n_major=False)
+                for got in (C, capi.linear_tc(xb[:M], gs, wd, wsd, 1.0, wksp, out_dtype=torch.float32)):
+                    assert not torch.isnan(got).any(), (order, N, M)
+                    want = exact[:M].repeat(1, N // _PERIOD + 1)[:, :N]
+                    err = (got.double() - want).square().view(M, -1, 128).sum((0, 2))      # per 128-row tile
+                    ref = want.square().view(M, -1, 128).sum((0, 2))
+                    assert (err / ref).max().sqrt() <= 1e-5, (order, N, M)
+    assert not wksp[:16384].any()
+
+
+def test_more_tiles_than_the_ticket_area_holds(capi, wide_weights):
+    """540672 rows have 4224 tickets: they are cleared before the launch and the area behind it."""
+    from reset_b200 import _lib
+    N, K, M = 540672, 512, 4
+    w, ws = onv.random_nvfp4((_PERIOD,), K, seed=8)
+    wd, wsd = cuda(w).repeat(N // _PERIOD, 1), capi.swizzle_blockscale(cuda(ws).repeat(N // _PERIOD, 1))
+    xc, xsf = onv.random_nvfp4((M,), K, seed=9)
+    exact = cuda(onv.linear_f64(w, ws, xc, xsf))
+    wksp = torch.zeros(80 << 20, dtype=torch.uint8, device="cuda")
+    wksp[16384:] = 0x41                                        # what partial sums of other shapes leave behind
+    for _ in range(2):
+        _lib.check(_lib.lib().nvfp4r_set_gemm_tuning(2, 0), "tuning")
+        C = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+        capi.gemm(cuda(xc), wd, cuda(onv.swizzle_blockscale(xsf)), wsd, C, 1.0, wksp, n_major=False)
+        err = (C.double() - exact.repeat(1, N // _PERIOD)).square().view(M, -1, 128).sum((0, 2))
+        assert (err / exact.square().view(M, -1, 128).sum((0, 2)).repeat(N // _PERIOD)).max().sqrt() <= 1e-5
+        assert not wksp[:16384].any()
+        _lib.lib().nvfp4r_set_gemm_tuning(0, 0)
+        K1, wd1, wsd1, _, xc1, xsf1, exact1 = wide_weights[4096]
+        C = torch.full((M, 4096), float("nan"), dtype=torch.float32, device="cuda")
+        capi.gemm(xc1[:M], wd1, cuda(onv.swizzle_blockscale(xsf1[:M])), wsd1, C, 1.0, wksp, n_major=False)
+        assert rel_l2(C.cpu().numpy(), exact1[:M].cpu().numpy()) <= 1e-5
