@@ -525,8 +525,8 @@ bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
     const int mt0 = (M + 255) / 256;
     for (int mt = mt0; mt <= mt0 + 4; ++mt) {
         int bn = ((M + mt - 1) / mt + 15) / 16 * 16;
-        if (row_major && mt > 1) bn = (bn + 127) / 128 * 128;     // a tile starts at a scale chunk
         if (g_large_bn) bn = g_large_bn;
+        if (row_major && M > bn) bn = (bn + 127) / 128 * 128;     // a tile starts at a scale chunk
         if (bn > 256) continue;
         const int tiles_m = (M + bn - 1) / bn;
         const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;

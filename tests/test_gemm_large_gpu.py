@@ -122,6 +122,20 @@ def test_gemm_row_major(capi, M, N, K, bn, sk, n_major, dtype):
     assert rel_l2(got, exact) <= {torch.float32: 1e-5, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
 
 
+@pytest.mark.parametrize("M,bn", [(130, 64), (130, 16), (257, 112), (257, 176), (520, 64)])
+def test_gemm_row_major_tiles_start_at_a_scale_chunk(capi, M, bn):
+    """Row-major token scales are addressed in chunks of 128 rows: with more than one tile a width asked for by
+    tuning is rounded up to that, for a tile may neither read another tile's scales nor past the last chunk."""
+    _tune(0, bn, 0)
+    N, K = 256, 512
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + bn)
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    C = torch.full((M, N), float("nan"), device="cuda")
+    wksp = torch.zeros(16 << 20, dtype=torch.uint8, device="cuda")
+    capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=False)
+    assert rel_l2(C.cpu().numpy(), exact) <= 1e-5
+
+
 def test_gemm_output_of_any_alignment(capi):
     """A 2-byte aligned output takes the narrow stores."""
     M, N, K = 48, 256, 512
