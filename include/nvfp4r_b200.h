@@ -214,11 +214,18 @@ NVFP4R_API int nvfp4r_linear_packed(const void* x, int64_t x_row_stride, int M, 
  *   nvfp4r_linear_packed_scratch_bytes   bytes of scratch, or 0 where nvfp4r_linear_packed is the
  *                                        faster kernel (few tokens) or the shape is unsupported:
  *                                        call that one then
+ *   nvfp4r_linear_packed_route           which of the two entry points is the faster one: _PACKED, _SCRATCH, or
+ *                                        _SCRATCH_CAPTURED where this one needs less device time, but a
+ *                                        call that launches its two kernels and allocates the scratch
+ *                                        each time needs more (up to 32 tokens). The torch operator asks;
+ *                                        a C program that keeps its scratch can go by the bytes alone
  *   nvfp4r_linear_packed_scratch         scratch >= that many bytes, 16-byte aligned, any contents; not
  *                                        kept after the launch
  * Same operands, arithmetic and rcp_mode meaning; the weight must be final before the preceding
  * kernel of the stream is launched. */
 NVFP4R_API size_t nvfp4r_linear_packed_scratch_bytes(int M, int N, int K);
+typedef enum nvfp4r_route { NVFP4R_ROUTE_PACKED = 0, NVFP4R_ROUTE_SCRATCH_CAPTURED = 1, NVFP4R_ROUTE_SCRATCH = 2 } nvfp4r_route;
+NVFP4R_API int nvfp4r_linear_packed_route(int M, int N, int K);
 NVFP4R_API int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride, int M, int K,
                                             const float* global_scale_inv, const void* packed, int N,
                                             float alpha, void* out, int out_dtype, int rcp_mode,

@@ -75,6 +75,7 @@ PROTOTYPES = {
     "nvfp4r_pack_weight": (_i, [_vp, _vp, _vp, _i, _i, _vp]),
     "nvfp4r_linear_packed": (_i, [_vp, _i64, _i, _i, _vp, _vp, _i, _f, _vp, _i, _i, _vp, _sz, _vp]),
     "nvfp4r_linear_packed_scratch_bytes": (_sz, [_i, _i, _i]),
+    "nvfp4r_linear_packed_route": (_i, [_i, _i, _i]),
     "nvfp4r_linear_packed_scratch": (_i, [_vp, _i64, _i, _i, _vp, _vp, _i, _f, _vp, _i, _i, _vp, _sz, _vp]),
     "nvfp4r_set_gemm_large_tuning": (_i, [_i, _i, _i]),
     "nvfp4r_linear_packed_ex": (_i, [C.POINTER(Prologue), _vp, _i64, _i, _i, _vp, _vp, _i, _f, _vp, _i, _i,

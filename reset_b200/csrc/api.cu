@@ -388,6 +388,7 @@ int nvfp4r_linear_packed(const void* x, int64_t x_row_stride, int M, int K, cons
 }
 
 size_t nvfp4r_linear_packed_scratch_bytes(int M, int N, int K) { return nvfp4r::large_scratch_bytes(M, N, K); }
+int nvfp4r_linear_packed_route(int M, int N, int K) { return nvfp4r::large_route(M, N, K); }
 
 int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride, int M, int K, const float* gs,
                                  const void* packed, int N, float alpha, void* out, int out_dtype, int rcp_mode,

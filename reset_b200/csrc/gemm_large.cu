@@ -35,6 +35,7 @@
 // 24.7 us (left: 32 tokens per pass).
 #include <cuda.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "kernels.h"
@@ -516,9 +517,8 @@ struct LargePlan {
 
 int g_large_bn = 0, g_large_sk = -1, g_large_min_m = 0;
 
-// Tile width and schedule by an estimate of the time in nanoseconds.
-bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
-    const int G = device_sm_count();
+// Tile width and schedule by an estimate of the time in nanoseconds, for G SMs.
+bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan) {
     const int kblocks = (K + kBK - 1) / kBK, tiles_n = N / kRows;
     double best = 1e30;
     bool found = false;
@@ -574,12 +574,40 @@ bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
     return true;
 }
 
+// A call asks three times (scratch size, its check, launch) and plans once: 0.3 us each.
+bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
+    struct Last { int M, N, K, G, bn, sk; bool row_major, found; LargePlan plan; };
+    static thread_local Last last = {};
+    const int G = device_sm_count();
+    if (last.M != M || last.N != N || last.K != K || last.G != G || last.bn != g_large_bn || last.sk != g_large_sk ||
+        last.row_major != row_major) {
+        last = Last{M, N, K, G, g_large_bn, g_large_sk, row_major, false, {}};
+        last.found = make_large_plan(M, N, K, row_major, G, &last.plan);
+    }
+    *plan = last.plan;
+    return last.found;
+}
+
 using Kern = void (*)(LargeParams);
 
-cudaError_t launch_with_pdl(Kern kern, const LargePlan& plan, const LargeParams& p, cudaStream_t stream) {
-    // per device, and only ever raised to the same value: a second thread repeats a harmless call
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
+constexpr int kInstances = 9;
+
+cudaError_t launch_with_pdl(int instance, const LargePlan& plan, const LargeParams& p, cudaStream_t stream) {
+    // packed operands, then row-major ones with M-major and with N-major output; bf16, fp16, fp32
+    static const Kern table[kInstances] = {
+        gemm_large_kernel<false, 0, false>, gemm_large_kernel<false, 1, false>, gemm_large_kernel<false, 2, false>,
+        gemm_large_kernel<true, 0, false>, gemm_large_kernel<true, 1, false>, gemm_large_kernel<true, 2, false>,
+        gemm_large_kernel<true, 0, true>, gemm_large_kernel<true, 1, true>, gemm_large_kernel<true, 2, true>};
+    const Kern kern = table[instance];
+    static std::atomic<bool> attr_done[kInstances][64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !attr_done[instance][dev].load(std::memory_order_relaxed)) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) attr_done[instance][dev].store(true, std::memory_order_relaxed);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(plan.grid));
     cfg.blockDim = dim3(kThreadsL);
@@ -627,26 +655,47 @@ void fill_common(const LargePlan& plan, LargeParams* p, void* out, int M, int N,
 // Tokens from which the row-major operands of the raw gemm operator take this path.
 constexpr int kLargeMinM = 33;
 
-// Tokens from which the packed linear takes it, where the caller can give it scratch. Up to 16 tokens the decode kernel
-// makes one pass over the weight as well and needs no second launch; its CTAs each quantize the tokens of their
-// K part, which grows with the tokens, while this path pays a few us for partial sums where the weight has few
-// row tiles and long rows. Measured, us, decode kernel / this one:
-//   N >= 6 K       34816x5120: 12 tokens 22.0 / 21.8, 16 tokens 26.4 / 21.5; 12288x2048: 13 tokens 8.2 / 6.4;
+// Tokens from which the packed linear takes it, where the caller can give it scratch: the device's side of the
+// choice. Up to 16 tokens the decode kernel makes one pass over the weight as well and needs no second launch; its
+// CTAs each quantize the tokens of their K part, which grows with the tokens, while this path pays a few us for
+// partial sums where the weight has few row tiles and long rows. Measured in CUDA graphs, us, decode kernel / this one:
+//   N >= 6 K       34816x5120: 13 tokens 25.6 / 21.3, 16 tokens 26.4 / 21.5; 12288x2048: 13 tokens 8.2 / 6.4;
 //                  but (N >= 16 K) 24576x1024: 13 tokens 6.1 / 6.8, 17 tokens 8.1 / 6.9
-//   N >= 1.5 K     24576x4096: 16 tokens 17.8 / 17.8, 17 tokens 27.0 / 18.0; 10240x5120: 17 tokens 15.9 / 11.6;
-//                  6144x4096: 17 tokens 10.0 / 9.7
-//   N >= K         4096x4096: 24 tokens 9.2 / 9.4, 32 tokens 11.3 / 9.5
+//   N >= 1.5 K     12288x4096: 17 tokens 15.3 / 10.5; 10240x5120: 17 tokens 15.9 / 11.6; 6144x4096: 17 tokens 10.0 / 9.7
+//   N >= K         4096x4096: 25 tokens 9.9 / 9.4, 32 tokens 11.3 / 9.5
 //   below          4096x12288: 24 tokens 13.2 / 15.7, 32 tokens 15.7 / 15.7; 1280x5120: 32 tokens 9.6 / 11.2
 int large_min_m(int N, int K) {
     const int64_t n = N, k = K;
     return n >= 6 * k && n < 16 * k ? 13 : 2 * n >= 3 * k ? 17 : n >= k ? 25 : kLargeMinM;
 }
 
+bool large_pays(int M, int N, int K) {
+    if (g_large_min_m) return M >= g_large_min_m;
+    if (M < large_min_m(N, K)) return false;
+    const int G = device_sm_count(), tiles = N / kRows;
+    // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two full rounds of
+    // 0.48 us a K block. 20480x2048: 13 tokens 8.9 / 10.7, 16 tokens 9.8 / 10.8; 24576x4096: 16 tokens 17.4 / 18.5;
+    // but 24064x2304, where the decode kernel splits K: 16 tokens 15.3 / 11.5; 22528x3072: 16 tokens 16.4 / 15.1.
+    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 3.9 + 0.96 * ((K + kBK - 1) / kBK);
+    return true;
+}
+
 size_t large_scratch_bytes(int M, int N, int K) {
     LargePlan plan;
-    if (M < (g_large_min_m ? g_large_min_m : large_min_m(N, K)) || N <= 0 || K <= 0 || N % kRows || K % 128) return 0;
+    if (N <= 0 || K <= 0 || N % kRows || K % 128 || !large_pays(M, N, K)) return 0;
     if (!plan_large(M, N, K, false, &plan)) return 0;
     return plan.token_bytes + plan.ticket_bytes + plan.partial_bytes;
+}
+
+// The host's side: a second launch and the scratch bring a call to 12 us or more even where the device needs 5, while
+// a call of the decode kernel ends at 8.5. So up to 32 tokens (one launch of it) that kernel keeps what it does in
+// less. Measured, us a call: 6144x1024, 16 tokens 8.5 / 12.0; 12288x2048, 16 tokens 8.9 / 12.0; 4096x4096, 32 tokens
+// 11.4 / 12.2; 6144x2048, 32 tokens 13.1 / 12.2; 8192x3072, 20 tokens 13.0 / 12.1.
+constexpr double kLargeCallUs = 12.0;
+
+int large_route(int M, int N, int K) {
+    if (N <= 0 || K <= 0 || N % kRows || K % 128 || !large_pays(M, N, K)) return NVFP4R_ROUTE_PACKED;
+    return g_large_min_m || M > 32 || packed_time_us(M, N, K) >= kLargeCallUs ? NVFP4R_ROUTE_SCRATCH : NVFP4R_ROUTE_SCRATCH_CAPTURED;
 }
 
 cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaStream_t stream) {
@@ -664,9 +713,7 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
                                  g.K, g.gs, g.rcp_mode == kRcpExact, tokens, plan.bn, plan.nch, plan.kblocks,
                                  p.tickets, plan.tiles - plan.sk_base);
     if (e != cudaSuccess) return e;
-    static const Kern table[3] = {gemm_large_kernel<false, 0, false>, gemm_large_kernel<false, 1, false>,
-                                  gemm_large_kernel<false, 2, false>};
-    return launch_with_pdl(table[g.out_dtype], plan, p, stream);
+    return launch_with_pdl(g.out_dtype, plan, p, stream);
 }
 
 // The raw operator on row-major operands. *taken stays false (nothing launched) where the workspace
@@ -690,11 +737,8 @@ cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* 
     if (e != cudaSuccess) return e;
     p.tickets = scratch.tickets;
     p.partials = scratch.partials;
-    static const Kern table[2][3] = {
-        {gemm_large_kernel<true, 0, false>, gemm_large_kernel<true, 1, false>, gemm_large_kernel<true, 2, false>},
-        {gemm_large_kernel<true, 0, true>, gemm_large_kernel<true, 1, true>, gemm_large_kernel<true, 2, true>}};
     *taken = true;
-    e = launch_with_pdl(table[g.c_n_major ? 1 : 0][g.out_dtype], plan, p, stream);
+    e = launch_with_pdl((g.c_n_major ? 6 : 3) + g.out_dtype, plan, p, stream);
     return e == cudaSuccess ? gemm_scratch_done(scratch, stream) : e;
 }
 

@@ -147,6 +147,7 @@ struct PackedLinearArgs {
     bool push_gather;            // finish the all-reduce inside the launch (see nvfp4r_prologue)
 };
 size_t packed_weight_bytes(int N, int K);
+double packed_time_us(int M, int N, int K);      // estimated device time of launch_linear_packed
 size_t packed_workspace_bytes(int M, int N, int K);
 cudaError_t launch_pack_weight(const void* w, const void* sf_flat, void* packed, int N, int K,
                                cudaStream_t stream);
@@ -160,6 +161,7 @@ cudaError_t read_packed_trace(unsigned long long* out16);
 // ---- gemm_large.cu --------------------------------------------------------
 // Scratch of the many-token linear over a packed weight; 0: launch_linear_packed is to be used.
 size_t large_scratch_bytes(int M, int N, int K);
+int large_route(int M, int N, int K);             // NVFP4R_ROUTE_*
 cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaStream_t stream);
 // *taken = false: nothing was launched, launch_linear_tc is to be used.
 cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* taken);

@@ -257,8 +257,12 @@ at::Tensor linear_packed_op(const at::Tensor& x, const at::Tensor& global_scale_
     auto out = at::empty({M, N}, x.options().dtype(dt));
     // many tokens: quantized once into scratch of this call (the caching allocator's, so capture and
     // streams are its business), one launch for all of them
-    const size_t scratch_bytes = nvfp4r_linear_packed_scratch_bytes(static_cast<int>(M), static_cast<int>(N),
-                                                                    static_cast<int>(K));
+    const int route = nvfp4r_linear_packed_route(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K));
+    size_t scratch_bytes = 0;
+    if (route == NVFP4R_ROUTE_SCRATCH ||
+        (route == NVFP4R_ROUTE_SCRATCH_CAPTURED &&
+         c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None))
+        scratch_bytes = nvfp4r_linear_packed_scratch_bytes(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K));
     if (scratch_bytes > 0) {
         auto scratch = at::empty({static_cast<int64_t>(scratch_bytes)}, x.options().dtype(at::kByte));
         check_status(nvfp4r_linear_packed_scratch(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),

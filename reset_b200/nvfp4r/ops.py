@@ -8,6 +8,8 @@ from typing import Optional
 
 import torch
 
+from . import _config
+
 
 def _ensure_3d(t: torch.Tensor, name: str) -> torch.Tensor:
     if t.dim() == 3:
@@ -70,7 +72,6 @@ def linear_packed(x: torch.Tensor, global_scale_inv: torch.Tensor, packed: torch
 
 def use_gemv(M: int, N: int, K: int, gemv_max_m: int) -> bool:
     """The measured crossover: True when the CUDA-core GEMV is the faster path."""
-    from . import _config
     if M > gemv_max_m or M not in _config.GEMV_MAX_WEIGHT_BYTES:
         return False
     if K % 32 or K < _config.GEMV_MIN_K:
@@ -115,7 +116,6 @@ def linear_auto(x, global_scale_inv, weight, weight_scale_flat, packed, N: int, 
     ``reduce`` (a ``reset_b200.comm.PeerAllReduce``) makes this a row-parallel linear of a
     tensor-parallel layer: the result is summed over the ranks, with the first half of the
     exchange running in the tensor-core kernel's epilogue where that kernel is chosen."""
-    from . import _config
     M, K = x.shape
     gemv = packed is None or (weight is not None and use_gemv(M, N, K, _config.GEMV_MAX_M))
     if reduce is not None and reduce.world > 1:

@@ -204,3 +204,18 @@ def test_reciprocals_the_packed_linear_divides_with_are_exact():
     for blocks in range(16, 129, 16):
         inv = ((1 << 20) + blocks - 1) // blocks
         assert all((i * inv) >> 20 == i // blocks for i in range(32 * 128 + 3 * 192 + 1))
+
+
+# M, N, K: the kernel that a captured call / an eager call of the packed linear takes. 1: the many-token kernel. The
+# measured times of both (us; device, whole call) are in the comments of gemm_large.cu.
+@pytest.mark.parametrize("M,N,K,device,call", [
+    (16, 6144, 1024, 1, 0), (13, 12288, 2048, 1, 0), (32, 1024, 1024, 1, 0), (17, 3072, 1024, 1, 0), (24, 16384, 1024, 1, 0),
+    (25, 4096, 4096, 1, 0), (16, 24576, 1024, 0, 0), (17, 24576, 1024, 1, 0), (13, 20480, 2048, 0, 0), (16, 20480, 2048, 0, 0),
+    (13, 24576, 4096, 0, 0), (16, 24576, 4096, 0, 0), (16, 24064, 2304, 1, 1), (16, 34816, 5120, 1, 1), (13, 34816, 5120, 1, 1), (32, 6144, 2048, 1, 1),
+    (20, 8192, 3072, 1, 1), (17, 10240, 5120, 1, 1), (32, 4096, 12288, 0, 1), (33, 1024, 1024, 1, 1), (45, 10240, 5120, 1, 1),
+])
+def test_kernel_of_a_packed_linear_of_13_to_33_tokens(M, N, K, device, call):
+    from reset_b200 import _lib
+    lib = _lib.lib()
+    assert (lib.nvfp4r_linear_packed_scratch_bytes(M, N, K) > 0) == bool(device)
+    assert lib.nvfp4r_linear_packed_route(M, N, K) == (0 if not device else 1 + call)

@@ -171,3 +171,20 @@ def test_linear_packed_under_capture(capi):
         out.zero_()
         g.replay()
         assert rel_l2(out.cpu().numpy(), exact) <= 1e-5
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 6144, 1024), (32, 1024, 1024), (17, 3072, 1024), (16, 34816, 1024), (32, 8192, 4096)])
+def test_eager_and_captured_calls_give_the_same_product(capi, M, N, K):
+    """Up to 32 tokens an eager call may take the decode kernel where a captured one takes this one: the operator's
+    result is the oracle's either way."""
+    from reset_b200 import _lib
+    assert _lib.lib().nvfp4r_linear_packed_scratch_bytes(M, N, K) > 0 or N >= 16 * K
+    w, ws, xb, gs, exact = _case(M, N, K, seed=N % 89)
+    packed, x = capi.pack_weight(cuda(w), cuda(ws)), xb.cuda()
+    eager = torch.ops.nvfp4r.linear_packed(x, gs, packed, N, 0.5, F32, 0)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = torch.ops.nvfp4r.linear_packed(x, gs, packed, N, 0.5, F32, 0)
+    g.replay()
+    for got in (eager, out):
+        assert rel_l2(got.cpu().numpy(), exact) <= 1e-5
