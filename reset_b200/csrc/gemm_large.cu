@@ -672,11 +672,16 @@ int large_min_m(int N, int K) {
 bool large_pays(int M, int N, int K) {
     if (g_large_min_m) return M >= g_large_min_m;
     if (M < large_min_m(N, K)) return false;
-    const int G = device_sm_count(), tiles = N / kRows;
+    const int G = device_sm_count(), tiles = N / kRows, kblocks = (K + kBK - 1) / kBK;
+    // A narrow weight with rows of 31 or 32 K blocks: the longest that still run as whole tiles here (0.48 us a
+    // block), while two launches of the decode kernel give each CTA one block and one token to add up. 33 / 48 / 64
+    // tokens: 640x8192 13.0 / 14.0 / 14.3, here 15.5 / 15.7 / 15.9; 1280x8192 14.3 / 15.5 / 18.6, here 16.0 / 15.9 / 16.2;
+    // 30 blocks, 1024x7680: 14.9 / 16.0 / 17.4, here 14.8 / 14.8 / 15.0; 33, 1792x8320: 17.2 / 18.4 / 22.4, here 16.8.
+    if (M <= 64 && kblocks > 30 && kblocks <= 32 && tiles <= (M <= 48 ? 16 : 8)) return false;
     // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two full rounds of
     // 0.48 us a K block. 20480x2048: 13 tokens 8.9 / 10.7, 16 tokens 9.8 / 10.8; 24576x4096: 16 tokens 17.4 / 18.5;
     // but 24064x2304, where the decode kernel splits K: 16 tokens 15.3 / 11.5; 22528x3072: 16 tokens 16.4 / 15.1.
-    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 3.9 + 0.96 * ((K + kBK - 1) / kBK);
+    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 3.9 + 0.96 * kblocks;
     return true;
 }
 

@@ -213,8 +213,10 @@ def test_reciprocals_the_packed_linear_divides_with_are_exact():
     (25, 4096, 4096, 1, 0), (16, 24576, 1024, 0, 0), (17, 24576, 1024, 1, 0), (13, 20480, 2048, 0, 0), (16, 20480, 2048, 0, 0),
     (13, 24576, 4096, 0, 0), (16, 24576, 4096, 0, 0), (16, 24064, 2304, 1, 1), (16, 34816, 5120, 1, 1), (13, 34816, 5120, 1, 1), (32, 6144, 2048, 1, 1),
     (20, 8192, 3072, 1, 1), (17, 10240, 5120, 1, 1), (32, 4096, 12288, 0, 1), (33, 1024, 1024, 1, 1), (45, 10240, 5120, 1, 1),
+    (64, 640, 8192, 0, 0), (33, 1280, 7808, 0, 0), (48, 2048, 8192, 0, 0), (64, 1280, 8192, 1, 1), (33, 1024, 7680, 1, 1),
+    (33, 1792, 8320, 1, 1), (65, 640, 8192, 1, 1), (33, 2560, 8192, 1, 1),
 ])
-def test_kernel_of_a_packed_linear_of_13_to_33_tokens(M, N, K, device, call):
+def test_kernel_of_a_packed_linear_of_13_to_65_tokens(M, N, K, device, call):
     from reset_b200 import _lib
     lib = _lib.lib()
     assert (lib.nvfp4r_linear_packed_scratch_bytes(M, N, K) > 0) == bool(device)
