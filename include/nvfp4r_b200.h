@@ -480,7 +480,7 @@ NVFP4R_API int nvfp4r_entropy(const float* logits, int64_t row_stride, int B, in
  * ------------------------------------------------------------------------- */
 NVFP4R_API int nvfp4r_set_gemv_tuning(int ctas_per_sm, int use_pdl, int force_generic);
 
-/* Tuning of the register-resident GEMV that takes launches of one or two tokens (same
+/* Tuning of the register-resident GEMV that takes launches of one token (same
  * standing as the call above: the reference's counterpart is its NVFP4R_GEMV_* environment,
  * kernels/cuda/gemv/gemv_nvfp4.cu:870-948).
  *   mode           0 = automatic (default), 1 = whenever the arguments allow it, -1 = never
@@ -491,6 +491,10 @@ NVFP4R_API int nvfp4r_set_gemv_tuning(int ctas_per_sm, int use_pdl, int force_ge
  *                  1..12 = one half, 13..32 = both
  */
 NVFP4R_API int nvfp4r_set_gemv_rows_tuning(int mode, int rows_per_step, int warps_per_sm);
+
+/* Tuning of the GEMV for two to eight tokens on mma.sync: 0 = wherever the arguments allow it (default), -1 = never:
+ * the ring and plain-load kernels take those launches. */
+NVFP4R_API int nvfp4r_set_gemv_mma_tuning(int mode);
 
 /* ------------------------------------------------------------------------- *
  * One-shot all-reduce (sum) of a small bf16 tensor over NVLink peer memory: the exchange

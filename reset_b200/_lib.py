@@ -99,6 +99,7 @@ PROTOTYPES = {
     "nvfp4r_status_mirror": (_i, [C.POINTER(C.POINTER(C.c_int))]),
     "nvfp4r_set_gemv_tuning": (_i, [_i, _i, _i]),
     "nvfp4r_set_gemv_rows_tuning": (_i, [_i, _i, _i]),
+    "nvfp4r_set_gemv_mma_tuning": (_i, [_i]),
     "nvfp4r_add_rmsnorm": (_i, [_vp, _vp, _vp, _vp, _i, _i, _f, _vp]),
     "nvfp4r_qk_norm_rope_kv": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _vp]),
     "nvfp4r_attn_decode_workspace_bytes": (_sz, [_i, _i]),

@@ -723,6 +723,12 @@ int nvfp4r_set_gemv_rows_tuning(int mode, int rows_per_step, int warps_per_sm) {
     return NVFP4R_OK;
 }
 
+int nvfp4r_set_gemv_mma_tuning(int mode) {
+    if (mode < -1 || mode > 0) return fail(NVFP4R_ERR_INVALID_ARGUMENT, "mma tuning: mode is -1 or 0");
+    nvfp4r::gemv_tuning().no_mma = mode < 0 ? 1 : 0;
+    return NVFP4R_OK;
+}
+
 int nvfp4r_status_mirror(volatile int** host_word) {
     if (!host_word) return fail(NVFP4R_ERR_INVALID_ARGUMENT, "status_mirror: null pointer");
     static int* host_ptr[64] = {};

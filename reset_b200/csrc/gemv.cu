@@ -455,7 +455,7 @@ cudaError_t read_and_clear_device_status(int* flag) {
 cudaError_t set_status_mirror_gemv(int* p) { return set_status_mirror_here(p); }
 
 GemvTuning& gemv_tuning() {
-    static GemvTuning t = {0, 1, 0};
+    static GemvTuning t = {0, 1, 0, 0};
     return t;
 }
 

@@ -419,7 +419,7 @@ cudaError_t launch_gemv_auto(const GemvArgs& a, cudaStream_t stream) {
         return (a.pro_kind == 0 && gemv_stream_supported(a)) ? launch_gemv_stream(a, stream) : cudaErrorNotSupported;
     if (a.pro_kind != 0)         // fused prologues exist in the register-resident kernel only
         return gemv_rows_supported(a) ? launch_gemv_rows(a, stream) : cudaErrorNotSupported;
-    if (!gemv_tuning().force_generic && gemv_mma_supported(a)) return launch_gemv_mma(a, stream);
+    if (!gemv_tuning().force_generic && !gemv_tuning().no_mma && gemv_mma_supported(a)) return launch_gemv_mma(a, stream);
     const bool ring = gemv_stream_supported(a);
     if (!gemv_tuning().force_generic && gemv_rows_supported(a)) {
         const int64_t wbytes = static_cast<int64_t>(a.N) * a.K * 9 / 16;

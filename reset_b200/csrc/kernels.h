@@ -61,9 +61,11 @@ bool gemv_stream_supported(const GemvArgs& a);
 cudaError_t launch_gemv_stream(const GemvArgs& a, cudaStream_t stream);
 cudaError_t launch_gemv_generic(const GemvArgs& a, cudaStream_t stream);
 
-// The register-resident kernel for one or two tokens (gemv_rows.cu).
-bool gemv_mma_supported(const GemvArgs& a);      // two to eight tokens (gemv_mma.cu)
+// Two to eight tokens through mma.sync (gemv_mma.cu).
+bool gemv_mma_supported(const GemvArgs& a);
 cudaError_t launch_gemv_mma(const GemvArgs& a, cudaStream_t stream);
+
+// The register-resident kernel for one token (gemv_rows.cu).
 bool gemv_rows_supported(const GemvArgs& a);
 cudaError_t launch_gemv_rows(const GemvArgs& a, cudaStream_t stream);
 // mode: 0 automatic, 1 whenever supported, -1 never; rows per step 0 (automatic), 2 or 4;
@@ -77,6 +79,7 @@ struct GemvTuning {
     int ctas_per_sm;   // grid = SMs * ctas_per_sm
     int use_pdl;       // launch with programmatic stream serialization
     int force_generic; // route everything to the generic kernel (tests)
+    int no_mma;        // several tokens through the CUDA-core kernels (tests)
 };
 GemvTuning& gemv_tuning();
 

@@ -32,18 +32,20 @@ def capi():
     return c
 
 
-@pytest.fixture(params=["stream", "rows", "generic"])
+@pytest.fixture(params=["stream", "rows", "generic", "auto"])
 def path(request):
-    """The three GEMV kernels: the bulk-copy ring kernel (the register-resident one switched off),
-    the register-resident single-token kernel wherever it can take the launch, the plain-load
-    fallback."""
+    """The GEMV kernels: the bulk-copy ring kernel (the register-resident and the MMA kernel switched off), the
+    register-resident kernel wherever it can take the launch (one token; the ring kernel beyond), the plain-load
+    fallback, and the automatic choice: the MMA kernel for two to eight tokens."""
     from reset_b200 import _lib
+    _lib.check(_lib.lib().nvfp4r_set_gemv_mma_tuning(0 if request.param == "auto" else -1), "mma tuning")
     _lib.check(_lib.lib().nvfp4r_set_gemv_tuning(-1, -1, 1 if request.param == "generic" else 0), "tuning")
-    _lib.check(_lib.lib().nvfp4r_set_gemv_rows_tuning({"stream": -1, "rows": 1, "generic": -1}[request.param], 0, 0),
+    _lib.check(_lib.lib().nvfp4r_set_gemv_rows_tuning({"stream": -1, "rows": 1, "generic": -1, "auto": 0}[request.param], 0, 0),
                "rows tuning")
     yield request.param
     _lib.check(_lib.lib().nvfp4r_set_gemv_tuning(-1, -1, 0), "tuning")
     _lib.check(_lib.lib().nvfp4r_set_gemv_rows_tuning(0, 0, 0), "rows tuning")
+    _lib.check(_lib.lib().nvfp4r_set_gemv_mma_tuning(0), "mma tuning")
 
 
 def _run(capi, w, ws, x, xs, L, dtype, alpha=1.0):
