@@ -669,9 +669,14 @@ int large_min_m(int N, int K) {
     return n >= 6 * k && n < 16 * k ? 13 : 2 * n >= 3 * k ? 17 : n >= k ? 25 : kLargeMinM;
 }
 
+// What the entry point takes.
+bool large_accepts(int M, int N, int K) {
+    return N > 0 && K > 0 && N % kRows == 0 && K % 128 == 0 && M >= (g_large_min_m ? g_large_min_m : large_min_m(N, K));
+}
+
 bool large_pays(int M, int N, int K) {
-    if (g_large_min_m) return M >= g_large_min_m;
-    if (M < large_min_m(N, K)) return false;
+    if (!large_accepts(M, N, K)) return false;
+    if (g_large_min_m) return true;
     const int G = device_sm_count(), tiles = N / kRows, kblocks = (K + kBK - 1) / kBK;
     // A narrow weight with rows of 31 or 32 K blocks: the longest that still run as whole tiles here (0.48 us a
     // block), while two launches of the decode kernel give each CTA one block and one token to add up. 33 / 48 / 64
@@ -685,12 +690,13 @@ bool large_pays(int M, int N, int K) {
     return true;
 }
 
-size_t large_scratch_bytes(int M, int N, int K) {
+size_t large_scratch_need(int M, int N, int K) {
     LargePlan plan;
-    if (N <= 0 || K <= 0 || N % kRows || K % 128 || !large_pays(M, N, K)) return 0;
-    if (!plan_large(M, N, K, false, &plan)) return 0;
+    if (!large_accepts(M, N, K) || !plan_large(M, N, K, false, &plan)) return 0;
     return plan.token_bytes + plan.ticket_bytes + plan.partial_bytes;
 }
+
+size_t large_scratch_bytes(int M, int N, int K) { return large_pays(M, N, K) ? large_scratch_need(M, N, K) : 0; }
 
 // The host's side: a second launch and the scratch bring a call to 12 us or more even where the device needs 5, while
 // a call of the decode kernel ends at 8.5. So up to 32 tokens (one launch of it) that kernel keeps what it does in
@@ -699,7 +705,7 @@ size_t large_scratch_bytes(int M, int N, int K) {
 constexpr double kLargeCallUs = 12.0;
 
 int large_route(int M, int N, int K) {
-    if (N <= 0 || K <= 0 || N % kRows || K % 128 || !large_pays(M, N, K)) return NVFP4R_ROUTE_PACKED;
+    if (!large_pays(M, N, K)) return NVFP4R_ROUTE_PACKED;
     return g_large_min_m || M > 32 || packed_time_us(M, N, K) >= kLargeCallUs ? NVFP4R_ROUTE_SCRATCH : NVFP4R_ROUTE_SCRATCH_CAPTURED;
 }
 

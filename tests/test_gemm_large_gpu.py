@@ -97,6 +97,27 @@ def test_packed_token_counts_stay_inside_the_output(capi, M):
     assert rel_l2(got[256:256 + M * N].reshape(M, N), exact) <= 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(40, 640, 8192), (13, 19456, 256 * 8)])
+def test_scratch_entry_takes_shapes_that_its_query_leaves_to_the_other(capi, M, N, K):
+    """The query says 0 where the decode kernel is the faster one; a program that calls all the same, with the size
+    that the plan needs, is served."""
+    from reset_b200 import _lib
+    lib = _lib.lib()
+    _tune(1, 0, -1)
+    n = lib.nvfp4r_linear_packed_scratch_bytes(M, N, K)
+    _tune(0, 0, -1)
+    assert n > 0 and lib.nvfp4r_linear_packed_scratch_bytes(M, N, K) == 0
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M)
+    packed, x = capi.pack_weight(cuda(w), cuda(ws)), xb.cuda()
+    scratch, out = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.full((M, N), float("nan"), device="cuda")
+    args = [x.data_ptr(), K, M, K, gs.data_ptr(), packed.data_ptr(), N, 0.5, out.data_ptr(), F32, 0, scratch.data_ptr(), n,
+            torch.cuda.current_stream().cuda_stream]
+    _lib.check(lib.nvfp4r_linear_packed_scratch(*args), "linear_packed_scratch")
+    assert rel_l2(out.cpu().numpy(), exact) <= 1e-5
+    args[2] = 12                                             # fewer tokens than any class starts with
+    assert lib.nvfp4r_linear_packed_scratch(*args) == -2
+
+
 @pytest.mark.parametrize("dtype,half_ulp", [(0, 2.0 ** -8), (1, 2.0 ** -11)])
 def test_packed_16_bit_outputs_round_once(capi, dtype, half_ulp):
     M, N, K = 131, 384, 1024
