@@ -89,7 +89,9 @@ NVFP4R_API int nvfp4r_quant(const void* x, int64_t x_row_stride, int M, int K,
  * the P axis is read, out [L,N] contiguous. Strides are in bytes for the uint8
  * operands. `w_stride_l == 0` (and `wsf_stride_l == 0`) means one weight
  * broadcast over the L decode tokens (Tensor.expand), the decode case: the
- * weight is then streamed from HBM once for all L tokens. K % 32 == 0.
+ * weight is then streamed from HBM once for all L tokens. K % 32 == 0. As with nvfp4r_linear
+ * below, weight and weight_scale must be final before the preceding kernel of the stream is
+ * launched; x and x_scale may be that kernel's output.
  * ------------------------------------------------------------------------- */
 NVFP4R_API int nvfp4r_gemv(const void* weight, const void* weight_scale,
                            const void* x, const void* x_scale, void* out,

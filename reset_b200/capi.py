@@ -429,7 +429,7 @@ def sample(logits: torch.Tensor, draws: torch.Tensor, *, seed: int = 0,
 
 
 def sample_workspace(B: int, device) -> torch.Tensor:
-    """Zeroed scratch of ``sample(..., top_k=, top_p=)`` for up to ``B`` rows."""
+    """The workspace argument of ``sample(..., top_k=, top_p=)`` for up to ``B`` rows: checked, not used."""
     n = L.lib().nvfp4r_sample_workspace_bytes(B)
     return torch.zeros((n + 7) // 8, dtype=torch.int64, device=device)
 

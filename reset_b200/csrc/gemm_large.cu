@@ -25,14 +25,15 @@
 // fp32 partials, in K order, by the one that finishes last (atomic ticket; nothing waits, results do not
 // depend on the order of arrival).
 //
-// What bounds it: the bytes that one SM takes in from L2. A stage of 128 x 256 x 256 K is 55 KB for 512
-// clocks of MMA; measured about 100 GB/s per SM (52 bytes per clock) whatever the width, so the time is
-// stages x bytes / that rate: hence the widest tile that still fills the SMs. The MMA issuer is
-// straight-line code per K block: rolled loops made each tcgen05 instruction wait for its operands
-// (24576x4096, 2048 tokens, weights L2-cold, quantizer included: 111 -> 102 us, 4.0 PFLOP/s).
+// What bounds it: the bytes that one SM takes in from L2. A stage of 128 x 256 x 256 K is 55 KB for 512 clocks of MMA,
+// 107 bytes per clock; profiled on 24576x4096 with 2048 tokens it takes in 60 (1.36 GB in 104 us), the tensor
+// pipe is busy for 56 % of the active clocks and DRAM for 17 % of the time. So the time is stages x bytes / that rate:
+// hence the widest tile that still fills the SMs. The MMA issuer is straight-line code per K block: rolled loops made
+// each tcgen05 instruction wait for its operands (same call, quantizer included: 111 -> 102 us in a burst at 1965 MHz,
+// 4.0 PFLOP/s; calls kept up for seconds settle at 122 us, 1515 MHz under the power cap).
 // Measured, one call: 24576x4096 with 2048 tokens 2994 -> 121 us, 6144x4096 with 333 tokens 158 -> 13.7 us,
 // 10240x5120 with 45 tokens 35.5 -> 12.6 us; nvfp4r.quant + nvfp4r.gemm 4096x12288 with 128 tokens 147 ->
-// 24.7 us (left: 32 tokens per pass).
+// 22.5 us (left: 32 tokens per pass).
 #include <cuda.h>
 
 #include <atomic>

@@ -16,8 +16,11 @@
 // bf16 tokens, quantized) once per CTA into shared memory, 16 bytes per lane and two MMAs without bank conflicts. The
 // warps' sums of a tile meet in shared memory and are added in warp order: results are bit-identical run to run.
 //
-// Bound: instruction issue with 16 warps per SM (61 % of the slots, conversion and f16 pipes first; waits for loads
-// are 0.7 of 6.5 stall cycles an instruction; 24576x4096: 3.7 TB/s), the launch and the token prologue on small weights. Measured against the ring kernel (gemv.cu) and, for K % 256 != 0, the
+// Bound: with one CTA of 16 warps per SM (24576x8192, 8 tokens) instruction issue: 61 % of the slots, conversion and f16
+// pipes first, waits for loads 0.7 of 6.5 stall cycles an instruction; 24576x4096 runs at 3.7 TB/s. With two CTAs of 8
+// warps (7168x5120, 2 tokens) waits for loads come first, 2.3 of 7.9, at 44 % of the slots, and the tile count:
+// 448 tiles on 296 CTAs leave half of them one tile, the others two. On small weights the launch and the token
+// prologue. Measured against the ring kernel (gemv.cu) and, for K % 256 != 0, the
 // plain-load fallback, fp16 out, weights cold in L2, us, before -> after:
 //   7168x5120     2 tokens 10.8 -> 8.2    4 tokens 15.4 -> 8.8    8 tokens 24.7 -> 10.0
 //   640x1024      2 tokens 2.26 -> 1.67                           8 tokens 4.3 -> 1.8

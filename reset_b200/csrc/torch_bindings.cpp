@@ -81,8 +81,8 @@ void gemv_op(const at::Tensor& weight, const at::Tensor& weight_scale, const at:
 // stays valid for the life of the process. A call that needs more than the fixed size raises
 // (set NVFP4R_WORKSPACE_MB before the first call to change it); a first call inside a stream
 // capture raises too, because memory allocated there belongs to the capturing graph.
-// kind 0: tickets + fp32 split-K partials of `gemm` / `linear_tc` (the kernel leaves the
-// tickets zeroed); kind 1: the split-K slots of `linear_packed` (all zero between launches).
+// kind 0: tickets + fp32 split-K partials of `gemm` / `linear_tc` (every call leaves the ticket
+// area zeroed); kind 1: the split-K slots of `linear_packed` (all zero between launches).
 // The two never share memory.
 size_t workspace_capacity() {
     static const size_t cap = [] {

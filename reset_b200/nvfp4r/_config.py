@@ -18,7 +18,10 @@ FALLBACK_BACKEND = os.environ.get("NVFP4R_FALLBACK_BACKEND", "vllm-cutlass").low
 # to GEMV_MAX_WEIGHT_BYTES[1] (1280x5120 3.5 vs 5.0 us, 5120x2048 3.3 vs 3.6 us, 4096x4096 3.7 vs
 # 4.2 us, 3584x5120 4.55 vs 4.8 us; 5120x4096 5.1 vs 4.4 us, 6144x4096 5.0 vs 4.7 us,
 # 4096x12288 7.3 vs 6.2 us, 10240x5120 7.8 vs 6.3 us above it). From two tokens on the tensor
-# cores win on every shape measured (5120x1024 3.5 vs 3.4 us, 1280x5120 6.1 vs 5.0 us). Index = M.
+# cores take every weight: from about 4 MB on they are the faster kernel (two tokens, mma.sync GEMV vs
+# tensor cores: 1280x5120 4.7 vs 4.7 us, 4096x4096 4.7 vs 3.9 us, 24576x4096 16.0 vs 9.7 us; eight tokens:
+# 4096x4096 7.6 vs 4.9 us); below, the GEMV is (640x1024 2.1 vs 2.7 us, 5120x1024 2.7 vs 3.1 us), which an
+# eager call, about 8 us of host time either way, does not show. Index = M.
 GEMV_MAX_WEIGHT_BYTES = {1: 10_500_000}
 # Rows shorter than this stay on the tensor cores at every M (5120x640: 3.6 vs 3.8 us).
 GEMV_MIN_K = 1024

@@ -77,7 +77,7 @@ def use_gemv(M: int, N: int, K: int, gemv_max_m: int) -> bool:
     if K % 32 or K < _config.GEMV_MIN_K:
         return False
     if M > 1 and K % 256:
-        return False     # above one token the ring kernel is the GEMV, and it wants K % 256 == 0
+        return False     # several tokens: the crossover was measured for whole 256-element blocks
     ring = _config.GEMV_RING_WARPS
     if 4 * ring < N <= 5 * ring and K > _config.GEMV_SHORT_ROW_K:
         return False

@@ -8,7 +8,8 @@
 
 Differences from the reference, all inside the dispatch:
 
-* every decode batch is ONE launch per 32 rows. Below the measured crossover
+* every decode batch is ONE launch (two where the many-token kernel takes it, from 13 tokens on at the
+  earliest). Below the measured crossover
   (``gemv_max_m`` and a weight-size bound, ``_config.GEMV_MAX_WEIGHT_BYTES``) that launch
   is ``torch.ops.nvfp4r.linear`` (quantize + CUDA-core GEMV fused, instead of
   ``scaled_fp4_quant`` + ``expand`` + ``empty`` + ``nvfp4r.gemv``); above it it is
@@ -108,8 +109,8 @@ def _nvfp4r_linear_impl(x_2d: torch.Tensor, weight: torch.Tensor, weight_scale_s
       crossover, the tcgen05 kernel over the packed weight above it;
     * M above ``gemm_pad_max_m`` (prefill): vLLM's own ``scaled_fp4_quant`` +
       ``cutlass_scaled_fp4_mm`` when that vLLM is importable and ``fallback_backend`` is not
-      ``none`` (the reference's fallback branch), else this library's kernels in launches of
-      32 rows, each of which streams the weight once.
+      ``none`` (the reference's fallback branch), else this library's many-token kernel
+      (up to 256 tokens per pass over the weight).
     """
     from .ops import use_gemv
     M, K = x_2d.shape
