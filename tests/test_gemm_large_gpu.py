@@ -65,6 +65,39 @@ def test_packed_tiles_and_schedules(capi, M, N, K, bn, sk):
     assert rel_l2(a.cpu().numpy(), exact) <= 1e-5
 
 
+def _mixed_plan(M, N, K, bn):
+    """True when the plan is whole tiles first, stream-K over the tiles that are left: read off the size of the scratch,
+    tokens + 4 bytes a shared tile (in 256s) + two partial tiles for each of the CTAs that share."""
+    from reset_b200 import _lib
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    blocks, tiles = (K + 255) // 256, -(-M // bn) * (N // 128)
+    tokens = -(-(-(-M // bn) * blocks * (bn * 128 + -(-bn // 128) * 2048)) // 256) * 256
+    tickets = (_lib.lib().nvfp4r_linear_packed_scratch_bytes(M, N, K) - tokens) % (2 * bn * 512)
+    return tiles > sms and 0 < tickets <= -(-(tiles - sms) * 4 // 256) * 256
+
+
+@pytest.mark.parametrize("M,N,K,bn", [(256, 2560, 512, 16), (130, 5120, 640, 16), (33, 20480, 1024, 16), (257, 20480, 512, 256),
+                                      (130, 20480, 1024, 128)])
+def test_whole_tiles_then_stream_k(capi, M, N, K, bn):
+    """A CTA crosses from whole tiles to a range of the tiles that are left (with the ring and, above 128 tokens a
+    tile, the one accumulator carried across); tickets and partial sums are counted from the first shared tile."""
+    _tune(1, bn, 1)
+    assert _mixed_plan(M, N, K, bn)
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + bn)
+    a = _packed(capi, w, ws, xb.cuda(), gs, N)
+    assert torch.equal(a, _packed(capi, w, ws, xb.cuda(), gs, N))
+    assert rel_l2(a.cpu().numpy(), exact) <= 1e-5
+    if bn < 128 or K % 256:
+        return
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    wksp = torch.zeros(64 << 20, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        C = torch.full((M, N), float("nan"), device="cuda")
+        capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=False)
+        assert rel_l2(C.cpu().numpy(), exact) <= 1e-5
+    assert not wksp[:16384].any()
+
+
 @pytest.mark.parametrize("N,K,first", [(1536, 256, 13), (4096, 256, 17), (384, 256, 17), (256, 256, 25), (256, 384, 33)])
 def test_first_token_count_follows_the_shape(capi, N, K, first):
     """Both sides of the line between the decode kernel and this one, per shape class, give the same product."""
