@@ -213,14 +213,13 @@ NVFP4R_API int nvfp4r_linear_packed(const void* x, int64_t x_row_stride, int M, 
 /* The same linear for more tokens than one decode launch takes, given scratch for the quantized
  * tokens: the tokens are quantized once into `scratch` and one launch multiplies all of them, the weight
  * tile re-used for up to 256 tokens (gemm_large.cu), instead of one pass over the weight per 32 rows.
- *   nvfp4r_linear_packed_scratch_bytes   bytes of scratch, or 0 where nvfp4r_linear_packed is the
- *                                        faster kernel (few tokens) or the shape is unsupported:
- *                                        call that one then
+ *   nvfp4r_linear_packed_scratch_bytes   bytes of scratch, or 0 where the shape (few tokens, sizes) is not
+ *                                        taken: call nvfp4r_linear_packed then
  *   nvfp4r_linear_packed_route           which of the two entry points is the faster one: _PACKED, _SCRATCH, or
  *                                        _SCRATCH_CAPTURED where this one needs less device time, but a
  *                                        call that launches its two kernels and allocates the scratch
- *                                        each time needs more (up to 32 tokens). The torch operator asks;
- *                                        a C program that keeps its scratch can go by the bytes alone
+ *                                        each time needs more (up to 32 tokens): the torch operator then
+ *                                        takes it under stream capture alone
  *   nvfp4r_linear_packed_scratch         scratch >= that many bytes, 16-byte aligned, any contents; not
  *                                        kept after the launch
  * Same operands, arithmetic and rcp_mode meaning; the weight must be final before the preceding

@@ -399,7 +399,7 @@ int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride, int M, int
         return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: bad rcp_mode");
     if (out_dtype < NVFP4R_BF16 || out_dtype > NVFP4R_F32)
         return fail(NVFP4R_ERR_INVALID_ARGUMENT, "linear_packed_scratch: bad out_dtype");
-    const size_t need = nvfp4r::large_scratch_need(M, N, K);
+    const size_t need = nvfp4r::large_scratch_bytes(M, N, K);
     if (need == 0)
         return fail(NVFP4R_ERR_UNSUPPORTED_SHAPE, "linear_packed_scratch: shape belongs to nvfp4r_linear_packed");
     if (scratch_bytes < need || !aligned(scratch, 16))

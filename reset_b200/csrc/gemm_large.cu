@@ -691,13 +691,11 @@ bool large_pays(int M, int N, int K) {
     return true;
 }
 
-size_t large_scratch_need(int M, int N, int K) {
+size_t large_scratch_bytes(int M, int N, int K) {
     LargePlan plan;
     if (!large_accepts(M, N, K) || !plan_large(M, N, K, false, &plan)) return 0;
     return plan.token_bytes + plan.ticket_bytes + plan.partial_bytes;
 }
-
-size_t large_scratch_bytes(int M, int N, int K) { return large_pays(M, N, K) ? large_scratch_need(M, N, K) : 0; }
 
 // The host's side: a second launch and the scratch bring a call to 12 us or more even where the device needs 5, while
 // a call of the decode kernel ends at 8.5. So up to 32 tokens (one launch of it) that kernel keeps what it does in

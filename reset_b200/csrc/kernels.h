@@ -162,9 +162,8 @@ cudaError_t read_packed_trace(unsigned long long* out16);
 #endif
 
 // ---- gemm_large.cu --------------------------------------------------------
-// Scratch of the many-token linear over a packed weight; 0: launch_linear_packed is to be used.
+// Scratch of the many-token linear over a packed weight; 0: only launch_linear_packed takes the shape.
 size_t large_scratch_bytes(int M, int N, int K);
-size_t large_scratch_need(int M, int N, int K);  // the same where it is accepted, whether or not it is the faster one
 int large_route(int M, int N, int K);             // NVFP4R_ROUTE_*
 cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaStream_t stream);
 // *taken = false: nothing was launched, launch_linear_tc is to be used.

@@ -94,11 +94,18 @@ size_t workspace_capacity() {
     return cap;
 }
 
+std::mutex g_fixed_mu;
+std::unordered_map<int, at::Tensor> g_fixed[2];
+
+bool has_fixed_workspace(int kind, const at::Device& dev) {
+    std::lock_guard<std::mutex> lock(g_fixed_mu);
+    const auto it = g_fixed[kind].find(dev.index());
+    return it != g_fixed[kind].end() && it->second.defined();
+}
+
 at::Tensor& fixed_workspace(int kind, const at::Device& dev, size_t bytes, const char* who) {
-    static std::mutex mu;
-    static std::unordered_map<int, at::Tensor> cache[2];
-    std::lock_guard<std::mutex> lock(mu);
-    at::Tensor& t = cache[kind][dev.index()];
+    std::lock_guard<std::mutex> lock(g_fixed_mu);
+    at::Tensor& t = g_fixed[kind][dev.index()];
     if (!t.defined()) {
         TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None, who,
                     ": the first call on a device allocates the operator's scratch; make it before "
@@ -255,14 +262,19 @@ at::Tensor linear_packed_op(const at::Tensor& x, const at::Tensor& global_scale_
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     const auto dt = out_dtype_int == 0 ? at::kBFloat16 : out_dtype_int == 1 ? at::kHalf : at::kFloat;
     auto out = at::empty({M, N}, x.options().dtype(dt));
-    // many tokens: quantized once into scratch of this call (the caching allocator's, so capture and
-    // streams are its business), one launch for all of them
+    // Many tokens: quantized once into scratch of this call (the caching allocator's, so capture and streams are its
+    // business), one launch for all of them. Also where the other kernel is the faster one but its workspace is not
+    // to be had: larger than the fixed buffer, or under a capture that no call came before.
     const int route = nvfp4r_linear_packed_route(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K));
-    size_t scratch_bytes = 0;
-    if (route == NVFP4R_ROUTE_SCRATCH ||
-        (route == NVFP4R_ROUTE_SCRATCH_CAPTURED &&
-         c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None))
-        scratch_bytes = nvfp4r_linear_packed_scratch_bytes(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K));
+    const size_t ws_bytes = nvfp4r_linear_packed_workspace_bytes(static_cast<int>(M), static_cast<int>(N),
+                                                                 static_cast<int>(K));
+    bool many = route == NVFP4R_ROUTE_SCRATCH;
+    if (!many && M > 12)
+        many = ws_bytes > workspace_capacity() ||
+               (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None &&
+                (route == NVFP4R_ROUTE_SCRATCH_CAPTURED || !has_fixed_workspace(1, x.device())));
+    const size_t scratch_bytes =
+        many ? nvfp4r_linear_packed_scratch_bytes(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)) : 0;
     if (scratch_bytes > 0) {
         auto scratch = at::empty({static_cast<int64_t>(scratch_bytes)}, x.options().dtype(at::kByte));
         check_status(nvfp4r_linear_packed_scratch(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),
@@ -273,9 +285,7 @@ at::Tensor linear_packed_op(const at::Tensor& x, const at::Tensor& global_scale_
                      "linear_packed");
         return out;
     }
-    at::Tensor& ws = fixed_workspace(1, x.device(),
-                                     nvfp4r_linear_packed_workspace_bytes(static_cast<int>(M), static_cast<int>(N),
-                                                                          static_cast<int>(K)), "linear_packed");
+    at::Tensor& ws = fixed_workspace(1, x.device(), ws_bytes, "linear_packed");
     const int st = nvfp4r_linear_packed(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),
                                         global_scale_inv.data_ptr<float>(), packed.data_ptr(),
                                         static_cast<int>(N), static_cast<float>(alpha), out.data_ptr(),

@@ -130,16 +130,13 @@ def test_packed_token_counts_stay_inside_the_output(capi, M):
     assert rel_l2(got[256:256 + M * N].reshape(M, N), exact) <= 1e-5
 
 
-@pytest.mark.parametrize("M,N,K", [(40, 640, 8192), (13, 19456, 256 * 8)])
-def test_scratch_entry_takes_shapes_that_its_query_leaves_to_the_other(capi, M, N, K):
-    """The query says 0 where the decode kernel is the faster one; a program that calls all the same, with the size
-    that the plan needs, is served."""
+@pytest.mark.parametrize("M,N,K", [(40, 640, 8192), (13, 19456, 2048)])
+def test_scratch_entry_takes_shapes_where_the_other_is_faster(capi, M, N, K):
+    """The route is advice: a program that calls with the scratch all the same is served."""
     from reset_b200 import _lib
     lib = _lib.lib()
-    _tune(1, 0, -1)
     n = lib.nvfp4r_linear_packed_scratch_bytes(M, N, K)
-    _tune(0, 0, -1)
-    assert n > 0 and lib.nvfp4r_linear_packed_scratch_bytes(M, N, K) == 0
+    assert n > 0 and lib.nvfp4r_linear_packed_route(M, N, K) == 0
     w, ws, xb, gs, exact = _case(M, N, K, seed=M)
     packed, x = capi.pack_weight(cuda(w), cuda(ws)), xb.cuda()
     scratch, out = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.full((M, N), float("nan"), device="cuda")
@@ -149,6 +146,41 @@ def test_scratch_entry_takes_shapes_that_its_query_leaves_to_the_other(capi, M, 
     assert rel_l2(out.cpu().numpy(), exact) <= 1e-5
     args[2] = 12                                             # fewer tokens than any class starts with
     assert lib.nvfp4r_linear_packed_scratch(*args) == -2
+
+
+_NO_FIXED_BUFFER = """
+import sys, torch
+import reset_b200.nvfp4r
+for M, N, K in ((16, 20480, 2048), (16, 6144, 1024), (33, 1024, 8192)):
+    w = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device="cuda")
+    s = torch.full((N, K // 16), 0x38, dtype=torch.uint8, device="cuda")                     # 0x38: scale 1
+    packed = torch.ops.nvfp4r.pack_weight(w, s)
+    x, gs = torch.full((M, K), 6.0, dtype=torch.bfloat16, device="cuda"), torch.ones(1, device="cuda")   # code 6, scale 1
+    call = lambda: torch.ops.nvfp4r.linear_packed(x, gs, packed, N, 1.0, 2, 0)
+    if sys.argv[1] == "captured":
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out = call()
+        g.replay()
+    else:
+        out = call()
+    table = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], device="cuda")
+    want = 6 * (table[(w & 15).long()].sum(1) + table[(w >> 4).long()].sum(1))
+    assert torch.equal(out, want.expand(M, N)), (M, N, K)                                    # sums of halves: exact
+"""
+
+
+@pytest.mark.parametrize("how,megabytes", [("captured", "128"), ("eager", "1")])
+def test_many_tokens_need_no_fixed_buffer(how, megabytes):
+    """In a process of its own: a captured call that no other came before, and calls for which the fixed buffer (1 MB)
+    is too small for the decode kernel's workspace, take this kernel wherever it takes the shape."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _NO_FIXED_BUFFER, how], env=dict(os.environ, NVFP4R_WORKSPACE_MB=megabytes),
+                       cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("dtype,half_ulp", [(0, 2.0 ** -8), (1, 2.0 ** -11)])
@@ -232,7 +264,7 @@ def test_eager_and_captured_calls_give_the_same_product(capi, M, N, K):
     """Up to 32 tokens an eager call may take the decode kernel where a captured one takes this one: the operator's
     result is the oracle's either way."""
     from reset_b200 import _lib
-    assert _lib.lib().nvfp4r_linear_packed_scratch_bytes(M, N, K) > 0 or N >= 16 * K
+    assert _lib.lib().nvfp4r_linear_packed_route(M, N, K) == (2 if K == 4096 else 1 if N < 16 * K else 0)
     w, ws, xb, gs, exact = _case(M, N, K, seed=N % 89)
     packed, x = capi.pack_weight(cuda(w), cuda(ws)), xb.cuda()
     eager = torch.ops.nvfp4r.linear_packed(x, gs, packed, N, 0.5, F32, 0)
