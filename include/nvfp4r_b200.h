@@ -233,7 +233,8 @@ NVFP4R_API int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride,
                                             void* scratch, size_t scratch_bytes, void* stream);
 /* Debug/tuning of that kernel: fewest tokens it takes (0 = automatic), tokens per tile (a multiple
  * of 16 up to 256, 0 = automatic; nvfp4r_gemm rounds it up to a multiple of 128 where the tokens
- * need more than one tile), schedule (0 whole tiles, 1 stream-K, -1 automatic). */
+ * need more than one tile), schedule (-1 automatic, 0 whole tiles, 1 stream-K, 2..8 clusters
+ * of that many CTAs per tile). */
 NVFP4R_API int nvfp4r_set_gemm_large_tuning(int min_m, int tile_tokens, int stream_k);
 
 /* The same linear with the operator that PRODUCES its input fused into the prologue, so

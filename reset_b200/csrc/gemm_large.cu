@@ -18,24 +18,31 @@
 //   row-major  codes through 2-D tensor maps (128-byte swizzle), scales in the 128x4-tiled layout as
 //              512-byte chunks: the operands of the raw gemm operator.
 //
-// Persistent CTAs, one per SM, ten warps: warp 0 producer, warp 1 MMA issuer, warps 2-9 epilogue (two
-// per TMEM lane quadrant, each half of the columns). Schedule: CTA c first computes whole tiles c, c + G, ...
-// for `dp_rounds` rounds; the K blocks of the tiles that are left, laid end to end, are then cut into one
-// equal range for each of `sk_ctas` CTAs (stream-K). A tile that two or more CTAs share is summed from
-// fp32 partials, in K order, by the one that finishes last (atomic ticket; nothing waits, results do not
-// depend on the order of arrival).
+// CTAs of ten warps, one per SM: warp 0 producer, warp 1 MMA issuer, warps 2-9 epilogue (two
+// per TMEM lane quadrant, each half of the columns). Three schedules, chosen by an estimate of the time:
+//   whole tiles  CTA c computes tiles c, c + G, ...
+//   stream-K     after the rounds of whole tiles the K blocks of the tiles that are left, laid end to end, are cut into
+//                one equal range for each of `sk_ctas` CTAs. A tile that two or more CTAs share is summed from fp32
+//                partials in scratch, in K order, by the one that finishes last (atomic ticket; nothing waits, results
+//                do not depend on the order of arrival).
+//   cluster      a cluster of `split` CTAs takes one tile, each CTA an equal share of the K blocks. Each sends its partial
+//                sums of the columns that a peer owns into that peer's shared memory (the ring, idle by then), and
+//                every CTA adds up and stores its own columns, in K order. The hardware places a cluster as a whole,
+//                so nothing waits for a CTA that might not be running, and no scratch is needed.
 //
-// What bounds it: the bytes that one SM takes in from L2. A stage of 128 x 256 x 256 K is 55 KB for 512 clocks of MMA,
-// 107 bytes per clock; profiled on 24576x4096 with 2048 tokens it takes in 60 (1.36 GB in 104 us), the tensor
-// pipe is busy for 56 % of the active clocks and DRAM for 17 % of the time. So the time is stages x bytes / that rate:
-// hence the widest tile that still fills the SMs. The MMA issuer is straight-line code per K block: rolled loops made
-// each tcgen05 instruction wait for its operands (same call, quantizer included: 111 -> 102 us in a burst at 1965 MHz,
-// 4.0 PFLOP/s; calls kept up for seconds settle at 122 us, 1515 MHz under the power cap).
-// Measured, one call: 24576x4096 with 2048 tokens 2994 -> 121 us, 6144x4096 with 333 tokens 158 -> 13.7 us,
-// 10240x5120 with 45 tokens 35.5 -> 12.6 us; nvfp4r.quant + nvfp4r.gemm 4096x12288 with 128 tokens 147 ->
-// 22.5 us (left: 32 tokens per pass).
+// What bounds it. Few tiles: the chain launch - quantizer - launch - first stage - MMAs - stores, of which a K block is
+// 0.24 us: 515 clocks of the issuing warp (12 tcgen05 instructions at 17 to 25 clocks, a wait, a commit) against 218 for
+// the tensor pipe at 16 tokens. Many tokens: the bytes that the SMs take in from L2, 13 to 15 TB/s over all of them; MMAs
+// alone would run at 107 bytes a clock and SM, and the loads get 55 to 60.
+// The producer's addresses are worked out once per segment and it was 740 clocks a stage before, more than the issuer;
+// the issuer is straight-line code per K block (rolled loops made each tcgen05 instruction wait for its operands).
+// Device time in a CUDA graph, weights cold, us, one CTA a tile or stream-K with all of that before -> after:
+//   10240x5120  45 tokens 12.4 -> 10.1     6144x4096  333 tokens 13.9 -> 11.2     34816x5120  16 tokens 21.9 -> 19.8
+//   1024x4096   16 tokens 8.5 -> 6.1 (clusters of 4)    4096x12288 128 tokens, quant + gemm 21.3 -> 14.8 (clusters of 4)
+//   24576x4096  2048 tokens 104.9 -> 103.7
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -56,13 +63,22 @@ constexpr int kACodes = kRows * 128;
 constexpr int kMaxStagesL = 8;
 constexpr int kEpiWarps = 8;
 constexpr int kThreadsL = (2 + kEpiWarps) * 32;
+constexpr int kStoreChunk = 16 * kRows * 2;          // 16 tokens x 128 rows of a 16-bit output on their way to memory
+constexpr int kStoreBytes = 2 * kStoreChunk;         // one for each column half
 constexpr int kSmemBudget = 225 * 1024;              // dynamic part, 1 KB of it for alignment
-// Time model of plan_large, nanoseconds, fitted to sweeps over tile widths and both schedules (eight weights,
-// 16 .. 2048 tokens): a stage costs 200 ns + 1.3 ns per token of the tile; sharing a tile costs 2 us (partial
-// stores, fence, ticket) and 0.7 us per part and 64 columns (one trip to L2 each).
-constexpr double kStageBase = 200.0, kStagePerToken = 1.3, kFixBase = 2000.0, kFixPerPart = 700.0;
+constexpr int kMaxSplit = 8;                         // the largest cluster that every device can place
+// Time model of plan_large, nanoseconds, fitted to sweeps over tile widths and schedules (eight weights, 16 .. 700
+// tokens). A K block costs the issuing warp 235 + 0.17 per token of the tile (30 more for the second chunk of token
+// scales), unless the SMs at work take in more than 15.5 TB/s from L2 together or the weight more than 6.3 TB/s from
+// memory. The last tile's stores take 10.5 per token, those of a tile before it 3 where the one accumulator waits.
+// A shared stream-K tile: partial stores, fence and ticket, then a trip to L2 per part and 32 columns. A cluster: two
+// cluster barriers, each CTA's partial sums sent to the peers and read back.
+constexpr double kStageBase = 235.0, kStagePerToken = 0.17, kStageChunk = 30.0, kL2Rate = 15500.0, kHbmRate = 6300.0;
+constexpr double kStorePerToken = 10.5, kStoreWait = 3.0, kFixBase = 2000.0, kFixPerPart = 400.0;
+constexpr double kSplitBase = 1100.0, kSplitPerToken = 12.0, kSplitPerPartToken = 2.2, kSecondWave = 3500.0;
 constexpr uint32_t kTmemColsL = 512;
-constexpr uint32_t kColSfaL = 256, kColSfbL = 288;   // two buffers of 16, two of 32 columns
+constexpr int kTwoAccTokens = 192;                   // widest tile with two accumulators
+constexpr uint32_t kColSfaL = 384, kColSfbL = 416;   // two buffers of 16, two of 32 columns
 
 struct alignas(64) LargeParams {
     CUtensorMap map_w, map_x;                        // row-major form only
@@ -74,6 +90,7 @@ struct alignas(64) LargeParams {
     int64_t ldc;
     int M, N, bn, nch, tiles, tiles_m, kblocks, k64; // nch = 128-row scale chunks per token tile
     int stages;
+    int split, split_cols;                           // cluster schedule: CTAs per tile (else 1), columns that each sums up
     int dp_rounds, sk_base, sk_ctas, sk_q, sk_r;     // stream-K from tile sk_base on: sk_q (+1 for the first sk_r) K blocks per CTA
     float alpha;
     float* partials;                                 // [2 * sk_ctas][bn / 4][128][4]
@@ -83,35 +100,48 @@ struct alignas(64) LargeParams {
 __device__ int g_large_status = 0;
 
 // ---- token quantizer -------------------------------------------------------------------------
-// One thread per 16-element block; four lanes share one 32-bit store of scales. Also clears the
-// tickets of the GEMM that follows.
+// One thread per 16-element block and row, kR rows a CTA with their loads in flight together; four lanes share one
+// 32-bit store of scales. Also clears the tickets of the GEMM that follows.
+template <int kR>
 __global__ void __launch_bounds__(256)
-quant_pack_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, int K, const float* __restrict__ gs_ptr,
+quant_pack_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, int M, int K, const float* __restrict__ gs_ptr,
                   bool exact, uint8_t* __restrict__ packed, int bn, int nch, int kblocks,
                   unsigned* __restrict__ tickets, int n_tickets) {
     pdl_launch_dependents();
-    const int row = blockIdx.x;
-    const int mt = row / bn, r = row - mt * bn;
+    const int row0 = blockIdx.x * kR;
+    int mt = row0 / bn, r = row0 - mt * bn;
     const int col = blockIdx.y * 256 + threadIdx.x;
     const float gs = __ldg(gs_ptr);
     const QuantScales q = exact ? make_quant_scales<kRcpExact>(gs) : make_quant_scales<kRcpApprox>(gs);
     pdl_wait_prior();
     if (blockIdx.y == 0)
-        for (int i = row * 256 + threadIdx.x; i < n_tickets; i += gridDim.x * 256) tickets[i] = 0u;
+        for (int i = blockIdx.x * 256 + threadIdx.x; i < n_tickets; i += gridDim.x * 256) tickets[i] = 0u;
     if (col >= K / kBlockElems) return;               // K % 128 == 0: groups of eight lanes leave together
-    const uint4* src = reinterpret_cast<const uint4*>(x + row * x_row_stride + static_cast<int64_t>(col) * kBlockElems);
-    const uint4 lo = __ldg(src), hi = __ldg(src + 1);
-    uint32_t c[2];
-    const uint32_t sf = quantize_block16_rt(lo, hi, q, exact, c);
+    uint4 lo[kR], hi[kR];
+#pragma unroll
+    for (int i = 0; i < kR; ++i) {
+        const int row = min(row0 + i, M - 1);
+        const uint4* src = reinterpret_cast<const uint4*>(x + row * x_row_stride + static_cast<int64_t>(col) * kBlockElems);
+        lo[i] = __ldg(src);
+        hi[i] = __ldg(src + 1);
+    }
     const int kb = col >> 4, b = col & 15;
-    uint8_t* base = packed + (static_cast<int64_t>(mt) * kblocks + kb) * (bn * 128 + nch * 2048);
-    *reinterpret_cast<uint2*>(base + swz128(r, b * 8)) = make_uint2(c[0], c[1]);
     const unsigned live = __activemask();
-    uint32_t s4 = sf << (8 * (b & 3));
-    s4 |= __shfl_xor_sync(live, s4, 1);
-    s4 |= __shfl_xor_sync(live, s4, 2);
-    if ((b & 3) == 0)
-        *reinterpret_cast<uint32_t*>(base + bn * 128 + (r >> 7) * 2048 + (b >> 2) * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4) = s4;
+    const int tile_bytes = bn * 128 + nch * 2048;
+    uint8_t* base = packed + (static_cast<int64_t>(mt) * kblocks + kb) * tile_bytes;
+#pragma unroll
+    for (int i = 0; i < kR; ++i) {
+        if (row0 + i >= M) break;
+        uint32_t c[2];
+        const uint32_t sf = quantize_block16_rt(lo[i], hi[i], q, exact, c);
+        *reinterpret_cast<uint2*>(base + swz128(r, b * 8)) = make_uint2(c[0], c[1]);
+        uint32_t s4 = sf << (8 * (b & 3));
+        s4 |= __shfl_xor_sync(live, s4, 1);
+        s4 |= __shfl_xor_sync(live, s4, 2);
+        if ((b & 3) == 0)
+            *reinterpret_cast<uint32_t*>(base + bn * 128 + (r >> 7) * 2048 + (b >> 2) * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4) = s4;
+        if (++r == bn) { r = 0; base += static_cast<int64_t>(kblocks) * tile_bytes; }
+    }
 }
 
 // ---- work of one CTA -------------------------------------------------------------------------
@@ -125,6 +155,13 @@ struct Walker {
         end = c < p.sk_ctas ? cur + p.sk_q + (c < p.sk_r ? 1 : 0) : cur;
     }
     __device__ __forceinline__ bool next(const LargeParams& p, Segment& s) {
+        if (p.split > 1) {
+            const int part = static_cast<int>(cluster_ctarank());
+            s.tile = static_cast<int>(cluster_id());
+            s.k0 = p.kblocks * part / p.split;
+            s.k1 = p.kblocks * (part + 1) / p.split;
+            return round++ == 0;
+        }
         if (round < p.dp_rounds) {
             s.tile = blockIdx.x + round * gridDim.x;
             ++round;
@@ -151,24 +188,18 @@ __device__ __forceinline__ int sk_start(const LargeParams& p, int c) { return c 
 
 // One K block: the scale copies first, so that no MMA waits behind its own copy. Straight-line code with
 // compile-time counts: with rolled loops every instruction waits for its operands to reach uniform registers.
-template <int kChunks>
+template <int kChunks, int kSteps>
 __device__ __forceinline__ void issue_block(uint32_t d, uint64_t a, uint64_t b, uint64_t sa, uint64_t sb, uint32_t idesc,
                                             uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < kSteps; ++k) {
         tc_cp_scales(sfa + 4 * k, sa + 32 * k);
 #pragma unroll
         for (int j = 0; j < kChunks; ++j) tc_cp_scales(sfb + 4 * kChunks * k + 4 * j, sb + 128 * j + 32 * k);
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < kSteps; ++k)
         tc_mma_nvf4(d, a + 2 * k, b + 2 * k, idesc, sfa + 4 * k, sfb + 4 * kChunks * k, k == 0 ? accumulate : 1u);
-}
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
 }
 
 template <int kDtype>
@@ -181,24 +212,35 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Store 16 accumulator columns (tokens m0 .. m0+15) of this lane's weight row n.
-// M-major 16-bit: neighbouring lanes hold neighbouring n, so a pair of lanes trades halves and every
-// store is 4 bytes: 16 lanes x 4 B for token m from the even lanes, the same for m + 1 from the odd.
+// Stores 16 accumulator columns (tokens m0 .. m0+15) of the tile's 128 rows; the four warps of a column half call it
+// together, each lane with its weight row n = n0 + row.
+//   N-major         a lane's 16 tokens are contiguous.
+//   M-major, fp32   the lanes of a warp write 128 contiguous bytes per token.
+//   M-major, 16-bit a warp's share of a token is 64 bytes: the half's 16 x 128 values meet in shared memory and leave
+//                   in 16-byte pieces, 256 contiguous bytes per token. Straight from the registers (pairs of lanes
+//                   trading halves, 4 bytes a store) a tile of 128 x 112 took 2.4 us.
+struct Store {
+    uint8_t* chunk;     // this half's, in shared memory
+    int half, row, align;
+};
+
 template <int kDtype, bool kNMajor>
-__device__ __forceinline__ void store16(const LargeParams& p, int n, int m0, const float v[16], int lane, bool vec) {
-    const float al = p.alpha;
+__device__ __forceinline__ void store16(const LargeParams& p, Store& st, int n0, int m0, float v[16]) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
     if (kNMajor) {
+        const int64_t at = static_cast<int64_t>(n0 + st.row) * p.ldc + m0;
         if (kDtype == 2) {
-            float* o = static_cast<float*>(p.out) + static_cast<int64_t>(n) * p.ldc + m0;
+            float* o = static_cast<float*>(p.out) + at;
 #pragma unroll
             for (int j = 0; j < 16; ++j)
-                if (m0 + j < p.M) o[j] = v[j] * al;
+                if (m0 + j < p.M) o[j] = v[j];
         } else {
-            uint16_t* o = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(n) * p.ldc + m0;
+            uint16_t* o = static_cast<uint16_t*>(p.out) + at;
             uint32_t w[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) w[j] = pack2<kDtype>(v[2 * j] * al, v[2 * j + 1] * al);
-            if (vec && m0 + 16 <= p.M) {
+            for (int j = 0; j < 8; ++j) w[j] = pack2<kDtype>(v[2 * j], v[2 * j + 1]);
+            if (st.align == 16 && m0 + 16 <= p.M) {
                 reinterpret_cast<uint4*>(o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
                 reinterpret_cast<uint4*>(o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
             } else {
@@ -208,34 +250,88 @@ __device__ __forceinline__ void store16(const LargeParams& p, int n, int m0, con
             }
         }
     } else if (kDtype == 2) {
-        float* o = static_cast<float*>(p.out) + static_cast<int64_t>(m0) * p.ldc + n;
+        float* o = static_cast<float*>(p.out) + static_cast<int64_t>(m0) * p.ldc + n0 + st.row;
 #pragma unroll
         for (int j = 0; j < 16; ++j)
-            if (m0 + j < p.M) o[static_cast<int64_t>(j) * p.ldc] = v[j] * al;
+            if (m0 + j < p.M) o[static_cast<int64_t>(j) * p.ldc] = v[j];
     } else {
-        const bool odd = lane & 1;
-        uint16_t* o = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(m0 + (odd ? 1 : 0)) * p.ldc + (n & ~1);
-        const int lim = p.M - m0 - (odd ? 1 : 0);
+        uint16_t* mine = reinterpret_cast<uint16_t*>(st.chunk) + st.row;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const uint32_t mine = pack2<kDtype>(v[2 * j] * al, v[2 * j + 1] * al);
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            const uint32_t w = odd ? prmt(other, mine, 0x7632) : prmt(mine, other, 0x5410);
-            if (2 * j < lim) {
-                uint16_t* d = o + static_cast<int64_t>(2 * j) * p.ldc;
-                if (vec) {
-                    *reinterpret_cast<uint32_t*>(d) = w;
-                } else {
-                    d[0] = static_cast<uint16_t>(w);
-                    d[1] = static_cast<uint16_t>(w >> 16);
+            const uint32_t w = pack2<kDtype>(v[2 * j], v[2 * j + 1]);
+            mine[2 * j * kRows] = static_cast<uint16_t>(w);
+            mine[(2 * j + 1) * kRows] = static_cast<uint16_t>(w >> 16);
+        }
+        named_barrier(2 + st.half, kRows);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int token = u * 8 + (st.row >> 4), piece = st.row & 15;
+            if (m0 + token >= p.M) break;
+            const uint4 w = *reinterpret_cast<const uint4*>(st.chunk + token * (kRows * 2) + piece * 16);
+            uint16_t* o = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(m0 + token) * p.ldc + n0 + piece * 8;
+            if (st.align == 16) {
+                *reinterpret_cast<uint4*>(o) = w;
+            } else {
+                const uint32_t e[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (st.align == 4) {
+                        reinterpret_cast<uint32_t*>(o)[j] = e[j];
+                    } else {
+                        o[2 * j] = static_cast<uint16_t>(e[j]);
+                        o[2 * j + 1] = static_cast<uint16_t>(e[j] >> 16);
+                    }
                 }
             }
         }
+        named_barrier(2 + st.half, kRows);             // read before the next 16 tokens are written
+    }
+}
+
+// The issuing warp: all lanes walk, one elected lane issues.
+template <int kChunks>
+__device__ __forceinline__ void issue_all(const LargeParams& p, uint32_t ring, uint32_t tmem, uint32_t bar_full,
+                                          uint32_t bar_empty, uint32_t bar_accfull, uint32_t bar_accempty, WaitFail& wf) {
+    const bool lead = elect_one();
+    const uint32_t b_codes = static_cast<uint32_t>(p.bn) * 128u;
+    const uint32_t stage_bytes = kABytes + b_codes + kChunks * 2048u;
+    const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.bn >> 3) << 17) | (1u << 27);
+    const int n_acc = p.bn <= kTwoAccTokens ? 2 : 1, stages = p.stages;
+    const int whole = p.k64 >> 2;                     // K % 256 == 128: the last block has two of four steps
+    Walker wk(p);
+    Segment sg;
+    uint32_t s = 0, phase = 0, odd = 0;
+    for (int t = 0; !wf.failed && wk.next(p, sg); ++t) {
+        const int buf = n_acc == 2 ? (t & 1) : 0;
+        const int use = n_acc == 2 ? (t >> 1) : t;    // how often this buffer was used before
+        if (use > 0 && !wf.wait(bar_accempty + 8 * buf, (use - 1) & 1)) break;
+        tc_fence_after();
+        const uint32_t d = tmem + buf * kTwoAccTokens;
+        uint32_t more = 0;
+        for (int kb = sg.k0; kb < sg.k1; ++kb) {
+            if (!wf.wait(bar_full + 8 * s, phase)) break;
+            tc_fence_after();
+            const uint32_t a_smem = ring + s * stage_bytes;
+            const uint64_t a_desc = desc_operand(a_smem), b_desc = desc_operand(a_smem + kABytes);
+            const uint64_t sa_desc = desc_scales(a_smem + kACodes), sb_desc = desc_scales(a_smem + kABytes + b_codes);
+            const uint32_t sfa = tmem + kColSfaL + odd * 16, sfb = tmem + kColSfbL + odd * 32;
+            if (lead) {
+                if (kb < whole) issue_block<kChunks, 4>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
+                else issue_block<kChunks, 2>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
+                tc_commit(bar_empty + 8 * s);
+            }
+            __syncwarp();
+            more = 1;
+            odd ^= 1u;
+            if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
+        }
+        if (lead) tc_commit(bar_accfull + 8 * buf);
+        __syncwarp();
     }
 }
 
 template <bool kTma, int kDtype, bool kNMajor>
-__global__ void __launch_bounds__(kThreadsL, 1)
+__global__ void __launch_bounds__(kThreadsL, 2)
 gemm_large_kernel(const __grid_constant__ LargeParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -249,7 +345,7 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
     const uint32_t stage_bytes = kABytes + b_codes + static_cast<uint32_t>(nch) * 2048u;
     const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = smem_u32(&bars[kMaxStagesL]);
     const uint32_t bar_accfull = smem_u32(&bars[2 * kMaxStagesL]), bar_accempty = bar_accfull + 16;
-    const int n_acc = bn <= 128 ? 2 : 1;             // accumulator buffers in 256 columns
+    const int n_acc = bn <= kTwoAccTokens ? 2 : 1;
 
     if (warp == 0 && lane < 2 * kMaxStagesL + 4) {
         mbar_init(bar_full + 8 * lane, lane >= 2 * kMaxStagesL + 2 ? kEpiWarps : 1);
@@ -269,149 +365,170 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
         // tokens are read by every column of tiles, a weight tile by tiles_m CTAs at about the same time
         const uint64_t keep = l2_policy_evict_last();
         const uint64_t policy = p.tiles_m > 1 ? l2_policy_evict_normal() : l2_policy_evict_first();
-        auto load_a = [&](const Segment& sg, int kb, int s) {
-            const int nt = sg.tile / p.tiles_m;
-            const uint32_t dst = ring + s * stage_bytes;
+        const uint32_t b_bytes = b_codes + static_cast<uint32_t>(nch) * 2048u;
+        // Where a segment's operands lie, worked out once per segment: with the divisions and products in the block
+        // loop a stage cost this warp 740 clocks, more than its MMAs.
+        struct Source {
+            const uint8_t *a, *b;                     // packed: next block; row-major: next scales
+            int ax, ay, by, ch;                       // row-major: code coordinates, scale chunks of the token tile
+        };
+        auto source = [&](const Segment& sg) {
+            const int nt = sg.tile / p.tiles_m, mt = sg.tile - nt * p.tiles_m;
+            Source o;
             if (kTma) {
-                tma_load_2d(dst, &p.map_w, kb * 128, nt * kRows, bar_full + 8 * s, policy);
-                bulk_g2s(dst + kACodes, p.wsf + (static_cast<int64_t>(nt) * p.k64 + kb * 4) * 512, 2048, bar_full + 8 * s, policy);
+                o.a = p.wsf + (static_cast<int64_t>(nt) * p.k64 + sg.k0 * 4) * 512;
+                o.b = p.xsf + (static_cast<int64_t>(mt * nch) * p.k64 + sg.k0 * 4) * 512;
+                o.ax = sg.k0 * 128;
+                o.ay = nt * kRows;
+                o.by = mt * bn;
+                o.ch = min(nch, (p.M - mt * bn + 127) >> 7);          // chunks that exist in xsf
             } else {
-                bulk_g2s(dst, p.w + (static_cast<int64_t>(nt) * p.kblocks + kb) * kABytes, kABytes, bar_full + 8 * s, policy);
+                o.a = p.w + (static_cast<int64_t>(nt) * p.kblocks + sg.k0) * kABytes;
+                o.b = p.x + (static_cast<int64_t>(mt) * p.kblocks + sg.k0) * b_bytes;
+                o.ch = nch;
+            }
+            return o;
+        };
+        auto load_a = [&](const Source& o, uint32_t dst, uint32_t bar) {
+            mbar_expect_tx(bar, kABytes + b_codes + static_cast<uint32_t>(o.ch) * 2048u);
+            if (kTma) {
+                tma_load_2d(dst, &p.map_w, o.ax, o.ay, bar, policy);
+                bulk_g2s(dst + kACodes, o.a, 2048, bar, policy);
+            } else {
+                bulk_g2s(dst, o.a, kABytes, bar, policy);
             }
         };
-        auto load_b = [&](const Segment& sg, int kb, int s, int valid_ch) {
-            const int mt = sg.tile % p.tiles_m;
-            const uint32_t dst = ring + s * stage_bytes + kABytes;
+        auto load_b = [&](const Source& o, uint32_t dst, uint32_t bar) {
             if (kTma) {
-                tma_load_2d(dst, &p.map_x, kb * 128, mt * bn, bar_full + 8 * s, keep);
-                for (int j = 0; j < valid_ch; ++j)
-                    bulk_g2s(dst + b_codes + j * 2048, p.xsf + (static_cast<int64_t>(mt * nch + j) * p.k64 + kb * 4) * 512,
-                             2048, bar_full + 8 * s, keep);
+                tma_load_2d(dst, &p.map_x, o.ax, o.by, bar, keep);
+                for (int j = 0; j < o.ch; ++j)
+                    bulk_g2s(dst + b_codes + j * 2048, o.b + static_cast<int64_t>(j) * p.k64 * 512, 2048, bar, keep);
             } else {
-                const uint32_t bytes = b_codes + static_cast<uint32_t>(nch) * 2048u;
-                bulk_g2s(dst, p.x + (static_cast<int64_t>(mt) * p.kblocks + kb) * bytes, bytes, bar_full + 8 * s, keep);
+                bulk_g2s(dst, o.b, b_bytes, bar, keep);
             }
         };
-        auto chunks_of = [&](const Segment& sg) {     // 128-row scale chunks of the tile that exist in xsf
-            if (!kTma) return nch;
-            const int rows = p.M - (sg.tile % p.tiles_m) * bn;
-            return min(nch, (rows + 127) >> 7);
+        auto advance = [&](Source& o) {
+            o.a += kTma ? 2048 : kABytes;
+            o.b += kTma ? 2048u : b_bytes;
+            o.ax += 128;
         };
         // The weight does not depend on the kernel before: the weight half of the first stages is
         // requested ahead of the wait, the token half behind it.
-        Walker wa(p);
-        Segment sa;
         int pre = 0;
         {
-            bool more = wa.next(p, sa);
-            int kb = more ? sa.k0 : 0;
-            while (more && pre < stages) {
-                if (lead) {
-                    mbar_expect_tx(bar_full + 8 * pre, kABytes + b_codes + static_cast<uint32_t>(chunks_of(sa)) * 2048u);
-                    load_a(sa, kb, pre);
+            Walker wa(p);
+            Segment sa;
+            uint32_t dst = ring, bar = bar_full;
+            while (pre < stages && wa.next(p, sa)) {
+                Source o = source(sa);
+                for (int kb = sa.k0; kb < sa.k1 && pre < stages; ++kb, ++pre) {
+                    if (lead) load_a(o, dst, bar);
+                    __syncwarp();
+                    advance(o);
+                    dst += stage_bytes;
+                    bar += 8;
                 }
-                ++pre;
-                if (++kb == sa.k1) { more = wa.next(p, sa); kb = sa.k0; }
             }
         }
         pdl_wait_prior();
         Walker wk(p);
         Segment sg;
         int i = 0;
-        uint32_t s = 0, phase = 1;                    // phase the empty barrier must have completed
+        uint32_t s = 0, phase = 1, dst = ring;        // phase the empty barrier must have completed
         while (!wf.failed && wk.next(p, sg)) {
-            const int ch = chunks_of(sg);
+            Source o = source(sg);
             for (int kb = sg.k0; kb < sg.k1; ++kb, ++i) {
                 if (i >= stages && !wf.wait(bar_empty + 8 * s, phase)) break;
                 if (lead) {
-                    if (i >= pre) {
-                        mbar_expect_tx(bar_full + 8 * s, kABytes + b_codes + static_cast<uint32_t>(ch) * 2048u);
-                        load_a(sg, kb, s);
-                    }
-                    load_b(sg, kb, s, ch);
+                    if (i >= pre) load_a(o, dst, bar_full + 8 * s);
+                    load_b(o, dst + kABytes, bar_full + 8 * s);
                 }
                 __syncwarp();
-                if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
+                advance(o);
+                dst += stage_bytes;
+                if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; dst = ring; }
             }
         }
         if (wf.failed)                                 // let the copies in flight land before the CTA goes
             for (int j = max(0, i - stages); j < i; ++j) mbar_wait_bounded(bar_full + 8 * (j % stages), (j / stages) & 1, 100000u);
     } else if (warp == 1) {
         // ---------------- MMA issuer -----------------------------------------------------------
-        const bool lead = elect_one();
-        const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(bn >> 3) << 17) | (1u << 27);
-        Walker wk(p);
-        Segment sg;
-        uint32_t s = 0, phase = 0;
-        int i = 0;
-        for (int t = 0; !wf.failed && wk.next(p, sg); ++t) {
-            const int buf = n_acc == 2 ? (t & 1) : 0;
-            const int use = n_acc == 2 ? (t >> 1) : t;           // how often this buffer was used before
-            if (use > 0 && !wf.wait(bar_accempty + 8 * buf, (use - 1) & 1)) break;
-            tc_fence_after();
-            const uint32_t d = tmem + buf * 128;
-            for (int kb = sg.k0; kb < sg.k1; ++kb, ++i) {
-                if (!wf.wait(bar_full + 8 * s, phase)) break;
-                tc_fence_after();
-                const uint32_t a_smem = ring + s * stage_bytes;
-                const uint64_t a_desc = desc_operand(a_smem), b_desc = desc_operand(a_smem + kABytes);
-                const uint64_t sa_desc = desc_scales(a_smem + kACodes), sb_desc = desc_scales(a_smem + kABytes + b_codes);
-                const uint32_t sfa = tmem + kColSfaL + (i & 1) * 16, sfb = tmem + kColSfbL + (i & 1) * 32;
-                if (lead) {
-                    const uint32_t more = kb > sg.k0 ? 1u : 0u;
-                    if (p.k64 - kb * 4 < 4) {                     // K % 256 == 128: the last block has two of four
-                        for (int k = 0; k < 2; ++k) {
-                            tc_cp_scales(sfa + 4 * k, sa_desc + 32 * k);
-                            for (int j = 0; j < nch; ++j) tc_cp_scales(sfb + 4 * nch * k + 4 * j, sb_desc + 128 * j + 32 * k);
-                        }
-                        for (int k = 0; k < 2; ++k)
-                            tc_mma_nvf4(d, a_desc + 2 * k, b_desc + 2 * k, idesc, sfa + 4 * k, sfb + 4 * nch * k, k == 0 ? more : 1u);
-                    } else if (nch == 1) {
-                        issue_block<1>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
-                    } else {
-                        issue_block<2>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
-                    }
-                    tc_commit(bar_empty + 8 * s);
-                }
-                __syncwarp();
-                if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
-            }
-            if (lead) tc_commit(bar_accfull + 8 * buf);
-            __syncwarp();
-        }
+        if (nch == 1) issue_all<1>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
+        else issue_all<2>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
     } else {
         // ---------------- epilogue (warps 2..9) ------------------------------------------------
         pdl_wait_prior();                              // out, partials and tickets may still be in use before it
         const int q = warp & 3, half = (warp - 2) >> 2;
         const int row = q * 32 + lane;
         const int cols_half = (((bn >> 4) + 1) >> 1) << 4;
-        const int c_lo = half ? cols_half : 0, c_n = half ? bn - cols_half : cols_half;
-        const bool vec = kNMajor ? (p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)
-                                 : (reinterpret_cast<uintptr_t>(p.out) & 3) == 0;
+        const int c_lo = half ? cols_half : 0, groups = (half ? bn - cols_half : cols_half) >> 4;
+        const uintptr_t out_at = reinterpret_cast<uintptr_t>(p.out) | (kDtype == 2 ? 0 : static_cast<uintptr_t>(p.ldc) * 2);
+        Store st;
+        st.chunk = smem_raw + (ring + stages * stage_bytes - smem_u32(smem_raw)) + half * kStoreChunk;
+        st.half = half;
+        st.row = row;
+        st.align = (out_at & 15) == 0 ? 16 : (out_at & 3) == 0 ? 4 : 2;
         Walker wk(p);
         Segment sg;
+        // Rolled loops of 16 columns: a tile's columns leave the tensor memory at the pace of the stores. Unrolled over
+        // the tile (all of it in registers first) the code was fetched cold once per launch, and 200 registers a thread
+        // left no room for these CTAs beside the quantizer's.
         for (int t = 0; wk.next(p, sg); ++t) {
             const int buf = n_acc == 2 ? (t & 1) : 0;
             const int use = n_acc == 2 ? (t >> 1) : t;
             const int nt = sg.tile / p.tiles_m, mt = sg.tile - nt * p.tiles_m;
-            const int n = nt * kRows + row, m0 = mt * bn;
+            const int n0 = nt * kRows, m0 = mt * bn;
             wf.wait(bar_accfull + 8 * buf, use & 1);   // after a time-out: walk on, the warps meet at barriers below
             tc_fence_after();
-            const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * 128 + c_lo;
-            const bool shared_tile = sg.k1 - sg.k0 != p.kblocks;
-            // drain the whole half into registers, then let the next tile's MMAs at the accumulator
-            float v[8][16];
+            const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * kTwoAccTokens + c_lo;
+            auto release = [&] {                       // the next tile's MMAs may have the accumulator
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_accempty + 8 * buf);
+            };
+            float v[16];
+            if (p.split > 1) {
+                const int S = p.split, w = p.split_cols, rank = static_cast<int>(cluster_ctarank());
+                cluster_sync_all();                    // every CTA of the cluster is through with its ring
+#pragma unroll 1
+                for (int g = 0; g < groups; ++g) {
+                    tmem_ld16(taddr + 16 * g, v);
+                    tmem_ld_wait();
+                    const int col = c_lo + 16 * g, owner = col / w;
+                    const uint32_t dst = cluster_map(ring + ((rank * w + col - owner * w) * kRows + row * 4) * 4, owner);
 #pragma unroll
-            for (int g = 0; g < 8; ++g)
-                if (16 * g < c_n) tmem_ld16(taddr + 16 * g, v[g]);
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_accempty + 8 * buf);
-            if (!shared_tile) {
+                    for (int j = 0; j < 4; ++j) cluster_st16(dst + j * (kRows * 16), v + 4 * j);
+                }
+                cluster_sync_all();
+                const int mine = min(w, bn - rank * w);
+#pragma unroll 1
+                for (int c = 16 * half; c < mine; c += 32) {
+                    const float4* src = reinterpret_cast<const float4*>(smem_raw + (ring - smem_u32(smem_raw))) +
+                                        (c >> 2) * kRows + row;
+#pragma unroll 4
+                    for (int r = 0; r < S; ++r) {      // K order
 #pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    if (16 * g < c_n) store16<kDtype, kNMajor>(p, n, m0 + c_lo + 16 * g, v[g], lane, vec);
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 x = src[(r * (w >> 2) + j) * kRows];
+                            v[4 * j] = r ? v[4 * j] + x.x : x.x;
+                            v[4 * j + 1] = r ? v[4 * j + 1] + x.y : x.y;
+                            v[4 * j + 2] = r ? v[4 * j + 2] + x.z : x.z;
+                            v[4 * j + 3] = r ? v[4 * j + 3] + x.w : x.w;
+                        }
+                    }
+                    store16<kDtype, kNMajor>(p, st, n0, m0 + rank * w + c, v);
+                }
+                continue;
+            }
+            if (sg.k1 - sg.k0 == p.kblocks) {
+#pragma unroll 1
+                for (int g = 0; g < groups; ++g) {
+                    tmem_ld16(taddr + 16 * g, v);
+                    tmem_ld_wait();
+                    if (g == groups - 1) release();
+                    store16<kDtype, kNMajor>(p, st, n0, m0 + c_lo + 16 * g, v);
+                }
+                if (groups == 0) release();
                 continue;
             }
             // stream-K: leave the partial sums, the last CTA of the tile to arrive adds all of them
@@ -421,16 +538,16 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
                 return reinterpret_cast<float4*>(p.partials) +
                        ((2 * static_cast<int64_t>(c) + (sk_start(p, c) >= base ? 0 : 1)) * bn + c_lo) / 4 * kRows + row;
             };
-            {
-                float4* mine = slot(blockIdx.x);
+            float4* own = slot(blockIdx.x);
+#pragma unroll 1
+            for (int g = 0; g < groups; ++g) {
+                tmem_ld16(taddr + 16 * g, v);
+                tmem_ld_wait();
 #pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    if (16 * g < c_n) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            __stcg(mine + (4 * g + j) * kRows, make_float4(v[g][4 * j], v[g][4 * j + 1], v[g][4 * j + 2], v[g][4 * j + 3]));
-                    }
+                for (int j = 0; j < 4; ++j)
+                    __stcg(own + (4 * g + j) * kRows, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
             }
+            release();
             named_barrier(1, kEpiWarps * 32);
             if (tid == 64) {
                 __threadfence();
@@ -441,33 +558,30 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
             }
             named_barrier(1, kEpiWarps * 32);
             if (s_last) {
-                // two parts: the sum of two does not depend on their order, so this CTA's stays in registers;
-                // more: all are added in K order, this CTA's own read back like the others
-                const bool two = last - first == 1;
 #pragma unroll 1
-                for (int c = first; c <= last; ++c) {
-                    if (two && c == static_cast<int>(blockIdx.x)) continue;
-                    const float4* src = slot(c);
-                    const bool add = two || c != first;
+                for (int g = 0; g < groups; ++g) {
+#pragma unroll 2
+                    for (int c = first; c <= last; ++c) {                // K order, this CTA's own among them
+                        const float4* src = slot(c) + 4 * g * kRows;
 #pragma unroll
-                    for (int g = 0; g < 8; ++g)
-                        if (16 * g < c_n) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const float4 t = __ldcg(src + (4 * g + j) * kRows);
-                                v[g][4 * j] = add ? v[g][4 * j] + t.x : t.x;
-                                v[g][4 * j + 1] = add ? v[g][4 * j + 1] + t.y : t.y;
-                                v[g][4 * j + 2] = add ? v[g][4 * j + 2] + t.z : t.z;
-                                v[g][4 * j + 3] = add ? v[g][4 * j + 3] + t.w : t.w;
-                            }
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 x = __ldcg(src + j * kRows);
+                            v[4 * j] = c != first ? v[4 * j] + x.x : x.x;
+                            v[4 * j + 1] = c != first ? v[4 * j + 1] + x.y : x.y;
+                            v[4 * j + 2] = c != first ? v[4 * j + 2] + x.z : x.z;
+                            v[4 * j + 3] = c != first ? v[4 * j + 3] + x.w : x.w;
                         }
+                    }
+                    store16<kDtype, kNMajor>(p, st, n0, m0 + c_lo + 16 * g, v);
                 }
-#pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    if (16 * g < c_n) store16<kDtype, kNMajor>(p, n, m0 + c_lo + 16 * g, v[g], lane, vec);
             }
             named_barrier(1, kEpiWarps * 32);          // s_last is written again for the next shared tile
         }
+    }
+    // the epilogue's two cluster barriers: all warps of all CTAs take part
+    if (p.split > 1 && warp < 2) {
+        cluster_sync_all();
+        cluster_sync_all();
     }
 
     if (wf.failed && lane == 0) report_timeout(&g_large_status, 6);
@@ -512,11 +626,45 @@ bool code_map(const void* p, int rows, int K, int box_rows, CUtensorMap* out) {
 
 struct LargePlan {
     int bn, nch, tiles_m, tiles, kblocks, stages, grid;
-    int dp_rounds, sk_base, sk_ctas;
+    int dp_rounds, sk_base, sk_ctas, split, split_cols;
     size_t smem, token_bytes, ticket_bytes, partial_bytes;
 };
 
 int g_large_bn = 0, g_large_sk = -1, g_large_min_m = 0;
+
+size_t stage_bytes_of(int bn) { return kABytes + bn * 128 + (bn + 127) / 128 * 2048; }
+int ring_stages(int bn) {
+    const int n = static_cast<int>((kSmemBudget - 1024 - kStoreBytes) / stage_bytes_of(bn));
+    return n > kMaxStagesL ? kMaxStagesL : n;
+}
+
+// Clusters of S one-per-SM CTAs that run at once: an SM of a GPC that is left over takes none (148 SMs: 74 pairs, 33 fours).
+int cluster_capacity(int S, int G) {
+    static std::atomic<int> known[64][kMaxSplit + 1] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return G / S;
+    int n = known[dev][S].load(std::memory_order_relaxed);
+    if (n == 0) {
+        const auto kern = gemm_large_kernel<false, 0, false>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(G / S * S));
+        cfg.blockDim = dim3(kThreadsL);
+        cfg.dynamicSmemBytes = kSmemBudget;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(S);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = G / S;
+        }
+        known[dev][S].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
 
 // Tile width and schedule by an estimate of the time in nanoseconds, for G SMs.
 bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan) {
@@ -533,20 +681,35 @@ bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan
         const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;
         if (tiles * kblocks > 0x3fffffff) continue;
         const int nch = (bn + 127) / 128;
-        const double stage = kStageBase + kStagePerToken * bn, epi = bn > 128 ? 500.0 : 100.0;
+        const double floor_ns = static_cast<double>(N) * K * 9 / 16 / kHbmRate, store = kStorePerToken * bn;
+        const auto stage_ns = [&](int64_t ctas) {
+            const double issue = kStageBase + kStagePerToken * bn + (nch - 1) * kStageChunk;
+            return std::max(issue, static_cast<double>(stage_bytes_of(bn)) * std::min<int64_t>(ctas, G) / kL2Rate);
+        };
+        const double stage = stage_ns(tiles), wait = bn > kTwoAccTokens ? kStoreWait * bn : 0.0;
         const int full = static_cast<int>(tiles / G);
-        auto consider = [&](int dp, int ctas, double t) {
+        auto consider = [&](int dp, int ctas, int split, double t) {
+            t = std::max(t, floor_ns + store);
             if (t >= best) return;
             best = t;
             found = true;
             plan->bn = bn; plan->nch = nch; plan->tiles_m = tiles_m; plan->tiles = static_cast<int>(tiles);
             plan->kblocks = kblocks; plan->dp_rounds = dp; plan->sk_ctas = ctas;
+            plan->split = split; plan->split_cols = (bn / 16 + split - 1) / split * 16;
         };
-        if (g_large_sk != 1) {
+        if (g_large_sk <= 0 || (g_large_sk > 1 && kblocks < g_large_sk)) {
             const int rounds = static_cast<int>((tiles + G - 1) / G);
-            consider(rounds, 0, rounds * (kblocks * stage + epi));
+            consider(rounds, 0, 1, rounds * kblocks * stage + (rounds - 1) * wait + store);
         }
-        if (g_large_sk == 0) continue;
+        for (int S = 2; S <= kMaxSplit && g_large_sk != 0 && g_large_sk != 1; ++S) {
+            if (kblocks < S || (g_large_sk > 1 && S != g_large_sk)) continue;
+            const int w = (bn / 16 + S - 1) / S * 16, at_once = cluster_capacity(S, G);
+            if (static_cast<size_t>(S) * w * kRows * 4 > static_cast<size_t>(ring_stages(bn)) * stage_bytes_of(bn)) continue;
+            const int rounds = static_cast<int>((tiles + at_once - 1) / at_once);
+            consider(0, 0, S, rounds * ((kblocks + S - 1) / S * stage_ns(tiles * S) + kSplitBase +
+                                        bn * (kSplitPerToken + S * kSplitPerPartToken)) + (rounds - 1) * kSecondWave);
+        }
+        if (g_large_sk == 0 || g_large_sk > 1) continue;
         for (int dp = full; dp >= 0 && dp >= full - 1; --dp) {
             const int64_t rest = tiles - static_cast<int64_t>(dp) * G;
             if (rest <= 0) continue;
@@ -556,18 +719,17 @@ bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan
                 if (rest * kblocks < ctas) continue;
                 const double share = static_cast<double>(rest) / ctas;                // tiles per CTA
                 const double gather = static_cast<double>(ctas) / rest + 1.0;         // parts of a shared tile, about
-                consider(dp, ctas, dp * (kblocks * stage + epi) + (share * kblocks + 1.0) * stage + epi + kFixBase +
-                                       gather * kFixPerPart * ((bn + 63) / 64));
+                consider(dp, ctas, 1, dp * (kblocks * stage + wait) + (share * kblocks + 1.0) * stage_ns(ctas) + store + kFixBase +
+                                          gather * kFixPerPart * ((bn + 31) / 32));
                 if (ctas == G) break;
             }
         }
     }
     if (!found) return false;
-    const size_t stage_bytes = kABytes + plan->bn * 128 + plan->nch * 2048;
-    int stages = static_cast<int>((kSmemBudget - 1024) / stage_bytes);
-    plan->stages = stages > kMaxStagesL ? kMaxStagesL : stages;
-    plan->smem = plan->stages * stage_bytes + 1024;
-    plan->grid = plan->dp_rounds > 0 && plan->tiles >= G ? G : (plan->dp_rounds > 0 ? plan->tiles : plan->sk_ctas);
+    plan->stages = ring_stages(plan->bn);
+    plan->smem = plan->stages * stage_bytes_of(plan->bn) + kStoreBytes + 1024;
+    plan->grid = plan->split > 1 ? plan->tiles * plan->split
+                 : plan->dp_rounds > 0 && plan->tiles >= G ? G : (plan->dp_rounds > 0 ? plan->tiles : plan->sk_ctas);
     plan->sk_base = plan->sk_ctas > 0 ? plan->dp_rounds * G : plan->tiles;
     plan->token_bytes = (static_cast<size_t>(plan->tiles_m) * kblocks * (plan->bn * 128 + plan->nch * 2048) + 255) / 256 * 256;
     plan->ticket_bytes = plan->sk_ctas ? (static_cast<size_t>(plan->tiles - plan->sk_base) * 4 + 255) / 256 * 256 : 0;
@@ -614,11 +776,21 @@ cudaError_t launch_with_pdl(int instance, const LargePlan& plan, const LargePara
     cfg.blockDim = dim3(kThreadsL);
     cfg.dynamicSmemBytes = plan.smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (plan.split > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(plan.split);
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (gemv_tuning().use_pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = gemv_tuning().use_pdl ? 1 : 0;
+    cfg.numAttrs = static_cast<unsigned>(n);
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
@@ -642,6 +814,7 @@ void fill_common(const LargePlan& plan, LargeParams* p, void* out, int M, int N,
     p->M = M; p->N = N;
     p->bn = plan.bn; p->nch = plan.nch; p->tiles = plan.tiles; p->tiles_m = plan.tiles_m;
     p->kblocks = plan.kblocks; p->k64 = K / 64; p->stages = plan.stages;
+    p->split = plan.split; p->split_cols = plan.split_cols;
     p->dp_rounds = plan.dp_rounds; p->sk_base = plan.sk_base; p->sk_ctas = plan.sk_ctas;
     if (plan.sk_ctas > 0) {
         const int total = (plan.tiles - plan.sk_base) * plan.kblocks;
@@ -718,10 +891,15 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
     p.x = tokens;
     p.tickets = reinterpret_cast<unsigned*>(tokens + plan.token_bytes);
     p.partials = reinterpret_cast<float*>(tokens + plan.token_bytes + plan.ticket_bytes);
-    const dim3 qgrid(static_cast<unsigned>(g.M), static_cast<unsigned>((g.K / kBlockElems + 255) / 256));
-    cudaError_t e = launch_small(quant_pack_kernel, qgrid, 256, stream, static_cast<const __nv_bfloat16*>(g.xb), g.xb_stride,
-                                 g.K, g.gs, g.rcp_mode == kRcpExact, tokens, plan.bn, plan.nch, plan.kblocks,
-                                 p.tickets, plan.tiles - plan.sk_base);
+    const unsigned pieces = static_cast<unsigned>((g.K / kBlockElems + 255) / 256);
+    const auto quant = [&](auto kern, int rows) {
+        return launch_small(kern, dim3(static_cast<unsigned>((g.M + rows - 1) / rows), pieces), 256, stream,
+                            static_cast<const __nv_bfloat16*>(g.xb), g.xb_stride, g.M, g.K, g.gs, g.rcp_mode == kRcpExact, tokens,
+                            plan.bn, plan.nch, plan.kblocks, p.tickets, plan.tiles - plan.sk_base);
+    };
+    // One row a CTA while the CTAs fit the device at once, four (and a quarter of the CTAs) beyond.
+    cudaError_t e = static_cast<int64_t>(g.M) * pieces <= 4 * device_sm_count() ? quant(quant_pack_kernel<1>, 1)
+                                                                             : quant(quant_pack_kernel<4>, 4);
     if (e != cudaSuccess) return e;
     return launch_with_pdl(g.out_dtype, plan, p, stream);
 }

@@ -81,6 +81,32 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
     asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(threads) : "memory");
 }
 
+// ---- thread-block clusters ----------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_id() {
+    uint32_t r;
+    asm("mov.u32 %0, %%clusterid.x;" : "=r"(r));
+    return r;
+}
+// Every thread of the cluster arrives; what was written before is seen behind it.
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// The address in CTA `rank` of the cluster that corresponds to this CTA's shared-memory address.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_st16(uint32_t addr, const float v[4]) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :: "r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+}
+
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups
 // 1024 B apart. Fields: start >> 4 in bits 0-13, stride-byte-offset >> 4 in bits 32-45,
 // fixed 1 in bit 46, swizzle mode 2 (128 B) in bits 61-63.

@@ -98,6 +98,30 @@ def test_whole_tiles_then_stream_k(capi, M, N, K, bn):
     assert not wksp[:16384].any()
 
 
+@pytest.mark.parametrize("parts", [2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("M,N,K,bn", [(1, 256, 2048, 16), (45, 384, 1920, 48), (100, 128, 4224, 112), (129, 640, 2304, 80),
+                                      (200, 256, 2176, 208), (300, 2560, 2048, 128)])
+def test_cluster_split(capi, M, N, K, bn, parts):
+    """One tile per cluster: more parts than 16-token columns to sum (parts without any), a ragged last part, shares of
+    K that differ by a block, a last block of half the steps, more clusters than fit at once."""
+    _tune(1, bn, parts)
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + parts)
+    a = _packed(capi, w, ws, xb.cuda(), gs, N)
+    assert torch.equal(a, _packed(capi, w, ws, xb.cuda(), gs, N))
+    assert rel_l2(a.cpu().numpy(), exact) <= 1e-5
+    assert rel_l2(_packed(capi, w, ws, xb.cuda(), gs, N, 0).double().cpu().numpy(), exact) <= 2.0 ** -8
+    if K % 256 or (M > bn and bn % 128):
+        return
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    wksp = torch.zeros(1 << 20, dtype=torch.int64, device="cuda")
+    for n_major in (True, False):
+        C = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=n_major)
+        got = C.double().cpu().numpy()
+        assert rel_l2(got.reshape(N, M).T if n_major else got, exact) <= 2.0 ** -11
+    assert not wksp.any()                                                  # no partial sums in memory
+
+
 @pytest.mark.parametrize("N,K,first", [(1536, 256, 13), (4096, 256, 17), (384, 256, 17), (256, 256, 25), (256, 384, 33)])
 def test_first_token_count_follows_the_shape(capi, N, K, first):
     """Both sides of the line between the decode kernel and this one, per shape class, give the same product."""
