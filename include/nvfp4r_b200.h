@@ -234,7 +234,7 @@ NVFP4R_API int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride,
 /* Debug/tuning of that kernel: fewest tokens it takes (0 = automatic), tokens per tile (a multiple
  * of 16 up to 256, 0 = automatic; nvfp4r_gemm rounds it up to a multiple of 128 where the tokens
  * need more than one tile), schedule (-1 automatic, 0 whole tiles, 1 stream-K, 2..8 clusters
- * of that many CTAs per tile). */
+ * of that many CTAs per tile, 9 pairs of SMs per tile). */
 NVFP4R_API int nvfp4r_set_gemm_large_tuning(int min_m, int tile_tokens, int stream_k);
 
 /* The same linear with the operator that PRODUCES its input fused into the prologue, so

@@ -415,8 +415,8 @@ int nvfp4r_linear_packed_scratch(const void* x, int64_t x_row_stride, int M, int
 }
 
 int nvfp4r_set_gemm_large_tuning(int min_m, int tile_tokens, int stream_k) {
-    if (min_m < 0 || tile_tokens < 0 || tile_tokens > 256 || tile_tokens % 16 || stream_k < -1 || stream_k > 8)
-        return fail(NVFP4R_ERR_INVALID_ARGUMENT, "gemm large tuning: min_m >= 0, tile_tokens 0..256 in 16s, stream_k -1..8");
+    if (min_m < 0 || tile_tokens < 0 || tile_tokens > 256 || tile_tokens % 16 || stream_k < -1 || stream_k > 9)
+        return fail(NVFP4R_ERR_INVALID_ARGUMENT, "gemm large tuning: min_m >= 0, tile_tokens 0..256 in 16s, stream_k -1..9");
     nvfp4r::set_large_tuning(min_m, tile_tokens, stream_k);
     return NVFP4R_OK;
 }

@@ -19,7 +19,7 @@
 //              512-byte chunks: the operands of the raw gemm operator.
 //
 // CTAs of ten warps, one per SM: warp 0 producer, warp 1 MMA issuer, warps 2-9 epilogue (two
-// per TMEM lane quadrant, each half of the columns). Three schedules, chosen by an estimate of the time:
+// per TMEM lane quadrant, each half of the columns). Four schedules, chosen by an estimate of the time:
 //   whole tiles  CTA c computes tiles c, c + G, ...
 //   stream-K     after the rounds of whole tiles the K blocks of the tiles that are left, laid end to end, are cut into
 //                one equal range for each of `sk_ctas` CTAs. A tile that two or more CTAs share is summed from fp32
@@ -30,16 +30,20 @@
 //                every CTA adds up and stores its own columns, in K order. The hardware places a cluster as a whole,
 //                so nothing waits for a CTA that might not be running, and no scratch is needed.
 //
+//   pairs        two SMs on one tile of 256 weight rows (cta_group::2): each holds its 128 rows and half of the tokens,
+//                36 KB a stage instead of 55 KB at 256 tokens; one of the two issues for both, the other announces
+//                its stages to it. For many tokens, where the bytes are the time.
+//
 // What bounds it. Few tiles: the chain launch - quantizer - launch - first stage - MMAs - stores, of which a K block is
 // 0.24 us: 515 clocks of the issuing warp (12 tcgen05 instructions at 17 to 25 clocks, a wait, a commit) against 218 for
 // the tensor pipe at 16 tokens. Many tokens: the bytes that the SMs take in from L2, 13 to 15 TB/s over all of them; MMAs
-// alone would run at 107 bytes a clock and SM, and the loads get 55 to 60.
+// alone would run at 107 bytes a clock and SM without pairing, 74 with, and the loads get 55 to 60.
 // The producer's addresses are worked out once per segment and it was 740 clocks a stage before, more than the issuer;
 // the issuer is straight-line code per K block (rolled loops made each tcgen05 instruction wait for its operands).
 // Device time in a CUDA graph, weights cold, us, one CTA a tile or stream-K with all of that before -> after:
-//   10240x5120  45 tokens 12.4 -> 10.1     6144x4096  333 tokens 13.9 -> 11.2     34816x5120  16 tokens 21.9 -> 19.8
-//   1024x4096   16 tokens 8.5 -> 6.1 (clusters of 4)    4096x12288 128 tokens, quant + gemm 21.3 -> 14.8 (clusters of 4)
-//   24576x4096  2048 tokens 104.9 -> 103.7
+//   10240x5120  45 tokens 12.4 -> 10.1     6144x4096  333 tokens 13.9 -> 11.2     34816x5120  16 tokens 21.9 -> 19.9
+//   1024x4096   16 tokens 8.5 -> 6.1 (clusters of 4)    4096x12288 128 tokens, quant + gemm 21.3 -> 14.9 (clusters of 4)
+//   24576x4096  512 tokens 32.5 -> 28.7, 1300 69.4 -> 57.0, 2048 104.9 -> 85 to 88 (pairs)
 #include <cuda.h>
 
 #include <algorithm>
@@ -63,22 +67,30 @@ constexpr int kACodes = kRows * 128;
 constexpr int kMaxStagesL = 8;
 constexpr int kEpiWarps = 8;
 constexpr int kThreadsL = (2 + kEpiWarps) * 32;
-constexpr int kStoreChunk = 16 * kRows * 2;          // 16 tokens x 128 rows of a 16-bit output on their way to memory
+constexpr int kStoreChunk = 32 * kRows * 2;          // 32 tokens x 128 rows of a 16-bit output on their way to memory
 constexpr int kStoreBytes = 2 * kStoreChunk;         // one for each column half
 constexpr int kSmemBudget = 225 * 1024;              // dynamic part, 1 KB of it for alignment
+constexpr int kPairTuning = 9;                       // set_large_tuning: pairs of SMs
 constexpr int kMaxSplit = 8;                         // the largest cluster that every device can place
 // Time model of plan_large, nanoseconds, fitted to sweeps over tile widths and schedules (eight weights, 16 .. 700
 // tokens). A K block costs the issuing warp 235 + 0.17 per token of the tile (30 more for the second chunk of token
 // scales), unless the SMs at work take in more than 15.5 TB/s from L2 together or the weight more than 6.3 TB/s from
-// memory. The last tile's stores take 10.5 per token, those of a tile before it 3 where the one accumulator waits.
+// memory. The last tile's stores take 10.5 per token, those of a tile before it 6,
+// beside the next tile's MMAs; where the accumulators overlap these wait 300.
 // A shared stream-K tile: partial stores, fence and ticket, then a trip to L2 per part and 32 columns. A cluster: two
 // cluster barriers, each CTA's partial sums sent to the peers and read back.
 constexpr double kStageBase = 235.0, kStagePerToken = 0.17, kStageChunk = 30.0, kL2Rate = 15500.0, kHbmRate = 6300.0;
-constexpr double kStorePerToken = 10.5, kStoreWait = 3.0, kFixBase = 2000.0, kFixPerPart = 400.0;
+constexpr double kStorePerToken = 10.5, kStoreWarm = 6.0, kStoreWait = 300.0, kFixBase = 2000.0, kFixPerPart = 400.0;
 constexpr double kSplitBase = 1100.0, kSplitPerToken = 12.0, kSplitPerPartToken = 2.2, kSecondWave = 3500.0;
+constexpr double kPairFix = 500.0;
 constexpr uint32_t kTmemColsL = 512;
-constexpr int kTwoAccTokens = 192;                   // widest tile with two accumulators
-constexpr uint32_t kColSfaL = 384, kColSfbL = 416;   // two buffers of 16, two of 32 columns
+// Tensor memory, 512 columns: two accumulators and the scales of a K block (16 + 32 columns; twice that, so that the next
+// block's copies pass the MMAs of this one, where the accumulators leave room). Two accumulators of more than 232 tokens
+// overlap: the tokens that both hold are stored first, then the next tile's MMAs may begin.
+constexpr int kTwoScales = 208, kNoOverlap = 232;
+__host__ __device__ constexpr int acc_stride(int bn) { return bn <= kTwoScales ? kTwoScales : bn <= kNoOverlap ? kNoOverlap : 2 * kNoOverlap - bn; }
+__host__ __device__ constexpr int acc_overlap(int bn) { return bn > kNoOverlap ? 2 * (bn - kNoOverlap) : 0; }
+constexpr uint32_t kColSfaL = 416, kColSfbL = 448, kColSfa1 = 464, kColSfb1 = 480;
 
 struct alignas(64) LargeParams {
     CUtensorMap map_w, map_x;                        // row-major form only
@@ -148,22 +160,24 @@ quant_pack_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, int
 struct Segment { int tile, k0, k1; };
 
 struct Walker {
-    int round = 0, cur, end;
-    __device__ __forceinline__ explicit Walker(const LargeParams& p) {
+    int round = 0, cur, end, unit, units;             // unit: this CTA, or its pair
+    __device__ __forceinline__ Walker(const LargeParams& p, bool pair) {
         const int c = blockIdx.x;
+        unit = pair ? c >> 1 : c;
+        units = pair ? gridDim.x / 2 : gridDim.x;
         cur = c * p.sk_q + min(c, p.sk_r);
         end = c < p.sk_ctas ? cur + p.sk_q + (c < p.sk_r ? 1 : 0) : cur;
     }
     __device__ __forceinline__ bool next(const LargeParams& p, Segment& s) {
         if (p.split > 1) {
-            const int part = static_cast<int>(cluster_ctarank());
-            s.tile = static_cast<int>(cluster_id());
+            s.tile = static_cast<int>(blockIdx.x) / p.split;
+            const int part = static_cast<int>(blockIdx.x) - s.tile * p.split;
             s.k0 = p.kblocks * part / p.split;
             s.k1 = p.kblocks * (part + 1) / p.split;
             return round++ == 0;
         }
         if (round < p.dp_rounds) {
-            s.tile = blockIdx.x + round * gridDim.x;
+            s.tile = unit + round * units;
             ++round;
             s.k0 = 0;
             s.k1 = p.kblocks;
@@ -188,18 +202,24 @@ __device__ __forceinline__ int sk_start(const LargeParams& p, int c) { return c 
 
 // One K block: the scale copies first, so that no MMA waits behind its own copy. Straight-line code with
 // compile-time counts: with rolled loops every instruction waits for its operands to reach uniform registers.
-template <int kChunks, int kSteps>
+template <int kChunks, int kSteps, bool kPair>
 __device__ __forceinline__ void issue_block(uint32_t d, uint64_t a, uint64_t b, uint64_t sa, uint64_t sb, uint32_t idesc,
                                             uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
+    const auto cp = [](uint32_t t, uint64_t desc) {
+        if (kPair) tc_cp_scales_pair(t, desc);
+        else tc_cp_scales(t, desc);
+    };
 #pragma unroll
     for (int k = 0; k < kSteps; ++k) {
-        tc_cp_scales(sfa + 4 * k, sa + 32 * k);
+        cp(sfa + 4 * k, sa + 32 * k);
 #pragma unroll
-        for (int j = 0; j < kChunks; ++j) tc_cp_scales(sfb + 4 * kChunks * k + 4 * j, sb + 128 * j + 32 * k);
+        for (int j = 0; j < kChunks; ++j) cp(sfb + 4 * kChunks * k + 4 * j, sb + 128 * j + 32 * k);
     }
 #pragma unroll
-    for (int k = 0; k < kSteps; ++k)
-        tc_mma_nvf4(d, a + 2 * k, b + 2 * k, idesc, sfa + 4 * k, sfb + 4 * kChunks * k, k == 0 ? accumulate : 1u);
+    for (int k = 0; k < kSteps; ++k) {
+        if (kPair) tc_mma_nvf4_pair(d, a + 2 * k, b + 2 * k, idesc, sfa + 4 * k, sfb + 4 * kChunks * k, k == 0 ? accumulate : 1u);
+        else tc_mma_nvf4(d, a + 2 * k, b + 2 * k, idesc, sfa + 4 * k, sfb + 4 * kChunks * k, k == 0 ? accumulate : 1u);
+    }
 }
 
 template <int kDtype>
@@ -212,11 +232,11 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Stores 16 accumulator columns (tokens m0 .. m0+15) of the tile's 128 rows; the four warps of a column half call it
-// together, each lane with its weight row n = n0 + row.
-//   N-major         a lane's 16 tokens are contiguous.
+// Stores kCols accumulator columns (tokens m0 .. m0 + kCols - 1) of the tile's 128 rows; the four warps of a column half
+// call it together, each lane with its weight row n = n0 + row.
+//   N-major         a lane's tokens are contiguous.
 //   M-major, fp32   the lanes of a warp write 128 contiguous bytes per token.
-//   M-major, 16-bit a warp's share of a token is 64 bytes: the half's 16 x 128 values meet in shared memory and leave
+//   M-major, 16-bit a warp's share of a token is 64 bytes: the half's values meet in shared memory and leave
 //                   in 16-byte pieces, 256 contiguous bytes per token. Straight from the registers (pairs of lanes
 //                   trading halves, 4 bytes a store) a tile of 128 x 112 took 2.4 us.
 struct Store {
@@ -224,47 +244,48 @@ struct Store {
     int half, row, align;
 };
 
-template <int kDtype, bool kNMajor>
-__device__ __forceinline__ void store16(const LargeParams& p, Store& st, int n0, int m0, float v[16]) {
+template <int kDtype, bool kNMajor, int kCols>
+__device__ __forceinline__ void store_cols(const LargeParams& p, const Store& st, int n0, int m0, float v[kCols]) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
+    for (int j = 0; j < kCols; ++j) v[j] *= p.alpha;
     if (kNMajor) {
         const int64_t at = static_cast<int64_t>(n0 + st.row) * p.ldc + m0;
         if (kDtype == 2) {
             float* o = static_cast<float*>(p.out) + at;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
+            for (int j = 0; j < kCols; ++j)
                 if (m0 + j < p.M) o[j] = v[j];
         } else {
             uint16_t* o = static_cast<uint16_t*>(p.out) + at;
-            uint32_t w[8];
+            uint32_t w[kCols / 2];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) w[j] = pack2<kDtype>(v[2 * j], v[2 * j + 1]);
-            if (st.align == 16 && m0 + 16 <= p.M) {
-                reinterpret_cast<uint4*>(o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                reinterpret_cast<uint4*>(o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            for (int j = 0; j < kCols / 2; ++j) w[j] = pack2<kDtype>(v[2 * j], v[2 * j + 1]);
+            if (st.align == 16 && m0 + kCols <= p.M) {
+#pragma unroll
+                for (int j = 0; j < kCols / 8; ++j)
+                    reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
+                for (int j = 0; j < kCols; ++j)
                     if (m0 + j < p.M) o[j] = static_cast<uint16_t>(j & 1 ? w[j >> 1] >> 16 : w[j >> 1]);
             }
         }
     } else if (kDtype == 2) {
         float* o = static_cast<float*>(p.out) + static_cast<int64_t>(m0) * p.ldc + n0 + st.row;
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
+        for (int j = 0; j < kCols; ++j)
             if (m0 + j < p.M) o[static_cast<int64_t>(j) * p.ldc] = v[j];
     } else {
         uint16_t* mine = reinterpret_cast<uint16_t*>(st.chunk) + st.row;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kCols / 2; ++j) {
             const uint32_t w = pack2<kDtype>(v[2 * j], v[2 * j + 1]);
             mine[2 * j * kRows] = static_cast<uint16_t>(w);
             mine[(2 * j + 1) * kRows] = static_cast<uint16_t>(w >> 16);
         }
         named_barrier(2 + st.half, kRows);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < kCols / 8; ++u) {
             const int token = u * 8 + (st.row >> 4), piece = st.row & 15;
             if (m0 + token >= p.M) break;
             const uint4 w = *reinterpret_cast<const uint4*>(st.chunk + token * (kRows * 2) + piece * 16);
@@ -284,29 +305,34 @@ __device__ __forceinline__ void store16(const LargeParams& p, Store& st, int n0,
                 }
             }
         }
-        named_barrier(2 + st.half, kRows);             // read before the next 16 tokens are written
+        named_barrier(2 + st.half, kRows);             // read before the next tokens are written
     }
 }
 
 // The issuing warp: all lanes walk, one elected lane issues.
-template <int kChunks>
+template <int kChunks, bool kPair>
 __device__ __forceinline__ void issue_all(const LargeParams& p, uint32_t ring, uint32_t tmem, uint32_t bar_full,
                                           uint32_t bar_empty, uint32_t bar_accfull, uint32_t bar_accempty, WaitFail& wf) {
     const bool lead = elect_one();
-    const uint32_t b_codes = static_cast<uint32_t>(p.bn) * 128u;
+    const uint32_t b_codes = static_cast<uint32_t>(p.bn) * (kPair ? 64u : 128u);
     const uint32_t stage_bytes = kABytes + b_codes + kChunks * 2048u;
-    const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.bn >> 3) << 17) | (1u << 27);
-    const int n_acc = p.bn <= kTwoAccTokens ? 2 : 1, stages = p.stages;
+    const uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.bn >> 3) << 17) | ((kPair ? 2u : 1u) << 27);
+    const int stages = p.stages, stride = acc_stride(p.bn);
+    const bool overlap = acc_overlap(p.bn) > 0, two_scales = p.bn <= kTwoScales;
+    const auto commit = [](uint32_t bar) {
+        if (kPair) tc_commit_pair(bar);
+        else tc_commit(bar);
+    };
     const int whole = p.k64 >> 2;                     // K % 256 == 128: the last block has two of four steps
-    Walker wk(p);
+    Walker wk(p, kPair);
     Segment sg;
     uint32_t s = 0, phase = 0, odd = 0;
     for (int t = 0; !wf.failed && wk.next(p, sg); ++t) {
-        const int buf = n_acc == 2 ? (t & 1) : 0;
-        const int use = n_acc == 2 ? (t >> 1) : t;    // how often this buffer was used before
-        if (use > 0 && !wf.wait(bar_accempty + 8 * buf, (use - 1) & 1)) break;
+        const int buf = t & 1;
+        // overlapping accumulators: one barrier, the tile before has left the tokens that both hold; else one per buffer
+        if (overlap ? t > 0 && !wf.wait(bar_accempty, (t - 1) & 1) : t > 1 && !wf.wait(bar_accempty + 8 * buf, ((t >> 1) - 1) & 1)) break;
         tc_fence_after();
-        const uint32_t d = tmem + buf * kTwoAccTokens;
+        const uint32_t d = tmem + buf * stride;
         uint32_t more = 0;
         for (int kb = sg.k0; kb < sg.k1; ++kb) {
             if (!wf.wait(bar_full + 8 * s, phase)) break;
@@ -314,23 +340,24 @@ __device__ __forceinline__ void issue_all(const LargeParams& p, uint32_t ring, u
             const uint32_t a_smem = ring + s * stage_bytes;
             const uint64_t a_desc = desc_operand(a_smem), b_desc = desc_operand(a_smem + kABytes);
             const uint64_t sa_desc = desc_scales(a_smem + kACodes), sb_desc = desc_scales(a_smem + kABytes + b_codes);
-            const uint32_t sfa = tmem + kColSfaL + odd * 16, sfb = tmem + kColSfbL + odd * 32;
+            const uint32_t sfa = tmem + (two_scales ? kColSfaL + odd * 16 : kColSfa1);
+            const uint32_t sfb = tmem + (two_scales ? kColSfbL + odd * 32 : kColSfb1);
             if (lead) {
-                if (kb < whole) issue_block<kChunks, 4>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
-                else issue_block<kChunks, 2>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
-                tc_commit(bar_empty + 8 * s);
+                if (kb < whole) issue_block<kChunks, 4, kPair>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
+                else issue_block<kChunks, 2, kPair>(d, a_desc, b_desc, sa_desc, sb_desc, idesc, sfa, sfb, more);
+                commit(bar_empty + 8 * s);
             }
             __syncwarp();
             more = 1;
             odd ^= 1u;
             if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
         }
-        if (lead) tc_commit(bar_accfull + 8 * buf);
+        if (lead) commit(bar_accfull + 8 * buf);
         __syncwarp();
     }
 }
 
-template <bool kTma, int kDtype, bool kNMajor>
+template <bool kTma, int kDtype, bool kNMajor, bool kPair>
 __global__ void __launch_bounds__(kThreadsL, 2)
 gemm_large_kernel(const __grid_constant__ LargeParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -341,21 +368,27 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bn = p.bn, stages = p.stages, nch = p.nch;
-    const uint32_t b_codes = static_cast<uint32_t>(bn) * 128u;
+    const uint32_t b_codes = static_cast<uint32_t>(bn) * (kPair ? 64u : 128u);      // a CTA of a pair holds half of the tokens
     const uint32_t stage_bytes = kABytes + b_codes + static_cast<uint32_t>(nch) * 2048u;
+    const int rank = kPair ? static_cast<int>(blockIdx.x & 1) : 0;                  // 0 issues for both
     const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = smem_u32(&bars[kMaxStagesL]);
     const uint32_t bar_accfull = smem_u32(&bars[2 * kMaxStagesL]), bar_accempty = bar_accfull + 16;
-    const int n_acc = bn <= kTwoAccTokens ? 2 : 1;
 
     if (warp == 0 && lane < 2 * kMaxStagesL + 4) {
-        mbar_init(bar_full + 8 * lane, lane >= 2 * kMaxStagesL + 2 ? kEpiWarps : 1);
+        // a pair: the issuing CTA's stages are full when the peer's are too, its accumulators empty when both are
+        const bool acc_empty = lane >= 2 * kMaxStagesL + 2;
+        mbar_init(bar_full + 8 * lane, acc_empty ? (kPair ? 2 : 1) * kEpiWarps : kPair && rank == 0 && lane < kMaxStagesL ? 2 : 1);
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(&s_tmem), kTmemColsL);
+    if (warp == 1) {
+        if (kPair) tmem_alloc_pair(smem_u32(&s_tmem), kTmemColsL);
+        else tmem_alloc(smem_u32(&s_tmem), kTmemColsL);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    if (kPair) cluster_sync_all();                     // the peer's barriers exist
     pdl_launch_dependents();
 
     WaitFail wf;
@@ -365,7 +398,7 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
         // tokens are read by every column of tiles, a weight tile by tiles_m CTAs at about the same time
         const uint64_t keep = l2_policy_evict_last();
         const uint64_t policy = p.tiles_m > 1 ? l2_policy_evict_normal() : l2_policy_evict_first();
-        const uint32_t b_bytes = b_codes + static_cast<uint32_t>(nch) * 2048u;
+        const uint32_t b_bytes = static_cast<uint32_t>(bn) * 128u + static_cast<uint32_t>(nch) * 2048u;      // in memory
         // Where a segment's operands lie, worked out once per segment: with the divisions and products in the block
         // loop a stage cost this warp 740 clocks, more than its MMAs.
         struct Source {
@@ -373,14 +406,16 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
             int ax, ay, by, ch;                       // row-major: code coordinates, scale chunks of the token tile
         };
         auto source = [&](const Segment& sg) {
-            const int nt = sg.tile / p.tiles_m, mt = sg.tile - nt * p.tiles_m;
+            const int t = sg.tile / p.tiles_m, mt = sg.tile - t * p.tiles_m;
+            // with an odd number of row tiles the last pair's second CTA repeats the first one's and stores nothing
+            const int nt = kPair ? min(2 * t + rank, (p.N / kRows) - 1) : t;
             Source o;
             if (kTma) {
                 o.a = p.wsf + (static_cast<int64_t>(nt) * p.k64 + sg.k0 * 4) * 512;
                 o.b = p.xsf + (static_cast<int64_t>(mt * nch) * p.k64 + sg.k0 * 4) * 512;
                 o.ax = sg.k0 * 128;
                 o.ay = nt * kRows;
-                o.by = mt * bn;
+                o.by = mt * bn + rank * (bn / 2);
                 o.ch = min(nch, (p.M - mt * bn + 127) >> 7);          // chunks that exist in xsf
             } else {
                 o.a = p.w + (static_cast<int64_t>(nt) * p.kblocks + sg.k0) * kABytes;
@@ -403,6 +438,9 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
                 tma_load_2d(dst, &p.map_x, o.ax, o.by, bar, keep);
                 for (int j = 0; j < o.ch; ++j)
                     bulk_g2s(dst + b_codes + j * 2048, o.b + static_cast<int64_t>(j) * p.k64 * 512, 2048, bar, keep);
+            } else if (kPair) {
+                bulk_g2s(dst, o.b + rank * static_cast<int>(b_codes), b_codes, bar, keep);
+                bulk_g2s(dst + b_codes, o.b + 2 * b_codes, b_bytes - 2 * b_codes, bar, keep);
             } else {
                 bulk_g2s(dst, o.b, b_bytes, bar, keep);
             }
@@ -416,7 +454,7 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
         // requested ahead of the wait, the token half behind it.
         int pre = 0;
         {
-            Walker wa(p);
+            Walker wa(p, kPair);
             Segment sa;
             uint32_t dst = ring, bar = bar_full;
             while (pre < stages && wa.next(p, sa)) {
@@ -431,7 +469,7 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
             }
         }
         pdl_wait_prior();
-        Walker wk(p);
+        Walker wk(p, kPair);
         Segment sg;
         int i = 0;
         uint32_t s = 0, phase = 1, dst = ring;        // phase the empty barrier must have completed
@@ -449,12 +487,38 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
                 if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; dst = ring; }
             }
         }
+        if (kPair) {
+            // the last stages are handed back by the issuing CTA: this one stays until it has heard of it
+            const int last = min(i, stages);
+            if (i < stages) { s = 0; phase = 0; }
+            for (int j = 0; j < last; ++j) {
+                if (!wf.wait(bar_empty + 8 * s, phase)) break;
+                if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
+            }
+        }
         if (wf.failed)                                 // let the copies in flight land before the CTA goes
             for (int j = max(0, i - stages); j < i; ++j) mbar_wait_bounded(bar_full + 8 * (j % stages), (j / stages) & 1, 100000u);
     } else if (warp == 1) {
         // ---------------- MMA issuer -----------------------------------------------------------
-        if (nch == 1) issue_all<1>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
-        else issue_all<2>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
+        if (kPair && rank != 0) {
+            // the peer's stages are announced to the issuing CTA
+            const bool lead = elect_one();
+            const uint32_t there = cluster_map(bar_full, 0);
+            Walker wk(p, kPair);
+            Segment sg;
+            uint32_t s = 0, phase = 0;
+            while (!wf.failed && wk.next(p, sg))
+                for (int kb = sg.k0; kb < sg.k1; ++kb) {
+                    if (!wf.wait(bar_full + 8 * s, phase)) break;
+                    if (lead) mbar_arrive_cluster(there + 8 * s);
+                    __syncwarp();
+                    if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
+                }
+        } else if (nch == 1) {
+            issue_all<1, kPair>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
+        } else {
+            issue_all<2, kPair>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
+        }
     } else {
         // ---------------- epilogue (warps 2..9) ------------------------------------------------
         pdl_wait_prior();                              // out, partials and tickets may still be in use before it
@@ -462,45 +526,49 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
         const int row = q * 32 + lane;
         const int cols_half = (((bn >> 4) + 1) >> 1) << 4;
         const int c_lo = half ? cols_half : 0, groups = (half ? bn - cols_half : cols_half) >> 4;
+        const bool overlap = acc_overlap(bn) > 0;
         const uintptr_t out_at = reinterpret_cast<uintptr_t>(p.out) | (kDtype == 2 ? 0 : static_cast<uintptr_t>(p.ldc) * 2);
         Store st;
         st.chunk = smem_raw + (ring + stages * stage_bytes - smem_u32(smem_raw)) + half * kStoreChunk;
         st.half = half;
         st.row = row;
         st.align = (out_at & 15) == 0 ? 16 : (out_at & 3) == 0 ? 4 : 2;
-        Walker wk(p);
+        Walker wk(p, kPair);
         Segment sg;
-        // Rolled loops of 16 columns: a tile's columns leave the tensor memory at the pace of the stores. Unrolled over
+        // Rolled loops of 16 or 32 columns: a tile's columns leave the tensor memory at the pace of the stores. Unrolled over
         // the tile (all of it in registers first) the code was fetched cold once per launch, and 200 registers a thread
         // left no room for these CTAs beside the quantizer's.
         for (int t = 0; wk.next(p, sg); ++t) {
-            const int buf = n_acc == 2 ? (t & 1) : 0;
-            const int use = n_acc == 2 ? (t >> 1) : t;
+            const int buf = t & 1;
             const int nt = sg.tile / p.tiles_m, mt = sg.tile - nt * p.tiles_m;
-            const int n0 = nt * kRows, m0 = mt * bn;
-            wf.wait(bar_accfull + 8 * buf, use & 1);   // after a time-out: walk on, the warps meet at barriers below
+            const int n0 = (kPair ? 2 * nt + rank : nt) * kRows, m0 = mt * bn;
+            wf.wait(bar_accfull + 8 * buf, (t >> 1) & 1);   // after a time-out: walk on, the warps meet at barriers below
             tc_fence_after();
-            const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * kTwoAccTokens + c_lo;
-            auto release = [&] {                       // the next tile's MMAs may have the accumulator
+            const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * acc_stride(bn) + c_lo;
+            auto release = [&] {                       // the next tile's MMAs may have what was read
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_accempty + 8 * buf);
+                if (lane == 0) {
+                    const uint32_t bar = bar_accempty + (overlap ? 0 : 8 * buf);
+                    if (kPair) mbar_arrive_cluster(cluster_map(bar, 0));
+                    else mbar_arrive(bar);
+                }
             };
             float v[16];
-            if (p.split > 1) {
-                const int S = p.split, w = p.split_cols, rank = static_cast<int>(cluster_ctarank());
+            if (!kPair && p.split > 1) {
+                const int S = p.split, w = p.split_cols, part = static_cast<int>(blockIdx.x) % S;
                 cluster_sync_all();                    // every CTA of the cluster is through with its ring
 #pragma unroll 1
                 for (int g = 0; g < groups; ++g) {
                     tmem_ld16(taddr + 16 * g, v);
                     tmem_ld_wait();
                     const int col = c_lo + 16 * g, owner = col / w;
-                    const uint32_t dst = cluster_map(ring + ((rank * w + col - owner * w) * kRows + row * 4) * 4, owner);
+                    const uint32_t dst = cluster_map(ring + ((part * w + col - owner * w) * kRows + row * 4) * 4, owner);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) cluster_st16(dst + j * (kRows * 16), v + 4 * j);
                 }
                 cluster_sync_all();
-                const int mine = min(w, bn - rank * w);
+                const int mine = min(w, bn - part * w);
 #pragma unroll 1
                 for (int c = 16 * half; c < mine; c += 32) {
                     const float4* src = reinterpret_cast<const float4*>(smem_raw + (ring - smem_u32(smem_raw))) +
@@ -516,19 +584,30 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
                             v[4 * j + 3] = r ? v[4 * j + 3] + x.w : x.w;
                         }
                     }
-                    store16<kDtype, kNMajor>(p, st, n0, m0 + rank * w + c, v);
+                    store_cols<kDtype, kNMajor, 16>(p, st, n0, m0 + part * w + c, v);
                 }
                 continue;
             }
-            if (sg.k1 - sg.k0 == p.kblocks) {
+            if (kPair || sg.k1 - sg.k0 == p.kblocks) {
+                // Whole tile, 32 columns at a time, from the end that the other accumulator overlaps. A half is through with
+                // the overlap after `free_at` columns (none: its last tile is drained, this one's need not be); without
+                // overlap the accumulator is handed back when all of it has been read.
+                const int free_at = !overlap ? 16 * groups : half == buf ? 0 : acc_overlap(bn);
+                if (free_at == 0) release();
+                int done = 0;
 #pragma unroll 1
-                for (int g = 0; g < groups; ++g) {
-                    tmem_ld16(taddr + 16 * g, v);
+                while (done < 16 * groups) {
+                    const int n = min(32, 16 * groups - done), at = overlap && buf == 0 ? 16 * groups - done - n : done;
+                    float u[32];
+                    tmem_ld16(taddr + at, u);
+                    if (n == 32) tmem_ld16(taddr + at + 16, u + 16);
                     tmem_ld_wait();
-                    if (g == groups - 1) release();
-                    store16<kDtype, kNMajor>(p, st, n0, m0 + c_lo + 16 * g, v);
+                    if (done < free_at && done + n >= free_at) release();
+                    done += n;
+                    if (kPair && n0 >= p.N) continue;
+                    if (n == 32) store_cols<kDtype, kNMajor, 32>(p, st, n0, m0 + c_lo + at, u);
+                    else store_cols<kDtype, kNMajor, 16>(p, st, n0, m0 + c_lo + at, u);
                 }
-                if (groups == 0) release();
                 continue;
             }
             // stream-K: leave the partial sums, the last CTA of the tile to arrive adds all of them
@@ -572,14 +651,14 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
                             v[4 * j + 3] = c != first ? v[4 * j + 3] + x.w : x.w;
                         }
                     }
-                    store16<kDtype, kNMajor>(p, st, n0, m0 + c_lo + 16 * g, v);
+                    store_cols<kDtype, kNMajor, 16>(p, st, n0, m0 + c_lo + 16 * g, v);
                 }
             }
             named_barrier(1, kEpiWarps * 32);          // s_last is written again for the next shared tile
         }
     }
     // the epilogue's two cluster barriers: all warps of all CTAs take part
-    if (p.split > 1 && warp < 2) {
+    if (!kPair && p.split > 1 && warp < 2) {
         cluster_sync_all();
         cluster_sync_all();
     }
@@ -587,9 +666,11 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
     if (wf.failed && lane == 0) report_timeout(&g_large_status, 6);
     tc_fence_before();
     __syncthreads();
+    if (kPair) cluster_sync_all();                     // neither leaves while the other may still reach into it
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, kTmemColsL);
+        if (kPair) tmem_dealloc_pair(tmem, kTmemColsL);
+        else tmem_dealloc(tmem, kTmemColsL);
     }
 }
 
@@ -627,14 +708,15 @@ bool code_map(const void* p, int rows, int K, int box_rows, CUtensorMap* out) {
 struct LargePlan {
     int bn, nch, tiles_m, tiles, kblocks, stages, grid;
     int dp_rounds, sk_base, sk_ctas, split, split_cols;
+    bool pair;
     size_t smem, token_bytes, ticket_bytes, partial_bytes;
 };
 
 int g_large_bn = 0, g_large_sk = -1, g_large_min_m = 0;
 
-size_t stage_bytes_of(int bn) { return kABytes + bn * 128 + (bn + 127) / 128 * 2048; }
-int ring_stages(int bn) {
-    const int n = static_cast<int>((kSmemBudget - 1024 - kStoreBytes) / stage_bytes_of(bn));
+size_t stage_bytes_of(int bn, bool pair = false) { return kABytes + bn * (pair ? 64 : 128) + (bn + 127) / 128 * 2048; }
+int ring_stages(int bn, bool pair = false) {
+    const int n = static_cast<int>((kSmemBudget - 1024 - kStoreBytes) / stage_bytes_of(bn, pair));
     return n > kMaxStagesL ? kMaxStagesL : n;
 }
 
@@ -645,7 +727,7 @@ int cluster_capacity(int S, int G) {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return G / S;
     int n = known[dev][S].load(std::memory_order_relaxed);
     if (n == 0) {
-        const auto kern = gemm_large_kernel<false, 0, false>;
+        const auto kern = gemm_large_kernel<false, 0, false, false>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(G / S * S));
         cfg.blockDim = dim3(kThreadsL);
@@ -686,20 +768,28 @@ bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan
             const double issue = kStageBase + kStagePerToken * bn + (nch - 1) * kStageChunk;
             return std::max(issue, static_cast<double>(stage_bytes_of(bn)) * std::min<int64_t>(ctas, G) / kL2Rate);
         };
-        const double stage = stage_ns(tiles), wait = bn > kTwoAccTokens ? kStoreWait * bn : 0.0;
+        const double stage = stage_ns(tiles), wait = acc_overlap(bn) > 0 ? kStoreWait : 0.0;
         const int full = static_cast<int>(tiles / G);
-        auto consider = [&](int dp, int ctas, int split, double t) {
+        auto consider = [&](int dp, int ctas, int split, double t, bool pair = false) {
             t = std::max(t, floor_ns + store);
             if (t >= best) return;
             best = t;
             found = true;
             plan->bn = bn; plan->nch = nch; plan->tiles_m = tiles_m; plan->tiles = static_cast<int>(tiles);
             plan->kblocks = kblocks; plan->dp_rounds = dp; plan->sk_ctas = ctas;
+            plan->pair = pair;
             plan->split = split; plan->split_cols = (bn / 16 + split - 1) / split * 16;
         };
-        if (g_large_sk <= 0 || (g_large_sk > 1 && kblocks < g_large_sk)) {
+        if (g_large_sk < 0 || g_large_sk == kPairTuning) {
+            const int64_t pairs = static_cast<int64_t>(tiles_m) * ((tiles_n + 1) / 2);
+            const int at_once = cluster_capacity(2, G), rounds = static_cast<int>((pairs + at_once - 1) / at_once);
+            const double bytes = static_cast<double>(stage_bytes_of(bn, true)) * 2 * std::min<int64_t>(pairs, at_once);
+            const double block = std::max(kStageBase + kStagePerToken * bn + (nch - 1) * kStageChunk, bytes / kL2Rate);
+            consider(rounds, 0, 1, rounds * std::max(kblocks * block, kStoreWarm * bn) + (rounds - 1) * wait + store + kPairFix, true);
+        }
+        if (g_large_sk <= 0 || (g_large_sk > 1 && g_large_sk <= kMaxSplit && kblocks < g_large_sk)) {
             const int rounds = static_cast<int>((tiles + G - 1) / G);
-            consider(rounds, 0, 1, rounds * kblocks * stage + (rounds - 1) * wait + store);
+            consider(rounds, 0, 1, rounds * std::max(kblocks * stage, kStoreWarm * bn) + (rounds - 1) * wait + store);
         }
         for (int S = 2; S <= kMaxSplit && g_large_sk != 0 && g_large_sk != 1; ++S) {
             if (kblocks < S || (g_large_sk > 1 && S != g_large_sk)) continue;
@@ -726,9 +816,12 @@ bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan
         }
     }
     if (!found) return false;
-    plan->stages = ring_stages(plan->bn);
-    plan->smem = plan->stages * stage_bytes_of(plan->bn) + kStoreBytes + 1024;
-    plan->grid = plan->split > 1 ? plan->tiles * plan->split
+    plan->stages = ring_stages(plan->bn, plan->pair);
+    plan->smem = plan->stages * stage_bytes_of(plan->bn, plan->pair) + kStoreBytes + 1024;
+    if (plan->pair) {
+        plan->tiles = plan->tiles_m * ((tiles_n + 1) / 2);
+        plan->grid = 2 * std::min(plan->tiles, cluster_capacity(2, G));
+    } else plan->grid = plan->split > 1 ? plan->tiles * plan->split
                  : plan->dp_rounds > 0 && plan->tiles >= G ? G : (plan->dp_rounds > 0 ? plan->tiles : plan->sk_ctas);
     plan->sk_base = plan->sk_ctas > 0 ? plan->dp_rounds * G : plan->tiles;
     plan->token_bytes = (static_cast<size_t>(plan->tiles_m) * kblocks * (plan->bn * 128 + plan->nch * 2048) + 255) / 256 * 256;
@@ -753,14 +846,17 @@ bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
 
 using Kern = void (*)(LargeParams);
 
-constexpr int kInstances = 9;
+constexpr int kInstances = 18;
 
-cudaError_t launch_with_pdl(int instance, const LargePlan& plan, const LargeParams& p, cudaStream_t stream) {
-    // packed operands, then row-major ones with M-major and with N-major output; bf16, fp16, fp32
-    static const Kern table[kInstances] = {
-        gemm_large_kernel<false, 0, false>, gemm_large_kernel<false, 1, false>, gemm_large_kernel<false, 2, false>,
-        gemm_large_kernel<true, 0, false>, gemm_large_kernel<true, 1, false>, gemm_large_kernel<true, 2, false>,
-        gemm_large_kernel<true, 0, true>, gemm_large_kernel<true, 1, true>, gemm_large_kernel<true, 2, true>};
+cudaError_t launch_with_pdl(int form, const LargePlan& plan, const LargeParams& p, cudaStream_t stream) {
+    // packed operands, then row-major ones with M-major and with N-major output; bf16, fp16, fp32; by one CTA, by a pair
+#define NVFP4R_FORMS(PAIR)                                                                                             \
+    gemm_large_kernel<false, 0, false, PAIR>, gemm_large_kernel<false, 1, false, PAIR>, gemm_large_kernel<false, 2, false, PAIR>, \
+    gemm_large_kernel<true, 0, false, PAIR>, gemm_large_kernel<true, 1, false, PAIR>, gemm_large_kernel<true, 2, false, PAIR>,    \
+    gemm_large_kernel<true, 0, true, PAIR>, gemm_large_kernel<true, 1, true, PAIR>, gemm_large_kernel<true, 2, true, PAIR>
+    static const Kern table[kInstances] = {NVFP4R_FORMS(false), NVFP4R_FORMS(true)};
+#undef NVFP4R_FORMS
+    const int instance = form + (plan.pair ? kInstances / 2 : 0);
     const Kern kern = table[instance];
     static std::atomic<bool> attr_done[kInstances][64] = {};
     int dev = 0;
@@ -778,9 +874,9 @@ cudaError_t launch_with_pdl(int instance, const LargePlan& plan, const LargePara
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (plan.split > 1) {
+    if (plan.split > 1 || plan.pair) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = static_cast<unsigned>(plan.split);
+        attr[n].val.clusterDim.x = static_cast<unsigned>(plan.pair ? 2 : plan.split);
         attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
         ++n;
     }
@@ -826,9 +922,6 @@ void fill_common(const LargePlan& plan, LargeParams* p, void* out, int M, int N,
 
 }  // namespace
 
-// Tokens from which the row-major operands of the raw gemm operator take this path.
-constexpr int kLargeMinM = 33;
-
 // Tokens from which the packed linear takes it, where the caller can give it scratch: the device's side of the
 // choice. Up to 16 tokens the decode kernel makes one pass over the weight as well and needs no second launch; its
 // CTAs each quantize the tokens of their K part, which grows with the tokens, while this path pays a few us for
@@ -840,7 +933,7 @@ constexpr int kLargeMinM = 33;
 //   below          4096x12288: 24 tokens 13.2 / 15.7, 32 tokens 15.7 / 15.7; 1280x5120: 32 tokens 9.6 / 11.2
 int large_min_m(int N, int K) {
     const int64_t n = N, k = K;
-    return n >= 6 * k && n < 16 * k ? 13 : 2 * n >= 3 * k ? 17 : n >= k ? 25 : kLargeMinM;
+    return n >= 6 * k && n < 16 * k ? 13 : 2 * n >= 3 * k ? 17 : n >= k ? 25 : 33;
 }
 
 // What the entry point takes.
@@ -909,11 +1002,10 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
 cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* taken) {
     *taken = false;
     LargePlan plan;
-    if (g.xb != nullptr || g.M < (g_large_min_m ? g_large_min_m : kLargeMinM) || !plan_large(g.M, g.N, g.K, true, &plan))
-        return cudaSuccess;
+    if (g.xb != nullptr || g.M < (g_large_min_m ? g_large_min_m : 33) || !plan_large(g.M, g.N, g.K, true, &plan)) return cudaSuccess;
     LargeParams p = {};
     fill_common(plan, &p, g.out, g.M, g.N, g.K, g.alpha, g.c_n_major);
-    if (!code_map(g.w, g.N, g.K, kRows, &p.map_w) || !code_map(g.a_codes, g.M, g.K, plan.bn, &p.map_x)) return cudaSuccess;
+    if (!code_map(g.w, g.N, g.K, kRows, &p.map_w) || !code_map(g.a_codes, g.M, g.K, plan.pair ? plan.bn / 2 : plan.bn, &p.map_x)) return cudaSuccess;
     p.wsf = static_cast<const uint8_t*>(g.wsf_swizzled);
     p.xsf = static_cast<const uint8_t*>(g.a_sf_swizzled);
     // The workspace, tickets included, is shared with the decode-sized kernel: both leave the tickets zero.

@@ -65,6 +65,35 @@ __device__ __forceinline__ void tc_mma_nvf4(uint32_t d_tmem, uint64_t a_desc, ui
         :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem),
            "r"(accumulate) : "memory");
 }
+// The same for a pair of CTAs (cta_group::2): one of the two issues, tensor memory and shared memory of both take part.
+// Allocation and release are executed by one warp of each CTA.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_dst), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(taddr), "r"(cols) : "memory");
+}
+// Arrives at the barrier of that address in both CTAs.
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 :: "r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+}
+// Each CTA's tensor memory from its own shared memory.
+__device__ __forceinline__ void tc_cp_scales_pair(uint32_t taddr, uint64_t desc) {
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" :: "r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void tc_mma_nvf4_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                 uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem,
+                                                 uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X "
+        "[%0], %1, %2, %3, [%4], [%5], p;\n\t}"
+        :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem),
+           "r"(accumulate) : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -82,16 +111,6 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
 }
 
 // ---- thread-block clusters ----------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_id() {
-    uint32_t r;
-    asm("mov.u32 %0, %%clusterid.x;" : "=r"(r));
-    return r;
-}
 // Every thread of the cluster arrives; what was written before is seen behind it.
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -124,6 +143,13 @@ __device__ __forceinline__ uint64_t desc_scales(uint32_t smem_addr) {
 __device__ __forceinline__ uint32_t swz128(int row, int b) {
     return static_cast<uint32_t>((row >> 3) * 1024 + (row & 7) * 128 +
                                  ((((b >> 4) ^ (row & 7)) << 4) | (b & 15)));
+}
+
+// Arrives at another CTA's barrier. Nothing that this thread wrote through the generic proxy is handed over by it (stages
+// are written by the bulk copies that its own barrier counted, accumulators are ordered by the tcgen05 fences); the
+// cluster-scope release and acquire cost the pair's issuing loop 1100 clocks a stage.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
 }
 
 struct WaitFail {

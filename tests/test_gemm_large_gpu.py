@@ -122,6 +122,29 @@ def test_cluster_split(capi, M, N, K, bn, parts):
     assert not wksp.any()                                                  # no partial sums in memory
 
 
+@pytest.mark.parametrize("M,N,K,bn", [(1, 128, 256, 16), (45, 384, 640, 48), (200, 256, 4224, 208), (300, 2560, 2048, 256),
+                                      (257, 20480, 512, 128), (600, 10368, 896, 192),
+                                      (700, 10368, 1280, 240), (1000, 10240, 768, 256), (1000, 10240, 768, 224)])
+def test_pairs_of_sms(capi, M, N, K, bn):
+    """Two CTAs on one tile of 256 weight rows: an odd number of row tiles (the last pair has one), more pairs than fit at
+    once with accumulators side by side and overlapping (by 16 and 48 tokens), a last block of half the steps, fewer blocks than stages."""
+    _tune(1, bn, 9)
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + bn)
+    a = _packed(capi, w, ws, xb.cuda(), gs, N)
+    assert torch.equal(a, _packed(capi, w, ws, xb.cuda(), gs, N))
+    assert rel_l2(a.cpu().numpy(), exact) <= 1e-5
+    assert rel_l2(_packed(capi, w, ws, xb.cuda(), gs, N, 0).double().cpu().numpy(), exact) <= 2.0 ** -8
+    if K % 256 or (M > bn and bn % 128):
+        return
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    wksp = torch.zeros(1 << 20, dtype=torch.int64, device="cuda")
+    for n_major in (True, False):
+        C = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=n_major)
+        got = C.double().cpu().numpy()
+        assert rel_l2(got.reshape(N, M).T if n_major else got, exact) <= 2.0 ** -11
+
+
 @pytest.mark.parametrize("N,K,first", [(1536, 256, 13), (4096, 256, 17), (384, 256, 17), (256, 256, 25), (256, 384, 33)])
 def test_first_token_count_follows_the_shape(capi, N, K, first):
     """Both sides of the line between the decode kernel and this one, per shape class, give the same product."""
