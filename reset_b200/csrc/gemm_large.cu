@@ -234,7 +234,9 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 
 // Stores kCols accumulator columns (tokens m0 .. m0 + kCols - 1) of the tile's 128 rows; the four warps of a column half
 // call it together, each lane with its weight row n = n0 + row.
-//   N-major         a lane's tokens are contiguous.
+//   N-major         a lane's tokens are contiguous. Where rows are not 16-byte aligned (16-bit output, M % 8 != 0) a warp
+//                   turns its 32 rows in shared memory and writes row by row: 32 single stores of a lane each went to 32
+//                   rows at once (16384x2048 with 333 tokens 61 us, with 1000 tokens 24).
 //   M-major, fp32   the lanes of a warp write 128 contiguous bytes per token.
 //   M-major, 16-bit a warp's share of a token is 64 bytes: the half's values meet in shared memory and leave
 //                   in 16-byte pieces, 256 contiguous bytes per token. Straight from the registers (pairs of lanes
@@ -265,9 +267,27 @@ __device__ __forceinline__ void store_cols(const LargeParams& p, const Store& st
                 for (int j = 0; j < kCols / 8; ++j)
                     reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
             } else {
+                // [row][token pair], 16 words a row, pairs of rows rotated so that neither side meets a bank twice
+                const int lane = st.row & 31;
+                uint32_t* turn = reinterpret_cast<uint32_t*>(st.chunk) + (st.row - lane) * 16;
 #pragma unroll
-                for (int j = 0; j < kCols; ++j)
-                    if (m0 + j < p.M) o[j] = static_cast<uint16_t>(j & 1 ? w[j >> 1] >> 16 : w[j >> 1]);
+                for (int j = 0; j < kCols / 2; ++j) turn[lane * 16 + (j ^ (lane >> 1))] = w[j];
+                __syncwarp();
+                uint16_t* first = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(n0 + st.row - lane) * p.ldc + m0;
+                if (st.align >= 4) {                   // M even
+                    const int pair = lane & 15;
+                    if (pair < kCols / 2 && m0 + 2 * pair < p.M)
+#pragma unroll 4
+                        for (int i = 0; i < 16; ++i) {
+                            const int r = 2 * i + (lane >> 4);
+                            *reinterpret_cast<uint32_t*>(first + r * p.ldc + 2 * pair) = turn[r * 16 + (pair ^ i)];
+                        }
+                } else if (lane < kCols && m0 + lane < p.M) {
+#pragma unroll 4
+                    for (int r = 0; r < 32; ++r)
+                        first[r * p.ldc + lane] = reinterpret_cast<const uint16_t*>(turn + r * 16 + ((lane >> 1) ^ (r >> 1)))[lane & 1];
+                }
+                __syncwarp();
             }
         }
     } else if (kDtype == 2) {
@@ -997,12 +1017,18 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
     return launch_with_pdl(g.out_dtype, plan, p, stream);
 }
 
-// The raw operator on row-major operands. *taken stays false (nothing launched) where the workspace
-// does not hold what this path needs or a tensor map cannot be made: the caller's other kernel runs.
+// The raw operator on row-major operands, any number of tokens. The decode-sized kernel keeps the tokens of a K part in
+// shared memory and asks for the weight in one 16 KB tensor-map request a stage from a single lane; fp16 N-major output,
+// device us, that kernel / this one: 4864x7168 1 token 21.1 / 7.7, 32 tokens 47.4 / 7.9; 4096x4096 1 token 13.7 / 5.9;
+// 640x1024 1 token 6.1 / 3.3; 1920x11264 1 token 10.6 / 7.2. With fp32 output it stays up to 32 tokens: there
+// nvfp4r_linear_tc, which quantizes the tokens itself, is bound to give the same bits.
+// *taken stays false (nothing launched) where the workspace does not hold what this path needs or a tensor map cannot be
+// made: the caller's other kernel runs.
 cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* taken) {
     *taken = false;
     LargePlan plan;
-    if (g.xb != nullptr || g.M < (g_large_min_m ? g_large_min_m : 33) || !plan_large(g.M, g.N, g.K, true, &plan)) return cudaSuccess;
+    if (g.xb != nullptr || g.M < g_large_min_m || (g.M <= 32 && (tc_tuned() || g.out_dtype == NVFP4R_F32))) return cudaSuccess;
+    if (!plan_large(g.M, g.N, g.K, true, &plan)) return cudaSuccess;
     LargeParams p = {};
     fill_common(plan, &p, g.out, g.M, g.N, g.K, g.alpha, g.c_n_major);
     if (!code_map(g.w, g.N, g.K, kRows, &p.map_w) || !code_map(g.a_codes, g.M, g.K, plan.pair ? plan.bn / 2 : plan.bn, &p.map_x)) return cudaSuccess;

@@ -558,6 +558,8 @@ void set_tc_tuning(int splits, int stages) {
     g_force_stages = stages;
 }
 
+bool tc_tuned() { return g_force_splits > 0 || g_force_stages > 0; }
+
 cudaError_t set_status_mirror_tc(int* p) { return set_status_mirror_here(p); }
 
 cudaError_t read_and_clear_tc_status(int* flag) {

@@ -125,6 +125,7 @@ cudaError_t launch_linear_tc(const TcLinearArgs& g, cudaStream_t stream, const c
 cudaError_t read_and_clear_tc_status(int* flag);
 // 0 = automatic
 void set_tc_tuning(int splits, int stages);
+bool tc_tuned();             // a split or stage count is asked for: nvfp4r_gemm keeps to this kernel up to 32 rows
 
 // ---- linear_packed.cu -----------------------------------------------------
 struct PackedLinearArgs {

@@ -269,6 +269,25 @@ def test_gemm_row_major_tiles_start_at_a_scale_chunk(capi, M, bn):
     assert rel_l2(C.cpu().numpy(), exact) <= 1e-5
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (2, 640, 1024), (7, 384, 4096), (15, 256, 512), (16, 256, 2816), (17, 1280, 768),
+                                   (31, 256, 2048), (46, 256, 512), (77, 128, 768), (101, 19072, 256), (333, 640, 512)])
+def test_gemm_few_tokens_and_ragged_rows(capi, M, N, K, dtype):
+    """Up to 32 tokens, and N-major rows of every alignment (M odd, M % 8 in 2 .. 6): nothing outside the output is
+    written, 16-bit results are within half a unit of the exact sum."""
+    w, ws, xb, gs, exact = _case(M, N, K, seed=M + N)
+    xc, xsf = capi.quant(xb.cuda(), gs, swizzled=True)
+    buf = torch.full((M * N + 64,), 7.0, dtype=dtype, device="cuda")
+    C, wksp = buf[32:32 + M * N].view(M, N), torch.zeros(16 << 20, dtype=torch.int64, device="cuda")
+    for n_major in (True, False):
+        capi.gemm(xc, cuda(w), xsf, cuda(onv.swizzle_blockscale(ws)), C, 0.5, wksp, n_major=n_major)
+        got = C.double().cpu().numpy()
+        got = got.reshape(N, M).T if n_major else got
+        scale = np.abs(exact) + np.sqrt(np.mean(exact ** 2)) * 1e-3
+        assert np.max(np.abs(got - exact) / scale) <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.01
+        assert (buf[:32] == 7.0).all() and (buf[32 + M * N:] == 7.0).all()
+
+
 def test_gemm_output_of_any_alignment(capi):
     """A 2-byte aligned output takes the narrow stores."""
     M, N, K = 48, 256, 512
