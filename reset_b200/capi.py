@@ -4,6 +4,7 @@ raise on any non-zero status. PyTorch is used for memory and streams only."""
 
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 
 import torch
@@ -13,8 +14,17 @@ from . import _lib as L
 _DTYPE_CODE = {torch.bfloat16: L.BF16, torch.float16: L.F16, torch.float32: L.F32}
 
 
+_HERE = contextlib.nullcontext()
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream (torch.cuda.current_stream() builds an object around it: 3 us)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def _on(device: torch.device):
+    """Context with ``device`` current; where it already is, nothing is switched and switched back."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _need_cuda(*tensors):
@@ -41,7 +51,7 @@ def quant(x: torch.Tensor, global_scale_inv: torch.Tensor, *, swizzled: bool = F
     else:
         shape = (M, K // 16)
     scales = torch.empty(shape, dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         st = L.lib().nvfp4r_quant(x.data_ptr(), x.stride(0), M, K, global_scale_inv.data_ptr(),
                                   codes.data_ptr(), scales.data_ptr(),
                                   L.SF_SWIZZLED if swizzled else L.SF_FLAT, rcp_mode, _stream())
@@ -69,7 +79,7 @@ def gemv_out(weight, weight_scale, x, x_scale, out, alpha: float = 1.0) -> None:
         raise ValueError("out must be a contiguous [L, N] float16/bfloat16/float32 tensor")
     if w.stride(2) != 1 or ws.stride(2) != 1:
         raise ValueError("gemv: weight / weight_scale must have unit inner stride")
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         st = L.lib().nvfp4r_gemv(w.data_ptr(), ws.data_ptr(), a.data_ptr(), a_s.data_ptr(),
                                  out.data_ptr(), Lb, N, K, w.stride(0), w.stride(1),
                                  ws.stride(0), ws.stride(1), a.stride(0), a_s.stride(0),
@@ -94,7 +104,7 @@ def linear(x: torch.Tensor, global_scale_inv: torch.Tensor, weight: torch.Tensor
         out = torch.empty((M, N), dtype=out_dtype or x.dtype, device=x.device)
     elif tuple(out.shape) != (M, N) or not out.is_contiguous():
         raise ValueError("linear: out must be contiguous [M,N]")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         st = L.lib().nvfp4r_linear(x.data_ptr(), x.stride(0), M, K, global_scale_inv.data_ptr(),
                                    w.data_ptr(), ws.data_ptr(), N, float(alpha), out.data_ptr(),
                                    _DTYPE_CODE[out.dtype], rcp_mode, _stream())
@@ -119,7 +129,7 @@ def linear_tc(x: torch.Tensor, global_scale_inv: torch.Tensor, weight: torch.Ten
     w, ws = _u8(weight), _u8(weight_scale_swizzled)
     N = w.shape[0]
     out = torch.empty((M, N), dtype=out_dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         st = L.lib().nvfp4r_linear_tc(x.data_ptr(), x.stride(0), M, K, global_scale_inv.data_ptr(),
                                       w.data_ptr(), ws.data_ptr(), N, float(alpha), out.data_ptr(),
                                       _DTYPE_CODE[out_dtype], rcp_mode, workspace.data_ptr(),
@@ -136,7 +146,7 @@ def gemm(A, B, SFA, SFB, C: torch.Tensor, alpha: float, workspace: torch.Tensor,
     a, b, sa, sb = _u8(A), _u8(B), _u8(SFA), _u8(SFB)
     M, K2 = a.shape
     N = b.shape[0]
-    with torch.cuda.device(a.device):
+    with _on(a.device):
         st = L.lib().nvfp4r_gemm(a.data_ptr(), b.data_ptr(), sa.data_ptr(), sb.data_ptr(), C.data_ptr(),
                                  M, N, 2 * K2, float(alpha), _DTYPE_CODE[C.dtype],
                                  L.C_N_MAJOR if n_major else L.C_M_MAJOR, workspace.data_ptr(),
@@ -154,7 +164,7 @@ def pack_weight(weight: torch.Tensor, weight_scale_flat: torch.Tensor) -> torch.
     if n == 0:
         raise ValueError("pack_weight: needs N % 128 == 0 and K % 128 == 0")
     packed = torch.empty(n, dtype=torch.uint8, device=w.device)
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         st = L.lib().nvfp4r_pack_weight(w.data_ptr(), ws.data_ptr(), packed.data_ptr(), N, K, _stream())
     L.check(st, "nvfp4r_pack_weight")
     return packed
@@ -175,7 +185,7 @@ def linear_packed(x: torch.Tensor, global_scale_inv: torch.Tensor, packed: torch
     M, K = x.shape
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         st = L.lib().nvfp4r_linear_packed(x.data_ptr(), x.stride(0), M, K, global_scale_inv.data_ptr(),
                                           packed.data_ptr(), N, float(alpha), out.data_ptr(),
                                           _DTYPE_CODE[out.dtype], rcp_mode, workspace.data_ptr(),
@@ -197,7 +207,7 @@ def linear_packed_rmsnorm(delta, residual_in: torch.Tensor, residual_out: torch.
         out = torch.empty((M, N), dtype=out_dtype, device=residual_in.device)
     pro = L.Prologue(L.PROLOGUE_ADD_RMSNORM, float(eps), None if delta is None else delta.data_ptr(),
                      residual_in.data_ptr(), residual_out.data_ptr(), norm_weight.data_ptr())
-    with torch.cuda.device(residual_in.device):
+    with _on(residual_in.device):
         st = L.lib().nvfp4r_linear_packed_ex(C.byref(pro), None, 0, M, K, global_scale_inv.data_ptr(),
                                              packed.data_ptr(), N, float(alpha), out.data_ptr(),
                                              _DTYPE_CODE[out.dtype], rcp_mode, workspace.data_ptr(),
@@ -217,7 +227,7 @@ def linear_rmsnorm(delta, residual_in: torch.Tensor, residual_out: torch.Tensor,
     N = weight.shape[0]
     pro = L.Prologue(L.PROLOGUE_ADD_RMSNORM, float(eps), None if delta is None else delta.data_ptr(),
                      residual_in.data_ptr(), residual_out.data_ptr(), norm_weight.data_ptr())
-    with torch.cuda.device(residual_in.device):
+    with _on(residual_in.device):
         st = L.lib().nvfp4r_linear_ex(C.byref(pro), None, 0, M, K, global_scale_inv.data_ptr(), weight.data_ptr(),
                                       weight_scale_flat.data_ptr(), N, float(alpha), out.data_ptr(),
                                       _DTYPE_CODE[out.dtype], rcp_mode, _stream())
@@ -234,7 +244,7 @@ def linear_silu(gate_up: torch.Tensor, global_scale_inv: torch.Tensor, weight: t
     M, K2 = gate_up.shape
     N = weight.shape[0]
     pro = L.Prologue(L.PROLOGUE_SILU_MUL, 0.0, None, None, None, None)
-    with torch.cuda.device(gate_up.device):
+    with _on(gate_up.device):
         st = L.lib().nvfp4r_linear_ex(C.byref(pro), gate_up.data_ptr(), gate_up.stride(0), M, K2 // 2,
                                       global_scale_inv.data_ptr(), weight.data_ptr(), weight_scale_flat.data_ptr(),
                                       N, float(alpha), out.data_ptr(), _DTYPE_CODE[out.dtype], rcp_mode, _stream())
@@ -256,7 +266,7 @@ def linear_packed_silu(gate_up: torch.Tensor, global_scale_inv: torch.Tensor, pa
         out = torch.empty((M, N), dtype=out_dtype, device=gate_up.device)
     pro = L.Prologue(L.PROLOGUE_SILU_MUL, 0.0, None, None, None, None,
                      None if push is None else C.addressof(push), 1 if (gather and push is not None) else 0)
-    with torch.cuda.device(gate_up.device):
+    with _on(gate_up.device):
         st = L.lib().nvfp4r_linear_packed_ex(C.byref(pro), gate_up.data_ptr(), gate_up.stride(0), M, K,
                                              global_scale_inv.data_ptr(), packed.data_ptr(), N, float(alpha),
                                              out.data_ptr(), _DTYPE_CODE[out.dtype], rcp_mode,
@@ -270,7 +280,7 @@ def unswizzle_blockscale(swizzled: torch.Tensor, rows: int, K: int) -> torch.Ten
     _need_cuda(swizzled)
     sw = _u8(swizzled).contiguous()
     flat = torch.empty((rows, K // 16), dtype=torch.uint8, device=sw.device)
-    with torch.cuda.device(sw.device):
+    with _on(sw.device):
         st = L.lib().nvfp4r_unswizzle_blockscale(sw.data_ptr(), flat.data_ptr(), rows, K, _stream())
     L.check(st, "nvfp4r_unswizzle_blockscale")
     return flat
@@ -282,7 +292,7 @@ def swizzle_blockscale(flat: torch.Tensor) -> torch.Tensor:
     rows, cols = f.shape
     out = torch.empty(((rows + 127) // 128 * 128, (cols + 3) // 4 * 4), dtype=torch.uint8,
                       device=f.device)
-    with torch.cuda.device(f.device):
+    with _on(f.device):
         st = L.lib().nvfp4r_swizzle_blockscale(f.data_ptr(), out.data_ptr(), rows, cols * 16, _stream())
     L.check(st, "nvfp4r_swizzle_blockscale")
     return out
@@ -301,7 +311,7 @@ def entropy(logits: torch.Tensor, workspace: torch.Tensor | None = None) -> torc
     B, V = logits.shape
     ws = workspace if workspace is not None else reset_workspace(B, logits.device)
     out = torch.empty(B, dtype=torch.float32, device=logits.device)
-    with torch.cuda.device(logits.device):
+    with _on(logits.device):
         st = L.lib().nvfp4r_entropy(logits.data_ptr(), logits.stride(0), B, V, out.data_ptr(),
                                     ws.data_ptr(), ws.numel() * 8, _stream())
     L.check(st, "nvfp4r_entropy")
@@ -320,7 +330,7 @@ def reset_step(logits: torch.Tensor, states: torch.Tensor, params: L.ResetParams
         raise ValueError("reset_step: logits must be fp32 [B,V] with unit inner stride")
     B, V = logits.shape
     ptr = lambda t: t.data_ptr() if t is not None else None
-    with torch.cuda.device(logits.device):
+    with _on(logits.device):
         st = L.lib().nvfp4r_reset_step(logits.data_ptr(), logits.stride(0), B, V, states.data_ptr(),
                                        ptr(state_slots), ptr(last_ids), ptr(nl_bitmap),
                                        ptr(dnl_bitmap), C.byref(params), ptr(decisions),
@@ -348,7 +358,7 @@ def reset_step_per_request(logits: torch.Tensor, states: torch.Tensor, slot_para
             if bm is None or bm.numel() * bm.element_size() < n_id_sets * words * 4:
                 raise ValueError("reset_step_per_request: bitmaps must hold n_id_sets * ceil(V/32) words")
     ptr = lambda t: t.data_ptr() if t is not None else None
-    with torch.cuda.device(logits.device):
+    with _on(logits.device):
         st = L.lib().nvfp4r_reset_step_per_request(
             logits.data_ptr(), logits.stride(0), B, V, states.data_ptr(), ptr(state_slots), ptr(last_ids),
             ptr(nl_bitmaps), ptr(dnl_bitmaps), int(n_id_sets), slot_params.data_ptr(), ptr(decisions),
@@ -384,7 +394,7 @@ def lm_head_reset_step(x: torch.Tensor, weight: torch.Tensor, logits: torch.Tens
             if bm is None or bm.numel() * bm.element_size() < n_id_sets * words * 4:
                 raise ValueError("lm_head_reset_step: bitmaps must hold n_id_sets * ceil(V/32) words")
     ptr = lambda t: t.data_ptr() if t is not None else None
-    with torch.cuda.device(logits.device):
+    with _on(logits.device):
         st = L.lib().nvfp4r_lm_head_reset_step(
             x.data_ptr(), weight.data_ptr(), logits.data_ptr(), V, H, states.data_ptr(), ptr(state_slots),
             ptr(last_ids), ptr(nl_bitmaps), ptr(dnl_bitmaps), int(n_id_sets), slot_params.data_ptr(),
@@ -414,7 +424,7 @@ def sample(logits: torch.Tensor, draws: torch.Tensor, *, seed: int = 0,
     truncated = (0 < int(top_k) < V) or float(top_p) < 1.0
     if truncated and workspace is None:
         raise ValueError("sample: top_k / top_p need a workspace (capi.sample_workspace)")
-    with torch.cuda.device(logits.device):
+    with _on(logits.device):
         if truncated:
             st = L.lib().nvfp4r_sample_top_k_top_p(
                 logits.data_ptr(), logits.stride(0), B, V, int(top_k), float(top_p), int(seed) & (2 ** 64 - 1),
@@ -447,7 +457,7 @@ def linear_push(x: torch.Tensor, global_scale_inv: torch.Tensor, weight: torch.T
     if M != 1 or out.dtype != torch.bfloat16 or tuple(out.shape) != (1, N) or not out.is_contiguous():
         raise ValueError("linear_push: one token, out bf16 [1,N] contiguous")
     pro = L.Prologue(L.PROLOGUE_NONE, 0.0, None, None, None, None, C.addressof(push), 1)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         st = L.lib().nvfp4r_linear_ex(C.byref(pro), x.data_ptr(), x.stride(0), M, K, global_scale_inv.data_ptr(),
                                       w.data_ptr(), ws.data_ptr(), N, float(alpha), out.data_ptr(),
                                       _DTYPE_CODE[out.dtype], rcp_mode, _stream())
@@ -465,7 +475,7 @@ def linear_packed_push(x: torch.Tensor, global_scale_inv: torch.Tensor, packed: 
     _need_cuda(x, global_scale_inv, packed, workspace, out)
     M, K = x.shape
     pro = L.Prologue(L.PROLOGUE_NONE, 0.0, None, None, None, None, C.addressof(push), 1 if gather else 0)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         st = L.lib().nvfp4r_linear_packed_ex(C.byref(pro), x.data_ptr(), x.stride(0), M, K,
                                              global_scale_inv.data_ptr(), packed.data_ptr(), N, float(alpha),
                                              out.data_ptr(), _DTYPE_CODE[out.dtype], rcp_mode,

@@ -8,6 +8,7 @@
 // that replace multi-op sequences of the reference with one dispatch each.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 #include <torch/library.h>
@@ -37,6 +38,11 @@ inline int dtype_code(at::ScalarType t, const char* who) {
 
 inline void check_status(int st, const char* who) {
     TORCH_CHECK(st == NVFP4R_OK, who, ": ", nvfp4r_status_string(st), " (", st, "): ", nvfp4r_last_error());
+}
+
+// Uninitialised contiguous memory on `like`'s device, from the caching allocator without another trip through the dispatcher.
+inline at::Tensor new_tensor(at::IntArrayRef size, at::ScalarType dtype, const at::Tensor& like) {
+    return at::detail::empty_cuda(size, dtype, like.device(), c10::nullopt);
 }
 
 inline void* current_stream() { return static_cast<void*>(at::cuda::getCurrentCUDAStream().stream()); }
@@ -159,10 +165,10 @@ std::tuple<at::Tensor, at::Tensor> quant_op(const at::Tensor& x, const at::Tenso
                 "quant: global_scale_inv must be a float32 tensor");
     const int64_t M = x.size(0), K = x.size(1);
     const c10::cuda::OptionalCUDAGuard guard(x.device());
-    auto codes = at::empty({M, K / 2}, x.options().dtype(at::kByte));
+    auto codes = new_tensor({M, K / 2}, at::kByte, x);
     const int64_t rows = swizzled ? (M + 127) / 128 * 128 : M;
     const int64_t cols = swizzled ? (K / 16 + 3) / 4 * 4 : K / 16;
-    auto scales = at::empty({rows, cols}, x.options().dtype(at::kByte));
+    auto scales = new_tensor({rows, cols}, at::kByte, x);
     const int st = nvfp4r_quant(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),
                                 global_scale_inv.data_ptr<float>(), codes.data_ptr(), scales.data_ptr(),
                                 swizzled ? NVFP4R_SF_SWIZZLED : NVFP4R_SF_FLAT,
@@ -187,7 +193,7 @@ at::Tensor linear_op(const at::Tensor& x, const at::Tensor& global_scale_inv, co
                 "linear: weight / weight_scale shape mismatch with x");
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     const auto dt = out_dtype_int == 0 ? at::kBFloat16 : out_dtype_int == 1 ? at::kHalf : at::kFloat;
-    auto out = at::empty({M, N}, x.options().dtype(dt));
+    auto out = new_tensor({M, N}, dt, x);
     const int st = nvfp4r_linear(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),
                                  global_scale_inv.data_ptr<float>(), weight.data_ptr(),
                                  weight_scale_flat.data_ptr(), static_cast<int>(N),
@@ -215,7 +221,7 @@ at::Tensor linear_tc_op(const at::Tensor& x, const at::Tensor& global_scale_inv,
                 "linear_tc: swizzled weight_scale too small");
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     const auto dt = out_dtype_int == 0 ? at::kBFloat16 : out_dtype_int == 1 ? at::kHalf : at::kFloat;
-    auto out = at::empty({M, N}, x.options().dtype(dt));
+    auto out = new_tensor({M, N}, dt, x);
     at::Tensor& ws = fixed_workspace(0, x.device(),
                                      nvfp4r_gemm_workspace_bytes(static_cast<int>(M), static_cast<int>(N),
                                                                  static_cast<int>(K)), "linear_tc");
@@ -261,7 +267,7 @@ at::Tensor linear_packed_op(const at::Tensor& x, const at::Tensor& global_scale_
                 "linear_packed: packed weight does not match N and K");
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     const auto dt = out_dtype_int == 0 ? at::kBFloat16 : out_dtype_int == 1 ? at::kHalf : at::kFloat;
-    auto out = at::empty({M, N}, x.options().dtype(dt));
+    auto out = new_tensor({M, N}, dt, x);
     // Many tokens: quantized once into scratch of this call (the caching allocator's, so capture and streams are its
     // business), one launch for all of them. Also where the other kernel is the faster one but its workspace is not
     // to be had: larger than the fixed buffer, or under a capture that no call came before.
@@ -276,7 +282,7 @@ at::Tensor linear_packed_op(const at::Tensor& x, const at::Tensor& global_scale_
     const size_t scratch_bytes =
         many ? nvfp4r_linear_packed_scratch_bytes(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)) : 0;
     if (scratch_bytes > 0) {
-        auto scratch = at::empty({static_cast<int64_t>(scratch_bytes)}, x.options().dtype(at::kByte));
+        auto scratch = new_tensor({static_cast<int64_t>(scratch_bytes)}, at::kByte, x);
         check_status(nvfp4r_linear_packed_scratch(x.data_ptr(), x.stride(0), static_cast<int>(M), static_cast<int>(K),
                                                   global_scale_inv.data_ptr<float>(), packed.data_ptr(),
                                                   static_cast<int>(N), static_cast<float>(alpha), out.data_ptr(),

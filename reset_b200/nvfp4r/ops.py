@@ -30,7 +30,7 @@ def gemv(weight, weight_scale, x, x_scale, out: Optional[torch.Tensor] = None,
     a, a_s = _ensure_3d(x, "x"), _ensure_3d(x_scale, "x_scale")
     if out is None:
         out = torch.empty((w.shape[0], w.shape[1]), dtype=torch.float16, device=w.device)
-    torch.ops.nvfp4r.gemv(w, ws, a, a_s, out, alpha)
+    torch.ops.nvfp4r.gemv.default(w, ws, a, a_s, out, alpha)
     return out
 
 
@@ -38,7 +38,7 @@ def gemm(A, B, SFA, SFB, C, alpha: float = 1.0) -> torch.Tensor:
     """``C = alpha * A @ B^T`` on the tensor cores (ops.py:62-88). The kernel writes
     ``C``'s buffer N-major; the returned view is the [M,N] result."""
     M, N = C.shape
-    torch.ops.nvfp4r.gemm(A, B, SFA, SFB, C, alpha)
+    torch.ops.nvfp4r.gemm.default(A, B, SFA, SFB, C, alpha)
     return C.view(N, M).transpose(0, 1)
 
 
@@ -47,7 +47,7 @@ def quant(x: torch.Tensor, global_scale_inv: torch.Tensor, swizzled: bool = Fals
     """bf16 [M,K] -> (codes [M,K/2] u8, e4m3 scales u8), the op the reference borrows
     from vLLM (vllm_integration.py:213). ``rcp_mode`` 1 matches that op bit for bit,
     0 uses IEEE division."""
-    return torch.ops.nvfp4r.quant(x, global_scale_inv, swizzled, rcp_mode)
+    return torch.ops.nvfp4r.quant.default(x, global_scale_inv, swizzled, rcp_mode)
 
 
 def linear(x: torch.Tensor, global_scale_inv: torch.Tensor, weight: torch.Tensor,
@@ -55,19 +55,19 @@ def linear(x: torch.Tensor, global_scale_inv: torch.Tensor, weight: torch.Tensor
            rcp_mode: int = 1) -> torch.Tensor:
     """Quantize up to 16 bf16 tokens and multiply by one NVFP4 weight in one launch."""
     code = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[out_dtype]
-    return torch.ops.nvfp4r.linear(x, global_scale_inv, weight, weight_scale_flat, alpha, code, rcp_mode)
+    return torch.ops.nvfp4r.linear.default(x, global_scale_inv, weight, weight_scale_flat, alpha, code, rcp_mode)
 
 
 def pack_weight(weight: torch.Tensor, weight_scale_flat: torch.Tensor) -> torch.Tensor:
     """Re-lay a weight [N,K/2] + flat scales [N,K/16] out once for the tensor-core path."""
-    return torch.ops.nvfp4r.pack_weight(weight, weight_scale_flat)
+    return torch.ops.nvfp4r.pack_weight.default(weight, weight_scale_flat)
 
 
 def linear_packed(x: torch.Tensor, global_scale_inv: torch.Tensor, packed: torch.Tensor, N: int,
                   alpha: float, out_dtype: torch.dtype = torch.bfloat16, rcp_mode: int = 1) -> torch.Tensor:
     """Quantize M bf16 tokens and multiply by a packed NVFP4 weight on the tensor cores."""
     code = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[out_dtype]
-    return torch.ops.nvfp4r.linear_packed(x, global_scale_inv, packed, N, alpha, code, rcp_mode)
+    return torch.ops.nvfp4r.linear_packed.default(x, global_scale_inv, packed, N, alpha, code, rcp_mode)
 
 
 def use_gemv(M: int, N: int, K: int, gemv_max_m: int) -> bool:
