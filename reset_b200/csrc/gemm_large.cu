@@ -965,15 +965,16 @@ bool large_pays(int M, int N, int K) {
     if (!large_accepts(M, N, K)) return false;
     if (g_large_min_m) return true;
     const int G = device_sm_count(), tiles = N / kRows, kblocks = (K + kBK - 1) / kBK;
-    // A narrow weight with rows of 31 or 32 K blocks: the longest that still run as whole tiles here (0.48 us a
-    // block), while two launches of the decode kernel give each CTA one block and one token to add up. 33 / 48 / 64
+    // A narrow weight with rows of 31 or 32 K blocks: the longest that ran as whole tiles here before clusters shared
+    // them (0.48 us a block), while two launches of the decode kernel give each CTA one block and one token to add up. 33 / 48 / 64
     // tokens: 640x8192 13.0 / 14.0 / 14.3, here 15.5 / 15.7 / 15.9; 1280x8192 14.3 / 15.5 / 18.6, here 16.0 / 15.9 / 16.2;
     // 30 blocks, 1024x7680: 14.9 / 16.0 / 17.4, here 14.8 / 14.8 / 15.0; 33, 1792x8320: 17.2 / 18.4 / 22.4, here 16.8.
+    // (With clusters 640x8192 takes 7.7 / 7.8 / 8.2 here. The line stays where callers of the query found it.)
     if (M <= 64 && kblocks > 30 && kblocks <= 32 && tiles <= (M <= 48 ? 16 : 8)) return false;
-    // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two full rounds of
-    // 0.48 us a K block. 20480x2048: 13 tokens 8.9 / 10.7, 16 tokens 9.8 / 10.8; 24576x4096: 16 tokens 17.4 / 18.5;
-    // but 24064x2304, where the decode kernel splits K: 16 tokens 15.3 / 11.5; 22528x3072: 16 tokens 16.4 / 15.1.
-    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 3.9 + 0.96 * kblocks;
+    // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two rounds, 4.2 us and
+    // 0.66 a K block (the estimate of the other kernel is good to 4 %: 4.6 and 0.68). 24576x4096: 13 tokens 16.8 / 14.7, 16 tokens 18.7 / 14.6; 24576x2048: 13 tokens 9.6 / 9.9, 16 tokens
+    // 10.6 / 9.9; 19456x2048: 13 tokens 9.3 / 9.5.
+    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 4.6 + 0.68 * kblocks;
     return true;
 }
 
@@ -983,15 +984,16 @@ size_t large_scratch_bytes(int M, int N, int K) {
     return plan.token_bytes + plan.ticket_bytes + plan.partial_bytes;
 }
 
-// The host's side: a second launch and the scratch bring a call to 12 us or more even where the device needs 5, while
-// a call of the decode kernel ends at 8.5. So up to 32 tokens (one launch of it) that kernel keeps what it does in
-// less. Measured, us a call: 6144x1024, 16 tokens 8.5 / 12.0; 12288x2048, 16 tokens 8.9 / 12.0; 4096x4096, 32 tokens
-// 11.4 / 12.2; 6144x2048, 32 tokens 13.1 / 12.2; 8192x3072, 20 tokens 13.0 / 12.1.
-constexpr double kLargeCallUs = 12.0;
+// The host's side: a second launch and the scratch bring a call to 9.4 us or more even where the device needs 5, while
+// a call of the decode kernel ends at 6.5. So up to 32 tokens (one launch of it) that kernel keeps what it does in
+// less than 10 us; up to 16 tokens, where the device times lie close together, in less than 12. Measured, us a call:
+// 12288x2048 24 tokens 10.4 / 9.5; 8192x2048 20 tokens 11.3 / 9.6, 6144x4096 11.1 / 9.6; 12288x2048 20 tokens 9.5 / 10.1;
+// 24576x2048 16 tokens 9.9 / 10.6.
+constexpr double kLargeCallUs = 10.0, kLargeCallUsFew = 12.0;
 
 int large_route(int M, int N, int K) {
     if (!large_pays(M, N, K)) return NVFP4R_ROUTE_PACKED;
-    return g_large_min_m || M > 32 || packed_time_us(M, N, K) >= kLargeCallUs ? NVFP4R_ROUTE_SCRATCH : NVFP4R_ROUTE_SCRATCH_CAPTURED;
+    return g_large_min_m || M > 32 || packed_time_us(M, N, K) >= (M <= 16 ? kLargeCallUsFew : kLargeCallUs) ? NVFP4R_ROUTE_SCRATCH : NVFP4R_ROUTE_SCRATCH_CAPTURED;
 }
 
 cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaStream_t stream) {
