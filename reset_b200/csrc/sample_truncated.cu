@@ -7,11 +7,15 @@
 //      groups have an element at or above it). What reaches the bound goes to one CTA's list, a few more than k
 //      on unordered logits; with at most 512 entries that CTA settles the row by comparing all pairs, one
 //      entry per thread, and the launch ends;
-//   3. otherwise, per truncation (top-k by count, then top-p by mass) a radix descent over the order-preserving keys,
+//   3. otherwise, per truncation (top-k by count, then top-p by mass) one histogram of 2048 equal steps of the distance to
+//      the row maximum, 22.2 in all by mass (what lies further has none), 89 by count: the CTA whose bins cross the goal announces the
+//      bin, its entries go to one CTA's list, and with at most 512 of them that CTA finds the threshold by comparing all
+//      pairs. The distance rounds monotonically, so bins are in the order of the values;
+//   4. where more entries share the bin, or the goal lies beyond the steps, a radix descent over the order-preserving keys,
 //      11 + 11 + 10 bits: histogram of the keys that share the prefix found so far, each CTA sums 256 of the
 //      2048 bins over the eight histograms, and the CTA whose bins cross the goal announces the bin. After
 //      the last level the prefix is the key of the last token kept; equal keys are all kept;
-//   4. arg-max of logit + Gumbel noise among the keys at or above the threshold.
+//   5. arg-max of logit + Gumbel noise among the keys at or above the threshold.
 // Mass is exp(x - row max) scaled by 2^32 and truncated to an integer, so no result depends on the order of
 // the additions. Elements of mass 0 are left out of the top-p histograms: a bin of mass 0 is never the first
 // to reach the goal.
@@ -21,6 +25,11 @@
 //   top-k 20 top-p 0.95   1 row 57.7 -> 7.4    8 rows 70.9 -> 8.4    32 rows 133 -> 10.1   256 rows 956 -> 90
 //   top-p 0.9             1 row 38.3 -> 35.3   8 rows 49.5 -> 41.4   32 rows 105 -> 55.4   256 rows 700 -> 410
 //   top-k 1000            1 row 37.1 -> 24.1   8 rows 45.1 -> 26.1   32 rows 96 -> 34.8    256 rows 657 -> 268
+// and with phase 3, the masses in 32-bit halves and the draw's logarithms only where they can matter, device us in a CUDA
+// graph with the counters' reset, radix descent -> steps:
+//   top-p 0.9   1 row 31.6 -> 23.0   8 rows 39.4 -> 30.0   32 rows 53.8 -> 38.8     top-k 1000, 8 rows 27.9 -> 22.4
+//   top-k 150 top-p 0.8, 8 rows 40.2 -> 28.6
+// of which, 8 rows, thousand clocks: load 5, histogram 11, its bin 6, list 5, pairs 3, draw 13.
 // (the first line without phase 2: 35.1, 37.6, 47.2, 373)
 //
 //   * 8 CTAs of 512 threads: the largest cluster every device can place, and at 151936 entries two CTAs
@@ -56,6 +65,13 @@ constexpr int kListMax = kThreads;                // candidates that one CTA set
 __device__ __forceinline__ unsigned long long mass_of(float x, float m) {
     // the maximum itself weighs exactly 2^32, also when it is +inf
     return x == m ? (1ull << 32) : __float2ull_rd(__expf(x - m) * 4294967296.0f);
+}
+
+// The same number in two halves of 16 and 17 bits: powers of two and differences are exact, so no 64-bit conversion.
+__device__ __forceinline__ void mass_halves(float x, float m, uint32_t& w_lo, uint32_t& w_hi) {
+    const float t = x == m ? 65536.0f : __expf(x - m) * 65536.0f;
+    w_hi = static_cast<uint32_t>(t);
+    w_lo = static_cast<uint32_t>((t - static_cast<float>(w_hi)) * 65536.0f);
 }
 
 // kFew: 0 < top_k <= kGroups (its own instance: the list's code costs the descent registers)
@@ -253,6 +269,81 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
     }
 
     // ---- truncation --------------------------------------------------------------------------------
+    // Sum of the bins, in descending order of the values, up to the one that crosses the goal; called by all threads
+    // of the cluster behind a histogram. False: the bins do not reach the goal. The histogram is cleared.
+    auto find_bin = [&](int mode, unsigned long long above, unsigned long long& goal, bool first) {
+        cluster.sync();
+        // this CTA's bins in descending order: thread t has bin kBins - 1 - (rank * kSeg + t)
+        unsigned long long v = 0ull, incl = 0ull;
+        const int bin = kBins - 1 - (rank * kSeg + tid);
+        if (tid < kSeg) {
+#pragma unroll
+            for (int q = 0; q < kCtas; ++q) {
+                const uint32_t* h = cluster.map_shared_rank(s_hist, q);
+                if (mode == 0) v += h[bin];
+                else if (kCached) v += h[bin] + (static_cast<unsigned long long>(h[kBins + bin]) << 16);
+                else v += reinterpret_cast<const unsigned long long*>(h)[bin];
+            }
+            incl = v;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned long long o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += o;
+            }
+            if (lane == 31) s_scan[warp] = incl;
+        }
+        __syncthreads();
+        unsigned long long seg = 0ull;
+#pragma unroll
+        for (int w = 0; w < kSeg / 32; ++w) {
+            if (w < warp) incl += s_scan[w];
+            seg += s_scan[w];
+        }
+        if (tid < kCtas) *cluster.map_shared_rank(&s_peer_total[rank], tid) = seg;
+        cluster.sync();
+
+        unsigned long long total = 0ull, base = 0ull;
+#pragma unroll
+        for (int q = 0; q < kCtas; ++q) {
+            if (q < rank) base += s_peer_total[q];
+            total += s_peer_total[q];
+        }
+        if (mode == 1 && first) {
+            // candidate set = everything counted here (the top-k set when top-k ran before)
+            goal = static_cast<unsigned long long>(ceil(static_cast<double>(top_p) * static_cast<double>(total)));
+            if (goal < 1ull) goal = 1ull;
+        }
+        for (int i = tid; i < 2 * kBins / 4; i += kThreads)
+            reinterpret_cast<uint4*>(s_hist)[i] = make_uint4(0, 0, 0, 0);
+        if (tid == 0) s_count = 0;                            // (rank 0's is the one in use)
+        if (above + total < goal) return false;               // same decision in every thread of the cluster
+        const unsigned long long through = above + base + incl;
+        if (tid < kSeg && through >= goal && through - v < goal) {
+#pragma unroll
+            for (int q = 0; q < kCtas; ++q) {
+                *cluster.map_shared_rank(&s_pick_bin, q) = static_cast<uint32_t>(bin);
+                *cluster.map_shared_rank(&s_pick_above, q) = through - v;
+            }
+        }
+        cluster.sync();
+        return true;
+    };
+    auto add_mass = [&](uint32_t bin, float x) {
+        if (kCached) {
+            uint32_t w_lo, w_hi;
+            mass_halves(x, m, w_lo, w_hi);
+            if (w_lo != 0u) atomicAdd(&s_hist[bin], w_lo);
+            if (w_hi != 0u) atomicAdd(&s_hist[kBins + bin], w_hi);
+        } else {
+            const unsigned long long w = mass_of(x, m);
+            if (w != 0ull) atomicAdd(reinterpret_cast<unsigned long long*>(s_hist) + bin, w);
+        }
+    };
+    // bin 2047: the maximum; bin 0: everything beyond the steps, at a distance of 22.2 by mass, 89 by count
+    auto step_bin = [&](float x, int mode) {
+        return static_cast<uint32_t>(kBins - 1) -
+               (x == m ? 0u : static_cast<uint32_t>(fminf((m - x) * (mode == 0 ? 23.0f : 92.0f), static_cast<float>(kBins - 1))));
+    };
     uint32_t min_key = 0u, thr_key = 0u;                      // candidates / final set: key >= ...
 #pragma unroll 1
     for (int mode = 0; mode < 2; ++mode) {                    // 0: top-k by count, 1: top-p by mass
@@ -262,84 +353,70 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
         unsigned long long above = 0ull;                      // count / mass of the keys above the prefix
         unsigned long long goal = static_cast<unsigned long long>(top_k);
         bool all = false;
+
+        for_each([&](float x, int) {
+            if (!(x > -INFINITY) || sortable_key(x) < skip_below) return;      // -inf and NaN never enter the set
+            if (mode == 0) atomicAdd(&s_hist[step_bin(x, mode)], 1u);
+            else if (!(m - x > 22.25f)) add_mass(step_bin(x, mode), x);       // beyond: less than 2^-32, no mass
+        });
+        if (!find_bin(mode, 0ull, goal, true)) {
+            all = true;
+        } else if (s_pick_bin != 0u) {
+            const uint32_t pick = s_pick_bin;
+            int* count = cluster.map_shared_rank(&s_count, 0);
+            float* list_x = cluster.map_shared_rank(s_list_x, 0);
+            const float step = mode == 0 ? 23.0f : 92.0f, first = static_cast<float>(kBins - 1 - static_cast<int>(pick));
+            for_each([&](float x, int) {
+                const float d = x == m ? 0.0f : (m - x) * step;      // step_bin(x, mode) == pick; false for NaN
+                if (!(d >= first && d < first + 1.0f) || sortable_key(x) < skip_below) return;
+                const int at = atomicAdd(count, 1);
+                if (at < kListMax) list_x[at] = x;
+            });
+            cluster.sync();
+            const int n = *count;
+            if (n <= kListMax) {                              // same answer in every thread of the cluster
+                if (rank == 0) {
+                    // an entry stays while what is larger is less than the goal; the smallest that stays is the threshold
+                    const bool have = tid < n;
+                    const float x = have ? s_list_x[tid] : 0.0f;
+                    const uint32_t mine = have ? sortable_key(x) : 0u;
+                    if (tid == 0) s_bound = 0xffffffffu;
+                    unsigned long long* weight = reinterpret_cast<unsigned long long*>(s_hist + kListMax);
+                    s_hist[tid] = mine;
+                    weight[tid] = have ? (mode == 0 ? 1ull : mass_of(x, m)) : 0ull;
+                    __syncthreads();
+                    if (have) {
+                        unsigned long long larger = s_pick_above;
+                        for (int j = 0; j < n; ++j)
+                            if (s_hist[j] > mine) larger += weight[j];
+                        if (larger < goal) atomicMin(&s_bound, mine);
+                    }
+                    __syncthreads();
+                    if (tid < kCtas) *cluster.map_shared_rank(&s_pick_bin, tid) = s_bound;
+                    for (int i = tid; i < 3 * kListMax; i += kThreads) s_hist[i] = 0u;
+                }
+                cluster.sync();
+                thr_key = min_key = s_pick_bin;
+                continue;
+            }
+        }
 #pragma unroll 1
-        for (int level = 0; level < 3; ++level) {
+        for (int level = 0; level < 3 && !all; ++level) {
             const int shift = level_shift(level), prev_shift = level == 0 ? 31 : level_shift(level - 1);
             const uint32_t mask = static_cast<uint32_t>(level_bins(level) - 1);
             for_each([&](float x, int) {
-                if (!(x > -INFINITY)) return;                 // -inf and NaN never enter the set
+                if (!(x > -INFINITY)) return;
                 const uint32_t key = sortable_key(x);
                 if (key < skip_below) return;
                 if (level > 0 && (key >> prev_shift) != prefix) return;
                 const uint32_t bin = (key >> shift) & mask;
-                if (mode == 0) {
-                    atomicAdd(&s_hist[bin], 1u);
-                    return;
-                }
-                const unsigned long long w = mass_of(x, m);
-                if (kCached) {
-                    const uint32_t w_lo = static_cast<uint32_t>(w) & 0xffffu, w_hi = static_cast<uint32_t>(w >> 16);
-                    if (w_lo != 0u) atomicAdd(&s_hist[bin], w_lo);
-                    if (w_hi != 0u) atomicAdd(&s_hist[kBins + bin], w_hi);
-                } else if (w != 0ull) {
-                    atomicAdd(reinterpret_cast<unsigned long long*>(s_hist) + bin, w);
-                }
+                if (mode == 0) atomicAdd(&s_hist[bin], 1u);
+                else add_mass(bin, x);
             });
-            cluster.sync();
-
-            // this CTA's bins in descending order: thread t has bin kBins - 1 - (rank * kSeg + t)
-            unsigned long long v = 0ull, incl = 0ull;
-            const int bin = kBins - 1 - (rank * kSeg + tid);
-            if (tid < kSeg) {
-#pragma unroll
-                for (int q = 0; q < kCtas; ++q) {
-                    const uint32_t* h = cluster.map_shared_rank(s_hist, q);
-                    if (mode == 0) v += h[bin];
-                    else if (kCached) v += h[bin] + (static_cast<unsigned long long>(h[kBins + bin]) << 16);
-                    else v += reinterpret_cast<const unsigned long long*>(h)[bin];
-                }
-                incl = v;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const unsigned long long o = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (lane >= d) incl += o;
-                }
-                if (lane == 31) s_scan[warp] = incl;
+            if (!find_bin(mode, above, goal, false)) {
+                all = true;
+                break;
             }
-            __syncthreads();
-            unsigned long long seg = 0ull;
-#pragma unroll
-            for (int w = 0; w < kSeg / 32; ++w) {
-                if (w < warp) incl += s_scan[w];
-                seg += s_scan[w];
-            }
-            if (tid < kCtas) *cluster.map_shared_rank(&s_peer_total[rank], tid) = seg;
-            cluster.sync();
-
-            unsigned long long total = 0ull, base = 0ull;
-#pragma unroll
-            for (int q = 0; q < kCtas; ++q) {
-                if (q < rank) base += s_peer_total[q];
-                total += s_peer_total[q];
-            }
-            if (mode == 1 && level == 0) {
-                // candidate set = everything counted here (the top-k set when top-k ran before)
-                goal = static_cast<unsigned long long>(ceil(static_cast<double>(top_p) * static_cast<double>(total)));
-                if (goal < 1ull) goal = 1ull;
-            }
-            for (int i = tid; i < 2 * kBins / 4; i += kThreads)
-                reinterpret_cast<uint4*>(s_hist)[i] = make_uint4(0, 0, 0, 0);
-            all = above + total < goal;                       // same decision in every thread of the cluster
-            if (all) break;
-            const unsigned long long through = above + base + incl;
-            if (tid < kSeg && through >= goal && through - v < goal) {
-#pragma unroll
-                for (int q = 0; q < kCtas; ++q) {
-                    *cluster.map_shared_rank(&s_pick_bin, q) = static_cast<uint32_t>(bin);
-                    *cluster.map_shared_rank(&s_pick_above, q) = through - v;
-                }
-            }
-            cluster.sync();
             prefix = (level == 0 ? 0u : prefix << (level == 2 ? 10 : 11)) | s_pick_bin;
             above = s_pick_above;
         }
@@ -350,11 +427,21 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
     }
 
     // ---- Gumbel-max draw within the set --------------------------------------------------------------
+    // The two logarithms are taken only where they can matter: -log(-log u) <= -log(1 - u), so an element stays below
+    // the best score of the CTA so far when 1 - u > exp(x - best); the 1 % covers the rounding of both sides.
     const unsigned long long key = gumbel_key(seed, b, draws[b]);
+    if (tid == 0) s_bound = 0u;
+    __syncthreads();
+    volatile uint32_t* bound = &s_bound;                      // the CTA's best score, as a key
     for_each([&](float x, int i) {
         if (!(x > -INFINITY) || sortable_key(x) < thr_key) return;
-        const float s = x + gumbel_noise(key, i);
+        const float u = gumbel_uniform(key, i);
+        const uint32_t so_far = *bound;
+        if (so_far != 0u && 1.0f - u > 1.01f * __expf(x - key_value(so_far))) return;
+        const float s = x + gumbel_of(u);
         if (s > best) { best = s; arg = i; }
+        const uint32_t mine = sortable_key(s);
+        if (mine > so_far) atomicMax(&s_bound, mine);
     });
     block_best();
     if (tid == 0) {

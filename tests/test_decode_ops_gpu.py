@@ -503,3 +503,59 @@ def test_decode_step_runs_with_every_tensor_parallel_shard_shape(world, monkeypa
     torch.cuda.synchronize()
     assert torch.equal(m.logits_local, eager)
     assert _lib.lib().nvfp4r_check_device_status() == 0
+
+
+@pytest.mark.parametrize("V", [5000, 151936, 400003])
+@pytest.mark.parametrize("gap,per,peak,top_k,top_p", [
+    (0.37, 3, 0.0, 0, 0.9),          # few entries share the crossing step: settled by comparing pairs
+    (0.37, 3, 0.0, 130, 1.0),        # the same by count
+    (0.37, 3, 0.0, 200, 0.6),        # by count, then by mass of what is left
+    (0.002, 90, 0.0, 0, 0.5),        # several levels inside one step of the distance
+    (0.37, 700, 0.0, 0, 0.9),        # more entries in the step than the list holds: radix descent
+    (0.002, 400, 0.0, 1000, 1.0),
+    (0.37, 3, 60.0, 140, 1.0),       # one peak far above: the k-th lies beyond the steps
+    (0.37, 3, 60.0, 0, 0.9),         # and the nucleus is the peak alone
+    (0.37, 3, float("inf"), 140, 0.999),
+])
+def test_sample_threshold_between_levels(V, gap, per, peak, top_k, top_p):
+    """Logits on a ladder of levels, ``per`` equal entries each: the set ends between two levels or takes a whole one, so
+    rounding cannot move it. Every id drawn is in the set, and the lowest level of a small set is drawn too."""
+    from reset_b200 import capi
+    g = torch.Generator().manual_seed(V + per)
+    level = torch.arange(V) // per
+    x = -gap * level.double()
+    if peak:
+        x[1:] -= 1.0
+        x[0] = peak
+    x = x.float()
+    # the set in float64: count first, then mass over what is left; ties stay
+    d = x.double()
+    keep = torch.ones(V, dtype=torch.bool)
+    if top_k:
+        keep = d >= torch.topk(d, top_k).values[-1]
+    if top_p < 1.0:
+        w = (d == d.max()).double() if peak == float("inf") else torch.exp(d - d.max())
+        w = torch.where(keep, w, torch.zeros_like(w))
+        levels = torch.unique(d[w > 0]).flip(0)
+        above, goal = 0.0, top_p * w.sum().item()
+        for v in levels.tolist():
+            if above >= goal:
+                keep &= d > v
+                break
+            assert abs(above - goal) > 1e-5 * goal                       # the case is decided by more than rounding
+            above += w[d == v].sum().item()
+    perm = torch.randperm(V, generator=g)
+    rows = 64
+    logits = x[perm].repeat(rows, 1).contiguous().cuda()
+    allowed = keep[perm]
+    ids = []
+    draws = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    ws = capi.sample_workspace(rows, "cuda")
+    for _ in range(24):
+        ids.append(capi.sample(logits, draws, seed=11, top_k=top_k, top_p=top_p, workspace=ws).cpu().long())
+    ids = torch.cat(ids)
+    assert allowed[ids].all()
+    p = torch.softmax(torch.where(keep, d, torch.full_like(d, float("-inf"))), 0) if peak != float("inf") else keep.double() * 0
+    low = d[keep].min()
+    if p[d == low].sum() > 0.01:                                         # 1536 draws: missed with probability below 2e-7
+        assert (x[perm].double()[ids] == low).any()
