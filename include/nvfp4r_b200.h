@@ -139,9 +139,10 @@ NVFP4R_API int nvfp4r_linear(const void* x, int64_t x_row_stride, int M, int K,
  *             reference kernel writes (gemm_nvfp4.cu:581, ops.py:86-88);
  *             NVFP4R_C_M_MAJOR: element (m,n) at C[m*N + n].
  * Any M >= 1 (the reference needs M % 64 == 0), N % 128 == 0, K % 256 == 0, any
- * such K (the reference has a fixed table, gemm_nvfp4.cu:633-650). Up to 32 rows one
- * launch streams the weight once. More rows take one launch of the many-token kernel
- * (gemm_large.cu) where the workspace holds its partial sums, else 32 rows per launch.
+ * such K (the reference has a fixed table, gemm_nvfp4.cu:633-650). One launch of the
+ * many-token kernel (gemm_large.cu) where the workspace holds the partial sums that its
+ * schedule may need, else 32 rows per launch. Up to 32 rows with fp32 output one launch of
+ * the 32-row path: the same bits as nvfp4r_linear_tc.
  * `workspace` (>= nvfp4r_gemm_workspace_bytes(M, N, K) bytes, 16-byte aligned) holds
  * tile tickets and split-K partial sums. Its first NVFP4R_GEMM_TICKET_BYTES bytes (all
  * of it, if it is smaller) must be zero before the first use, and every call leaves
