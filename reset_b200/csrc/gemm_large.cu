@@ -971,10 +971,11 @@ bool large_pays(int M, int N, int K) {
     // 30 blocks, 1024x7680: 14.9 / 16.0 / 17.4, here 14.8 / 14.8 / 15.0; 33, 1792x8320: 17.2 / 18.4 / 22.4, here 16.8.
     // (With clusters 640x8192 takes 7.7 / 7.8 / 8.2 here. The line stays where callers of the query found it.)
     if (M <= 64 && kblocks > 30 && kblocks <= 32 && tiles <= (M <= 48 ? 16 : 8)) return false;
-    // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two rounds, 4.2 us and
-    // 0.66 a K block (the estimate of the other kernel is good to 4 %: 4.6 and 0.68). 24576x4096: 13 tokens 16.8 / 14.7, 16 tokens 18.7 / 14.6; 24576x2048: 13 tokens 9.6 / 9.9, 16 tokens
-    // 10.6 / 9.9; 19456x2048: 13 tokens 9.3 / 9.5.
-    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 4.6 + 0.68 * kblocks;
+    // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two rounds. The line was
+    // drawn when a K block took 0.48 us here (24576x4096, 16 tokens 17.4 / 18.5; 20480x2048 9.8 / 10.8; but 24064x2304, where
+    // the decode kernel splits K, 15.3 / 11.5) and is kept with the answers of the query; at 0.24 us a block this kernel
+    // gains on its own side of it: 24576x4096, 16 tokens 18.7 / 14.6, 13 tokens 16.8 / 14.7; 24576x2048 10.6 / 9.9.
+    if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 3.9 + 0.96 * kblocks;
     return true;
 }
 
@@ -986,10 +987,10 @@ size_t large_scratch_bytes(int M, int N, int K) {
 
 // The host's side: a second launch and the scratch bring a call to 9.4 us or more even where the device needs 5, while
 // a call of the decode kernel ends at 6.5. So up to 32 tokens (one launch of it) that kernel keeps what it does in
-// less than 10 us; up to 16 tokens, where the device times lie close together, in less than 12. Measured, us a call:
-// 12288x2048 24 tokens 10.4 / 9.5; 8192x2048 20 tokens 11.3 / 9.6, 6144x4096 11.1 / 9.6; 12288x2048 20 tokens 9.5 / 10.1;
-// 24576x2048 16 tokens 9.9 / 10.6.
-constexpr double kLargeCallUs = 10.0, kLargeCallUsFew = 12.0;
+// less than 11 us (the estimate is good to 4 %); up to 16 tokens, where the device times lie close together, in less
+// than 12. Measured, us a call: 8192x2048 20 tokens 11.3 / 9.6, 6144x4096 11.1 / 9.6; 12288x2048 24 tokens 10.4 / 9.5,
+// 20 tokens 9.5 / 10.1; 24576x2048 16 tokens 9.9 / 10.6.
+constexpr double kLargeCallUs = 11.0, kLargeCallUsFew = 12.0;
 
 int large_route(int M, int N, int K) {
     if (!large_pays(M, N, K)) return NVFP4R_ROUTE_PACKED;
