@@ -29,9 +29,8 @@
 //                sums of the columns that a peer owns into that peer's shared memory (the ring, idle by then), and
 //                every CTA adds up and stores its own columns, in K order. The hardware places a cluster as a whole,
 //                so nothing waits for a CTA that might not be running, and no scratch is needed.
-//
 //   pairs        two SMs on one tile of 256 weight rows (cta_group::2): each holds its 128 rows and half of the tokens,
-//                36 KB a stage instead of 55 KB at 256 tokens; one of the two issues for both, the other announces
+//                38 KB a stage instead of 55 KB at 256 tokens; one of the two issues for both, the other announces
 //                its stages to it. For many tokens, where the bytes are the time.
 //
 // What bounds it. Few tiles: the chain launch - quantizer - launch - first stage - MMAs - stores, of which a K block is
