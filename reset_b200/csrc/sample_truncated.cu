@@ -1,6 +1,6 @@
-// Top-k / top-p sampling of one id per row in one launch: one thread-block cluster of eight CTAs per row.
+// Top-k / top-p sampling of one id per row in one launch: one thread-block cluster of eight (or sixteen) CTAs per row.
 //
-// The row is read from memory once; each CTA keeps an eighth of it in shared memory and the eight exchange
+// The row is read from memory once; each CTA keeps its share of it in shared memory and all exchange
 // histograms, totals and picks through distributed shared memory with cluster barriers. Phases:
 //   1. load, row maximum;
 //   2. top-k up to 128: the k-th largest of the 128 warps' maxima bounds the k-th largest value from below (k
@@ -12,8 +12,8 @@
 //      bin, its entries go to one CTA's list, and with at most 512 of them that CTA finds the threshold by comparing all
 //      pairs. The distance rounds monotonically, so bins are in the order of the values;
 //   4. where more entries share the bin, or the goal lies beyond the steps, a radix descent over the order-preserving keys,
-//      11 + 11 + 10 bits: histogram of the keys that share the prefix found so far, each CTA sums 256 of the
-//      2048 bins over the eight histograms, and the CTA whose bins cross the goal announces the bin. After
+//      11 + 11 + 10 bits: histogram of the keys that share the prefix found so far, each CTA sums its share of the
+//      2048 bins over all histograms, and the CTA whose bins cross the goal announces the bin. After
 //      the last level the prefix is the key of the last token kept; equal keys are all kept;
 //   5. arg-max of logit + Gumbel noise among the keys at or above the threshold.
 // Mass is exp(x - row max) scaled by 2^32 and truncated to an integer, so no result depends on the order of
@@ -27,18 +27,21 @@
 //   top-k 1000            1 row 37.1 -> 24.1   8 rows 45.1 -> 26.1   32 rows 96 -> 34.8    256 rows 657 -> 268
 // and with phase 3, the masses in 32-bit halves and the draw's logarithms only where they can matter, device us in a CUDA
 // graph with the counters' reset, radix descent -> steps:
-//   top-p 0.9   1 row 31.6 -> 23.0   8 rows 39.4 -> 30.0   32 rows 53.8 -> 38.8     top-k 1000, 8 rows 27.9 -> 22.4
+//   top-p 0.9   1 row 31.6 -> 19.2   8 rows 39.4 -> 26.8   32 rows 53.8 -> 38.8     top-k 1000, 8 rows 27.9 -> 22.4
 //   top-k 150 top-p 0.8, 8 rows 40.2 -> 28.6
-// of which, 8 rows, thousand clocks: load 5, histogram 11, its bin 6, list 5, pairs 3, draw 13.
+// of which, 8 rows in clusters of eight, thousand clocks: load 5, histogram 11, its bin 6, list 5, pairs 3, draw 13.
 // (the first line without phase 2: 35.1, 37.6, 47.2, 373)
 //
-//   * 8 CTAs of 512 threads: the largest cluster every device can place, and at 151936 entries two CTAs
+//   * 8 CTAs of 512 threads (16 for a few rows of top-p alone, where the device can place them): the largest cluster every
+//     device can place, and at 151936 entries two CTAs
 //     (76 KB of row each) fit an SM, so 32 rows run at once.
 //   * A shared-memory add on a 64-bit word is a compare-and-swap loop, and logits crowd into few of the
 //     first level's bins. So masses are added as two 32-bit halves (16 + 17 bits; a slice has fewer than
 //     65536 elements, so neither overflows), and top-k counts only what reaches the bound of phase 2. Rows too
 //     long for shared memory are re-read from L2 and use 64-bit adds.
 #include <cooperative_groups.h>
+
+#include <atomic>
 
 #include "kernels.h"
 #include "nvfp4_ptx.cuh"
@@ -49,17 +52,16 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int kCtas = 8;                       // CTAs per row
+constexpr int kFewCtas = 8, kMostCtas = 16;    // CTAs per row
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kBins = 2048;
-constexpr int kSeg = kBins / kCtas;            // bins that one CTA sums
 constexpr int kMaxCached = 48 * 1024;          // elements of a slice kept in shared memory (192 KB)
 
 __host__ __device__ constexpr int level_shift(int level) { return level == 0 ? 21 : (level == 1 ? 10 : 0); }
 __host__ __device__ constexpr int level_bins(int level) { return level == 2 ? 1024 : 2048; }
 
-constexpr int kGroups = kCtas * kWarps;        // groups of a row: one per warp
+constexpr int kGroups = kFewCtas * kWarps;     // groups of a row for phase 2: one per warp
 constexpr int kListMax = kThreads;                // candidates that one CTA settles, one per thread
 
 __device__ __forceinline__ unsigned long long mass_of(float x, float m) {
@@ -75,11 +77,13 @@ __device__ __forceinline__ void mass_halves(float x, float m, uint32_t& w_lo, ui
 }
 
 // kFew: 0 < top_k <= kGroups (its own instance: the list's code costs the descent registers)
-template <bool kCached, bool kFew>
+template <bool kCached, bool kFew, int kCtas>
 __global__ void __launch_bounds__(kThreads, 2)
 sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int per, int top_k, float top_p,
                         unsigned long long seed, unsigned long long* __restrict__ draws,
                         int* __restrict__ last_ids, int* __restrict__ out) {
+    constexpr int kSeg = kBins / kCtas;                       // bins that one CTA sums
+    static_assert(!kFew || kCtas == kFewCtas, "one group per warp of eight CTAs");
     extern __shared__ __align__(16) float s_row[];            // [per] when kCached
     // counts [kBins]; masses: low halves [kBins] and high halves [kBins], or 64-bit words [kBins]
     __shared__ __align__(16) uint32_t s_hist[2 * kBins];
@@ -456,33 +460,70 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
     }
 }
 
+// Rows that clusters of 16 CTAs (more than every device can place) can have at once: asked once per device for slices that
+// leave room for two CTAs per SM and once for the largest.
+int rows_at_once(int dev, int per) {
+    if (dev < 0 || dev >= 64) return 0;
+    constexpr int kTwoPerSm = 22 * 1024;
+    static std::atomic<int> known[64][2] = {};                // answer + 1
+    const int large = per > kTwoPerSm;
+    const int last = known[dev][large].load(std::memory_order_acquire);
+    if (last > 0) return last - 1;
+    const auto kern = sample_truncated_kernel<true, false, kMostCtas>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kMostCtas, 1);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(large ? kMaxCached : kTwoPerSm) * sizeof(float);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kMostCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxCached * static_cast<int>(sizeof(float))) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    known[dev][large].store(n + 1, std::memory_order_release);
+    return n;
+}
+
 }  // namespace
 
 cudaError_t launch_sample_truncated(const float* logits, int64_t row_stride, int B, int V, int top_k, float top_p,
                                     unsigned long long seed, unsigned long long* draws, int* last_ids, int* out,
                                     cudaStream_t stream) {
-    const int per = static_cast<int>(((static_cast<int64_t>(V) + kCtas - 1) / kCtas + 3) / 4 * 4);
-    const bool cached = per <= kMaxCached;
     const bool few = top_k > 0 && top_k <= kGroups;
-    const auto kern = cached ? (few ? sample_truncated_kernel<true, true> : sample_truncated_kernel<true, false>)
-                             : (few ? sample_truncated_kernel<false, true> : sample_truncated_kernel<false, false>);
-    static bool attr_done[2][64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (cached && (dev < 0 || dev >= 64 || !attr_done[few][dev])) {
+    const auto slice = [&](int ctas) { return static_cast<int>(((static_cast<int64_t>(V) + ctas - 1) / ctas + 3) / 4 * 4); };
+    // Top-p alone is passes over the row: sixteen CTAs, while all rows find a place at once. 1 row 23.0 -> 19.2 us, 4 rows
+    // 29.8 -> 23.4, 8 rows 30.0 -> 26.8, 12 rows 30.4 -> 29.0. With top-k the row is counted in less time than the larger
+    // cluster's barriers add: 8 rows, top-k 1000 22.3 / 23.7, top-k 150 top-p 0.8 28.5 / 30.3.
+    const bool most = top_k <= 0 && slice(kMostCtas) <= kMaxCached && B <= rows_at_once(dev, slice(kMostCtas));
+    const int ctas = most ? kMostCtas : kFewCtas, per = slice(ctas);
+    const bool cached = per <= kMaxCached;
+    const auto kern = most ? sample_truncated_kernel<true, false, kMostCtas>
+                      : cached ? (few ? sample_truncated_kernel<true, true, kFewCtas> : sample_truncated_kernel<true, false, kFewCtas>)
+                               : (few ? sample_truncated_kernel<false, true, kFewCtas> : sample_truncated_kernel<false, false, kFewCtas>);
+    static bool attr_done[2][64] = {};
+    if (!most && cached && (dev < 0 || dev >= 64 || !attr_done[few][dev])) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxCached * static_cast<int>(sizeof(float)));
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_done[few][dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kCtas, static_cast<unsigned>(B));
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas), static_cast<unsigned>(B));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = cached ? static_cast<size_t>(per) * sizeof(float) : 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kCtas;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;

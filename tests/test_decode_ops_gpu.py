@@ -517,7 +517,8 @@ def test_decode_step_runs_with_every_tensor_parallel_shard_shape(world, monkeypa
     (0.37, 3, 60.0, 0, 0.9),         # and the nucleus is the peak alone
     (0.37, 3, float("inf"), 140, 0.999),
 ])
-def test_sample_threshold_between_levels(V, gap, per, peak, top_k, top_p):
+@pytest.mark.parametrize("rows", [4, 64])                                # clusters of 16 and of 8 CTAs
+def test_sample_threshold_between_levels(rows, V, gap, per, peak, top_k, top_p):
     """Logits on a ladder of levels, ``per`` equal entries each: the set ends between two levels or takes a whole one, so
     rounding cannot move it. Every id drawn is in the set, and the lowest level of a small set is drawn too."""
     from reset_b200 import capi
@@ -545,13 +546,12 @@ def test_sample_threshold_between_levels(V, gap, per, peak, top_k, top_p):
             assert abs(above - goal) > 1e-5 * goal                       # the case is decided by more than rounding
             above += w[d == v].sum().item()
     perm = torch.randperm(V, generator=g)
-    rows = 64
     logits = x[perm].repeat(rows, 1).contiguous().cuda()
     allowed = keep[perm]
     ids = []
     draws = torch.zeros(rows, dtype=torch.int64, device="cuda")
     ws = capi.sample_workspace(rows, "cuda")
-    for _ in range(24):
+    for _ in range(1536 // rows):
         ids.append(capi.sample(logits, draws, seed=11, top_k=top_k, top_p=top_p, workspace=ws).cpu().long())
     ids = torch.cat(ids)
     assert allowed[ids].all()
