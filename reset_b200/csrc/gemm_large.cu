@@ -291,9 +291,15 @@ __device__ __forceinline__ void store_cols(const LargeParams& p, const Store& st
         }
     } else if (kDtype == 2) {
         float* o = static_cast<float*>(p.out) + static_cast<int64_t>(m0) * p.ldc + n0 + st.row;
+        // A test and a product per store cost more than the store: 23680x1024 with 588 tokens 29.2 us, 18.0 without.
+        if (m0 + kCols <= p.M) {
 #pragma unroll
-        for (int j = 0; j < kCols; ++j)
-            if (m0 + j < p.M) o[static_cast<int64_t>(j) * p.ldc] = v[j];
+            for (int j = 0; j < kCols; ++j, o += p.ldc) *o = v[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < kCols; ++j, o += p.ldc)
+                if (m0 + j < p.M) *o = v[j];
+        }
     } else {
         uint16_t* mine = reinterpret_cast<uint16_t*>(st.chunk) + st.row;
 #pragma unroll
