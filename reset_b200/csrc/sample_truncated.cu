@@ -432,7 +432,8 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
 
     // ---- Gumbel-max draw within the set --------------------------------------------------------------
     // The two logarithms are taken only where they can matter: -log(-log u) <= -log(1 - u), so an element stays below
-    // the best score of the CTA so far when 1 - u > exp(x - best); the 1 % covers the rounding of both sides.
+    // the best score of the CTA so far when 1 - u > exp(x - best). The 1 % covers the rounding of the two sides; the sum
+    // x + noise rounds up by half a unit of best at most, which 2^-23 best in the exponent covers at any magnitude.
     const unsigned long long key = gumbel_key(seed, b, draws[b]);
     if (tid == 0) s_bound = 0u;
     __syncthreads();
@@ -441,7 +442,8 @@ sample_truncated_kernel(const float* __restrict__ logits, int64_t row_stride, in
         if (!(x > -INFINITY) || sortable_key(x) < thr_key) return;
         const float u = gumbel_uniform(key, i);
         const uint32_t so_far = *bound;
-        if (so_far != 0u && 1.0f - u > 1.01f * __expf(x - key_value(so_far))) return;
+        const float top = key_value(so_far);
+        if (so_far != 0u && 1.0f - u > 1.01f * __expf(fmaf(fabsf(top), 1.0f / 8388608.0f, x - top))) return;
         const float s = x + gumbel_of(u);
         if (s > best) { best = s; arg = i; }
         const uint32_t mine = sortable_key(s);

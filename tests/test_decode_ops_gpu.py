@@ -559,3 +559,26 @@ def test_sample_threshold_between_levels(rows, V, gap, per, peak, top_k, top_p):
     low = d[keep].min()
     if p[d == low].sum() > 0.01:                                         # 1536 draws: missed with probability below 2e-7
         assert (x[perm].double()[ids] == low).any()
+
+
+@pytest.mark.parametrize("rows", [4, 64])                                # clusters of 16 and of 8 CTAs
+@pytest.mark.parametrize("value", [3.0e5, 4.0e6, 1.0e8, -1.0e8])
+def test_sample_equal_scores_of_large_logits_go_to_the_lowest_index(rows, value):
+    """Logits so large that the fp32 score swallows part of the noise (a unit of 1/32 to 8 at these values): up to
+    hundreds of elements share the best score and the lowest index wins. The noise is known to 1e-5 (a few ulp of at
+    most 20); rows where that could move an element into or out of the best score are left out."""
+    from reset_b200 import capi
+    V, seed = 20011, 77
+    logits = torch.full((rows, V), value).cuda()
+    draws = torch.arange(rows, dtype=torch.int64, device="cuda")
+    ids = capi.sample(logits, draws, seed=seed, top_p=0.9, workspace=capi.sample_workspace(rows, "cuda")).tolist()
+    checked = 0
+    for b in range(rows):
+        exact = _gumbel_scores(np.full(V, value, np.float32), seed, b, b)
+        lo, hi = (exact - 1e-5).astype(np.float32), (exact + 1e-5).astype(np.float32)
+        best = hi.max()
+        if ((hi == best) & (lo < best)).any():
+            continue
+        checked += 1
+        assert ids[b] == int(np.argmax(lo == best)), b
+    assert checked >= rows // 2
