@@ -582,3 +582,32 @@ def test_sample_equal_scores_of_large_logits_go_to_the_lowest_index(rows, value)
         checked += 1
         assert ids[b] == int(np.argmax(lo == best)), b
     assert checked >= rows // 2
+
+
+@pytest.mark.parametrize("rows", [4, 64])                                # clusters of 16 and of 8 CTAs
+@pytest.mark.parametrize("V,spread,top_k,top_p", [
+    (151936, 3.0, 0, 0.9), (151936, 0.5, 0, 0.99), (20011, 1.0, 0, 0.5), (151936, 3.0, 1000, 1.0), (151936, 3.0, 400, 0.8),
+    (400003, 2.0, 0, 0.9),
+])
+def test_sample_draws_the_exact_id_of_a_wide_set(rows, V, spread, top_k, top_p):
+    """The id is the restated generator's arg-max over the exact set. The set's edge by mass is known to 1e-4 (masses are
+    exp() in fp32, cut at 2^-32 of the largest), and scores to 1e-4 as above: the id is in the wider set and scores no
+    less than the best of the narrower."""
+    from reset_b200 import capi
+    seed = 5
+    x = torch.randn(rows, V, generator=torch.Generator().manual_seed(V + top_k)) * spread
+    draws = torch.arange(rows, dtype=torch.int64, device="cuda")
+    ids = capi.sample(x.cuda(), draws, seed=seed, top_k=top_k, top_p=top_p,
+                      workspace=capi.sample_workspace(rows, "cuda")).tolist()
+    for b in range(min(rows, 6)):
+        row = x[b].numpy()
+        d = np.sort(row.astype(np.float64))[::-1]
+        if top_k:
+            d = d[:top_k]
+        floors = [d[-1], d[-1]]                                          # narrower set, wider set
+        if top_p < 1.0:
+            mass = np.cumsum(np.exp(d - d[0]))
+            floors = [d[min(np.searchsorted(mass, p * mass[-1]), d.size - 1)] for p in (top_p * (1 - 1e-4), top_p * (1 + 1e-4))]
+        score = _gumbel_scores(row, seed, b, b)
+        assert row[ids[b]] >= floors[1], b
+        assert score[ids[b]] >= score[row >= floors[0]].max() - 1e-4, b
