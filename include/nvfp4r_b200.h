@@ -156,6 +156,8 @@ NVFP4R_API int nvfp4r_linear(const void* x, int64_t x_row_stride, int M, int K,
  * nvfp4r_linear_tc and the 32-row path build a TMA descriptor on the host
  * (cuTensorMapEncodeTiled) and cache it per (pointer, shape); the many-token kernel
  * encodes two per call.
+ * Every operand, the weight and its scales among them, may be written by the preceding kernel
+ * of the stream.
  * ------------------------------------------------------------------------- */
 #define NVFP4R_GEMM_TICKET_BYTES 16384
 typedef enum nvfp4r_c_layout { NVFP4R_C_M_MAJOR = 0, NVFP4R_C_N_MAJOR = 1 } nvfp4r_c_layout;
@@ -169,7 +171,8 @@ NVFP4R_API int nvfp4r_gemm(const void* A, const void* B, const void* SFA, const 
  * branch of `_nvfp4r_linear_impl` (kernels/python/nvfp4r/vllm_integration.py:224-274:
  * scaled_fp4_quant + pad to 64 rows + nvfp4r.gemm + transpose + contiguous) in one
  * launch per 32 rows. weight [N,K/2]; weight_scale_swizzled in 128x4 tiles (the layout
- * vLLM keeps in layer.weight_scale); workspace as for nvfp4r_gemm. */
+ * vLLM keeps in layer.weight_scale); workspace as for nvfp4r_gemm. The weight and its scales are
+ * constants of the layer and must be final before the preceding kernel of the stream is launched. */
 NVFP4R_API int nvfp4r_linear_tc(const void* x, int64_t x_row_stride, int M, int K,
                                 const float* global_scale_inv, const void* weight,
                                 const void* weight_scale_swizzled, int N, float alpha,

@@ -41,7 +41,7 @@
 // the issuer is straight-line code per K block (rolled loops made each tcgen05 instruction wait for its operands).
 // Device time in a CUDA graph, weights cold, us, one CTA a tile or stream-K with all of that before -> after:
 //   10240x5120  45 tokens 12.4 -> 10.1     6144x4096  333 tokens 13.9 -> 11.2     34816x5120  16 tokens 21.9 -> 19.9
-//   1024x4096   16 tokens 8.5 -> 6.1 (clusters of 4)    4096x12288 128 tokens, quant + gemm 21.3 -> 14.9 (clusters of 4)
+//   1024x4096   16 tokens 8.5 -> 6.1 (clusters of 4)    4096x12288 128 tokens, quant + gemm 21.3 -> 14.0 (clusters of 4)
 //   24576x4096  512 tokens 32.5 -> 28.7, 1300 69.4 -> 57.0, 2048 104.9 -> 85 to 88 (pairs)
 #include <cuda.h>
 
@@ -475,10 +475,11 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
             o.b += kTma ? 2048u : b_bytes;
             o.ax += 128;
         };
-        // The weight does not depend on the kernel before: the weight half of the first stages is
-        // requested ahead of the wait, the token half behind it.
+        // A packed weight does not depend on the kernel before: the weight half of the first stages is requested ahead of the
+        // wait, the token half behind it. The raw operator's weight may be that kernel's output, and what it wrote is only
+        // sure to be visible behind the wait, also where it let this one in at its end. Behind a quantizer it costs nothing.
         int pre = 0;
-        {
+        if (!kTma) {
             Walker wa(p, kPair);
             Segment sa;
             uint32_t dst = ring, bar = bar_full;

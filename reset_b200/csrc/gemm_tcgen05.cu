@@ -149,14 +149,17 @@ linear_tc_kernel(const __grid_constant__ TcParams p) {
                  bar_full + 8 * s, policy);
     };
 
-    // The weight stream does not depend on the preceding kernel: fill the ring now.
+    // The fused linear's weight is a constant of the layer: the ring is filled while the preceding kernel may still run. The raw
+    // operator's may be that kernel's output, of which nothing is sure to be visible ahead of the wait.
     int issued = 0;
-    if (warp == 0 && lane == 0) {
-        const int first = min(p.stages, total);
-        for (; issued < first; ++issued) issue(issued);
-    }
+    auto fill = [&] {
+        if (warp != 0 || lane != 0) return;
+        for (const int first = min(p.stages, total); issued < first; ++issued) issue(issued);
+    };
+    if (p.xb != nullptr) fill();
     pdl_launch_dependents();
     pdl_wait_prior();
+    if (p.xb == nullptr) fill();
 
     // ---- prologue: activations of K range [it0*256, it1*256) into operand layout -------
     {

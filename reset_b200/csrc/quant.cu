@@ -7,10 +7,10 @@ namespace {
 
 // One CTA per row and 256 blocks of 16 elements, one thread per block: no division in the index, and the four scales of
 // a quad of lanes leave as one word of the swizzled layout. Bound: launch and one trip to memory. It is launched
-// programmatically; the next kernel is let in behind the stores, for a gemm fetches its weight ahead of its own wait and
-// the weight may be what was quantized here. Swizzled scales,
-// chained in a CUDA graph, us, one thread per scale with 64-bit divisions and a plain launch -> now: 2x12288 1.64 -> 1.41,
-// 128x12288 2.32 -> 1.82, 1000x4096 3.79 -> 3.12.
+// programmatically itself, but lets nothing in before it has ended: what it writes may be a weight, which the kernels that
+// multiply request before they wait for their predecessor, and launch_dependents makes no store visible. Swizzled scales,
+// chained in a CUDA graph, us, one thread per scale with 64-bit divisions and a plain launch -> now: 2x12288 1.64 -> 1.44,
+// 128x12288 2.32 -> 1.77, 1000x4096 3.79 -> 2.79.
 template <int kMode, bool kSwizzled>
 __global__ void __launch_bounds__(256)
 quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, int M, int cols, const float* __restrict__ gs_ptr,
@@ -36,7 +36,6 @@ quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_row_stride, int M, i
     } else {
         scales[kSwizzled ? swizzled_sf_offset(row, col, cols_out) : static_cast<int64_t>(row) * cols + col] = static_cast<uint8_t>(sf);
     }
-    pdl_launch_dependents();
 }
 
 template <bool kToFlat>

@@ -221,3 +221,17 @@ def test_kernel_of_a_packed_linear_of_13_to_65_tokens(M, N, K, device, call):
     lib = _lib.lib()
     assert lib.nvfp4r_linear_packed_route(M, N, K) == (0 if not device else 1 + call)
     assert lib.nvfp4r_linear_packed_scratch_bytes(M, N, K) > 0 or not device
+
+
+def test_kernels_that_write_operands_let_nothing_in_before_they_end():
+    """The fused linears and the GEMV request their weight ahead of griddepcontrol.wait, so the kernels that write one have no
+    griddepcontrol.launch_dependents of their own (it makes no store visible); the raw gemm waits before it requests."""
+    csrc = REPO / "reset_b200" / "csrc"
+    code = lambda text: re.sub(r"//[^\n]*", "", text)
+    assert "launch_dependents" not in code((csrc / "quant.cu").read_text())
+    linear = code((csrc / "linear_packed.cu").read_text())
+    pack = linear[linear.index("pack_weight_kernel("):]
+    assert "launch_dependents" not in pack[:pack.index("\n}\n")]
+    large = code((csrc / "gemm_large.cu").read_text())
+    before_wait = large[large.index("int pre = 0;"):]
+    assert re.match(r"int pre = 0;\s*if \(!kTma\) \{", before_wait)

@@ -340,3 +340,42 @@ def test_eager_and_captured_calls_give_the_same_product(capi, M, N, K):
     g.replay()
     for got in (eager, out):
         assert rel_l2(got.cpu().numpy(), exact) <= 1e-5
+
+
+@pytest.mark.parametrize("M,dtype", [(1, torch.bfloat16), (32, torch.float16), (32, torch.float32), (33, torch.float16), (300, torch.bfloat16),
+                                     (1500, torch.bfloat16)])
+def test_gemm_directly_behind_the_quantizer_of_its_weight(capi, M, dtype):
+    """The weight is quantized last, into buffers that hold the weight before it, and multiplied at once: the call gives
+    what it gives when everything has ended before it."""
+    from reset_b200 import _lib
+    lib, N, K = _lib.lib(), 2560, 4096
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, generator=gen, device="cuda").bfloat16()
+    weights = [torch.randn(N, K, generator=gen, device="cuda").bfloat16() for _ in range(3)]
+    gs = torch.tensor([300.0], device="cuda")
+    xc, xsf = capi.quant(x, gs, swizzled=True)
+    wc, wsf = torch.empty(N, K // 2, dtype=torch.uint8, device="cuda"), torch.empty(N, K // 16, dtype=torch.uint8, device="cuda")
+    wksp = torch.zeros(4 << 20, dtype=torch.int64, device="cuda")
+
+    def quantize(w):
+        _lib.check(lib.nvfp4r_quant(w.data_ptr(), K, N, K, gs.data_ptr(), wc.data_ptr(), wsf.data_ptr(), _lib.SF_SWIZZLED, 1,
+                                    torch.cuda.current_stream().cuda_stream), "quant")
+
+    def product():
+        C = torch.empty((M, N), dtype=dtype, device="cuda")
+        capi.gemm(xc, wc, xsf, wsf, C, 1e-5, wksp)
+        return C
+
+    want = []
+    for w in weights:
+        quantize(w)
+        torch.cuda.synchronize()
+        want.append(product())
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    got = []
+    for i in range(12):
+        quantize(weights[i % 3])
+        got.append(product())
+    for i in range(12):
+        assert torch.equal(got[i], want[i % 3]), i
