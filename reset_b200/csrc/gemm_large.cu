@@ -14,7 +14,8 @@
 //   packed     weight in the packed block format of linear_packed.cu (18 432 contiguous bytes per
 //              128 rows x 256 K), tokens written by quant_pack_kernel in the same kind of block for
 //              bn rows: [bn x 128 B of codes, 128-byte swizzle][2048 B of scales per 128 rows].
-//              A pipeline stage (256 K-elements) is two 1-D bulk copies.
+//              A pipeline stage (256 K-elements) is two 1-D bulk copies, in a CTA of a pair
+//              three tensor-map loads of the same bytes (weight, its half of the codes, token scales).
 //   row-major  codes through 2-D tensor maps (128-byte swizzle), scales in the 128x4-tiled layout as
 //              512-byte chunks: the operands of the raw gemm operator.
 //
@@ -30,8 +31,8 @@
 //                every CTA adds up and stores its own columns, in K order. The hardware places a cluster as a whole,
 //                so nothing waits for a CTA that might not be running, and no scratch is needed.
 //   pairs        two SMs on one tile of 256 weight rows (cta_group::2): each holds its 128 rows and half of the tokens,
-//                38 KB a stage instead of 55 KB at 256 tokens; one of the two issues for both, the other announces
-//                its stages to it. For many tokens, where the bytes are the time.
+//                38 KB a stage instead of 55 KB at 256 tokens; one of the two issues for both, and the other's loads
+//                complete on its barriers. For many tokens, where the bytes are the time.
 //
 // What bounds it. Few tiles: the chain launch - quantizer - launch - first stage - MMAs - stores, of which a K block is
 // 0.24 us: 515 clocks of the issuing warp (12 tcgen05 instructions at 17 to 25 clocks, a wait, a commit) against 218 for
@@ -48,6 +49,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.h"
 #include "quant_core.cuh"
@@ -69,6 +71,7 @@ constexpr int kThreadsL = (2 + kEpiWarps) * 32;
 constexpr int kStoreChunk = 32 * kRows * 2;          // 32 tokens x 128 rows of a 16-bit output on their way to memory
 constexpr int kStoreBytes = 2 * kStoreChunk;         // one for each column half
 constexpr int kSmemBudget = 225 * 1024;              // dynamic part, 1 KB of it for alignment
+constexpr int kMapRow = 1024;                        // contiguous operands of a pair as a map: bytes of a row
 constexpr int kPairTuning = 9;                       // set_large_tuning: pairs of SMs
 constexpr int kMaxSplit = 8;                         // the largest cluster that every device can place
 // Time model of plan_large, nanoseconds, fitted to sweeps over tile widths and schedules (eight weights, 16 .. 700
@@ -92,7 +95,8 @@ __host__ __device__ constexpr int acc_overlap(int bn) { return bn > kNoOverlap ?
 constexpr uint32_t kColSfaL = 416, kColSfbL = 448, kColSfa1 = 464, kColSfb1 = 480;
 
 struct alignas(64) LargeParams {
-    CUtensorMap map_w, map_x;                        // row-major form only
+    CUtensorMap map_w, map_x;                        // row-major form: codes; packed form, pairs: weight blocks, token codes
+    CUtensorMap map_xsf;                             // pairs: token scales
     const uint8_t* w;                                // packed weight blocks
     const uint8_t* x;                                // packed token blocks
     const uint8_t* wsf;                              // row-major form: 128x4-tiled scales
@@ -107,6 +111,11 @@ struct alignas(64) LargeParams {
     float* partials;                                 // [2 * sk_ctas][bn / 4][128][4]
     unsigned* tickets;                               // [tiles], zero before the launch, left zero
 };
+
+struct alignas(64) LargeParamsPairTma : LargeParams {
+    CUtensorMap map_wsf;                             // pairs of the row-major form: weight scales
+};
+template <bool kTma, bool kPair> using ParamsOf = std::conditional_t<kTma && kPair, LargeParamsPairTma, LargeParams>;
 
 __device__ int g_large_status = 0;
 
@@ -355,7 +364,8 @@ __device__ __forceinline__ void issue_all(const LargeParams& p, uint32_t ring, u
     for (int t = 0; !wf.failed && wk.next(p, sg); ++t) {
         const int buf = t & 1;
         // overlapping accumulators: one barrier, the tile before has left the tokens that both hold; else one per buffer
-        if (overlap ? t > 0 && !wf.wait(bar_accempty, (t - 1) & 1) : t > 1 && !wf.wait(bar_accempty + 8 * buf, ((t >> 1) - 1) & 1)) break;
+        const auto emptied = [&](uint32_t bar, uint32_t parity) { return kPair ? wf.wait_cluster(bar, parity) : wf.wait(bar, parity); };
+        if (overlap ? t > 0 && !emptied(bar_accempty, (t - 1) & 1) : t > 1 && !emptied(bar_accempty + 8 * buf, ((t >> 1) - 1) & 1)) break;
         tc_fence_after();
         const uint32_t d = tmem + buf * stride;
         uint32_t more = 0;
@@ -384,7 +394,7 @@ __device__ __forceinline__ void issue_all(const LargeParams& p, uint32_t ring, u
 
 template <bool kTma, int kDtype, bool kNMajor, bool kPair>
 __global__ void __launch_bounds__(kThreadsL, 2)
-gemm_large_kernel(const __grid_constant__ LargeParams p) {
+gemm_large_kernel(const __grid_constant__ ParamsOf<kTma, kPair> p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(8) uint64_t bars[2 * kMaxStagesL + 4];
@@ -400,9 +410,9 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
     const uint32_t bar_accfull = smem_u32(&bars[2 * kMaxStagesL]), bar_accempty = bar_accfull + 16;
 
     if (warp == 0 && lane < 2 * kMaxStagesL + 4) {
-        // a pair: the issuing CTA's stages are full when the peer's are too, its accumulators empty when both are
+        // a pair: the issuing CTA's accumulators are empty when both are
         const bool acc_empty = lane >= 2 * kMaxStagesL + 2;
-        mbar_init(bar_full + 8 * lane, acc_empty ? (kPair ? 2 : 1) * kEpiWarps : kPair && rank == 0 && lane < kMaxStagesL ? 2 : 1);
+        mbar_init(bar_full + 8 * lane, acc_empty ? (kPair ? 2 : 1) * kEpiWarps : 1);
         mbar_fence_init();
     }
     if (warp == 1) {
@@ -429,28 +439,48 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
         struct Source {
             const uint8_t *a, *b;                     // packed: next block; row-major: next scales
             int ax, ay, by, ch;                       // row-major: code coordinates, scale chunks of the token tile
+            int ar, br;                               // pairs: what a and b are, in rows of the maps
         };
         auto source = [&](const Segment& sg) {
             const int t = sg.tile / p.tiles_m, mt = sg.tile - t * p.tiles_m;
             // with an odd number of row tiles the last pair's second CTA repeats the first one's and stores nothing
             const int nt = kPair ? min(2 * t + rank, (p.N / kRows) - 1) : t;
             Source o;
+            o.ch = nch;
             if (kTma) {
-                o.a = p.wsf + (static_cast<int64_t>(nt) * p.k64 + sg.k0 * 4) * 512;
-                o.b = p.xsf + (static_cast<int64_t>(mt * nch) * p.k64 + sg.k0 * 4) * 512;
                 o.ax = sg.k0 * 128;
                 o.ay = nt * kRows;
                 o.by = mt * bn + rank * (bn / 2);
                 o.ch = min(nch, (p.M - mt * bn + 127) >> 7);          // chunks that exist in xsf
+                const int64_t a = static_cast<int64_t>(nt) * p.k64 + sg.k0 * 4, b = static_cast<int64_t>(mt * nch) * p.k64 + sg.k0 * 4;
+                o.a = p.wsf + a * 512;
+                o.b = p.xsf + b * 512;
+                o.ar = static_cast<int>(a / 2);                       // K % 256 == 0: four chunks a block
+                o.br = static_cast<int>(b / 2);
             } else {
-                o.a = p.w + (static_cast<int64_t>(nt) * p.kblocks + sg.k0) * kABytes;
-                o.b = p.x + (static_cast<int64_t>(mt) * p.kblocks + sg.k0) * b_bytes;
-                o.ch = nch;
+                const int64_t a = static_cast<int64_t>(nt) * p.kblocks + sg.k0, b = static_cast<int64_t>(mt) * p.kblocks + sg.k0;
+                o.a = p.w + a * kABytes;
+                o.b = p.x + b * b_bytes;
+                o.ar = static_cast<int>(a) * (kABytes / kMapRow);
+                o.br = static_cast<int>(b) * static_cast<int>(b_bytes / kMapRow);
             }
             return o;
         };
+        // A pair: all loads of a stage, the peer's too, complete on the issuing CTA's barrier, which expects all of their bytes.
         auto load_a = [&](const Source& o, uint32_t dst, uint32_t bar) {
-            mbar_expect_tx(bar, kABytes + b_codes + static_cast<uint32_t>(o.ch) * 2048u);
+            const uint32_t bytes = kABytes + b_codes + static_cast<uint32_t>(o.ch) * 2048u;
+            if (kPair) {
+                if (rank == 0) mbar_expect_tx(bar, 2 * bytes);
+                const uint32_t there = cluster_map(bar, 0);
+                if constexpr (kTma && kPair) {
+                    tma_load_2d_pair(dst, &p.map_w, o.ax, o.ay, there, policy);
+                    tma_load_2d_pair(dst + kACodes, &p.map_wsf, 0, o.ar, there, policy);
+                } else {
+                    tma_load_2d_pair(dst, &p.map_w, 0, o.ar, there, policy);
+                }
+                return;
+            }
+            mbar_expect_tx(bar, bytes);
             if (kTma) {
                 tma_load_2d(dst, &p.map_w, o.ax, o.ay, bar, policy);
                 bulk_g2s(dst + kACodes, o.a, 2048, bar, policy);
@@ -459,13 +489,19 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
             }
         };
         auto load_b = [&](const Source& o, uint32_t dst, uint32_t bar) {
-            if (kTma) {
+            if (kPair) {
+                const uint32_t there = cluster_map(bar, 0);
+                if constexpr (kTma && kPair) {
+                    tma_load_2d_pair(dst, &p.map_x, o.ax, o.by, there, keep);
+                    for (int j = 0; j < o.ch; ++j) tma_load_2d_pair(dst + b_codes + j * 2048, &p.map_xsf, 0, o.br + j * (p.k64 / 2), there, keep);
+                } else {
+                    tma_load_2d_pair(dst, &p.map_x, 0, o.br + rank * static_cast<int>(b_codes / kMapRow), there, keep);
+                    tma_load_2d_pair(dst + b_codes, &p.map_xsf, 0, o.br + static_cast<int>(2 * b_codes / kMapRow), there, keep);
+                }
+            } else if (kTma) {
                 tma_load_2d(dst, &p.map_x, o.ax, o.by, bar, keep);
                 for (int j = 0; j < o.ch; ++j)
                     bulk_g2s(dst + b_codes + j * 2048, o.b + static_cast<int64_t>(j) * p.k64 * 512, 2048, bar, keep);
-            } else if (kPair) {
-                bulk_g2s(dst, o.b + rank * static_cast<int>(b_codes), b_codes, bar, keep);
-                bulk_g2s(dst + b_codes, o.b + 2 * b_codes, b_bytes - 2 * b_codes, bar, keep);
             } else {
                 bulk_g2s(dst, o.b, b_bytes, bar, keep);
             }
@@ -474,6 +510,8 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
             o.a += kTma ? 2048 : kABytes;
             o.b += kTma ? 2048u : b_bytes;
             o.ax += 128;
+            o.ar += (kTma ? 2048 : kABytes) / kMapRow;
+            o.br += static_cast<int>((kTma ? 2048u : b_bytes) / kMapRow);
         };
         // A packed weight does not depend on the kernel before: the weight half of the first stages is requested ahead of the
         // wait, the token half behind it. The raw operator's weight may be that kernel's output, and what it wrote is only
@@ -522,24 +560,13 @@ gemm_large_kernel(const __grid_constant__ LargeParams p) {
                 if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
             }
         }
-        if (wf.failed)                                 // let the copies in flight land before the CTA goes
+        if (wf.failed && rank != 0) {                  // let the copies in flight land before the CTA goes: its own are
+            for (int j = 0; j < 1000; ++j) __nanosleep(1000);        // counted by the other's barriers, it has none to ask
+        } else if (wf.failed)
             for (int j = max(0, i - stages); j < i; ++j) mbar_wait_bounded(bar_full + 8 * (j % stages), (j / stages) & 1, 100000u);
     } else if (warp == 1) {
         // ---------------- MMA issuer -----------------------------------------------------------
-        if (kPair && rank != 0) {
-            // the peer's stages are announced to the issuing CTA
-            const bool lead = elect_one();
-            const uint32_t there = cluster_map(bar_full, 0);
-            Walker wk(p, kPair);
-            Segment sg;
-            uint32_t s = 0, phase = 0;
-            while (!wf.failed && wk.next(p, sg))
-                for (int kb = sg.k0; kb < sg.k1; ++kb) {
-                    if (!wf.wait(bar_full + 8 * s, phase)) break;
-                    if (lead) mbar_arrive_cluster(there + 8 * s);
-                    __syncwarp();
-                    if (++s == static_cast<uint32_t>(stages)) { s = 0; phase ^= 1u; }
-                }
+        if (kPair && rank != 0) {                      // the other CTA issues for both
         } else if (nch == 1) {
             issue_all<1, kPair>(p, ring, tmem, bar_full, bar_empty, bar_accfull, bar_accempty, wf);
         } else {
@@ -731,6 +758,20 @@ bool code_map(const void* p, int rows, int K, int box_rows, CUtensorMap* out) {
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Contiguous memory of that many rows of kMapRow bytes, box of whole rows, no swizzle. (Promoted to 256 bytes in L2 the loads cost
+// 24576x4096 with 512 tokens 27.4 us, 27.2 so.)
+bool row_map(const void* p, int64_t rows, int box_rows, CUtensorMap* out) {
+    EncodeFn fn = encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[2] = {kMapRow / 8, static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {kMapRow};
+    const cuuint32_t box[2] = {kMapRow / 8, static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t estr[2] = {1, 1};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<void*>(p), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 struct LargePlan {
     int bn, nch, tiles_m, tiles, kblocks, stages, grid;
     int dp_rounds, sk_base, sk_ctas, split, split_cols;
@@ -870,20 +911,21 @@ bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
     return last.found;
 }
 
-using Kern = void (*)(LargeParams);
-
 constexpr int kInstances = 18;
 
-cudaError_t launch_with_pdl(int form, const LargePlan& plan, const LargeParams& p, cudaStream_t stream) {
+// p: a LargeParamsPairTma where the plan is for pairs and the form row-major.
+cudaError_t launch_with_pdl(int form, const LargePlan& plan, const LargeParams* p, cudaStream_t stream) {
     // packed operands, then row-major ones with M-major and with N-major output; bf16, fp16, fp32; by one CTA, by a pair
-#define NVFP4R_FORMS(PAIR)                                                                                             \
-    gemm_large_kernel<false, 0, false, PAIR>, gemm_large_kernel<false, 1, false, PAIR>, gemm_large_kernel<false, 2, false, PAIR>, \
-    gemm_large_kernel<true, 0, false, PAIR>, gemm_large_kernel<true, 1, false, PAIR>, gemm_large_kernel<true, 2, false, PAIR>,    \
-    gemm_large_kernel<true, 0, true, PAIR>, gemm_large_kernel<true, 1, true, PAIR>, gemm_large_kernel<true, 2, true, PAIR>
-    static const Kern table[kInstances] = {NVFP4R_FORMS(false), NVFP4R_FORMS(true)};
+#define NVFP4R_KERN(...) reinterpret_cast<const void*>(&gemm_large_kernel<__VA_ARGS__>)
+#define NVFP4R_FORMS(PAIR)                                                                                                     \
+    NVFP4R_KERN(false, 0, false, PAIR), NVFP4R_KERN(false, 1, false, PAIR), NVFP4R_KERN(false, 2, false, PAIR),                 \
+    NVFP4R_KERN(true, 0, false, PAIR), NVFP4R_KERN(true, 1, false, PAIR), NVFP4R_KERN(true, 2, false, PAIR),                    \
+    NVFP4R_KERN(true, 0, true, PAIR), NVFP4R_KERN(true, 1, true, PAIR), NVFP4R_KERN(true, 2, true, PAIR)
+    static const void* const table[kInstances] = {NVFP4R_FORMS(false), NVFP4R_FORMS(true)};
+#undef NVFP4R_KERN
 #undef NVFP4R_FORMS
     const int instance = form + (plan.pair ? kInstances / 2 : 0);
-    const Kern kern = table[instance];
+    const void* kern = table[instance];
     static std::atomic<bool> attr_done[kInstances][64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -913,7 +955,8 @@ cudaError_t launch_with_pdl(int form, const LargePlan& plan, const LargeParams& 
     }
     cfg.attrs = attr;
     cfg.numAttrs = static_cast<unsigned>(n);
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    void* args[1] = {const_cast<LargeParams*>(p)};
+    return cudaLaunchKernelExC(&cfg, kern, args);
 }
 
 template <typename... Params, typename... Args>
@@ -1023,7 +1066,13 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
     cudaError_t e = static_cast<int64_t>(g.M) * pieces <= 4 * device_sm_count() ? quant(quant_pack_kernel<1>, 1)
                                                                              : quant(quant_pack_kernel<4>, 4);
     if (e != cudaSuccess) return e;
-    return launch_with_pdl(g.out_dtype, plan, p, stream);
+    if (plan.pair) {                                   // made while the quantizer is on its way
+        const int64_t blocks = static_cast<int64_t>(plan.tiles_m) * plan.kblocks, rows = blocks * (plan.bn * 128 + plan.nch * 2048) / kMapRow;
+        if (!row_map(g.packed, static_cast<int64_t>(g.N / kRows) * plan.kblocks * (kABytes / kMapRow), kABytes / kMapRow, &p.map_w) ||
+            !row_map(tokens, rows, plan.bn * 64 / kMapRow, &p.map_x) || !row_map(tokens, rows, plan.nch * 2048 / kMapRow, &p.map_xsf))
+            return cudaErrorInvalidValue;
+    }
+    return launch_with_pdl(g.out_dtype, plan, &p, stream);
 }
 
 // The raw operator on row-major operands, any number of tokens. The decode-sized kernel keeps the tokens of a K part in
@@ -1038,9 +1087,12 @@ cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* 
     LargePlan plan;
     if (g.xb != nullptr || g.M < g_large_min_m || (g.M <= 32 && (tc_tuned() || g.out_dtype == NVFP4R_F32))) return cudaSuccess;
     if (!plan_large(g.M, g.N, g.K, true, &plan)) return cudaSuccess;
-    LargeParams p = {};
+    LargeParamsPairTma p = {};
     fill_common(plan, &p, g.out, g.M, g.N, g.K, g.alpha, g.c_n_major);
     if (!code_map(g.w, g.N, g.K, kRows, &p.map_w) || !code_map(g.a_codes, g.M, g.K, plan.pair ? plan.bn / 2 : plan.bn, &p.map_x)) return cudaSuccess;
+    if (plan.pair && (!row_map(g.wsf_swizzled, static_cast<int64_t>(g.N / kRows) * p.k64 / 2, 2, &p.map_wsf) ||
+                      !row_map(g.a_sf_swizzled, static_cast<int64_t>((g.M + 127) / 128) * p.k64 / 2, 2, &p.map_xsf)))
+        return cudaSuccess;
     p.wsf = static_cast<const uint8_t*>(g.wsf_swizzled);
     p.xsf = static_cast<const uint8_t*>(g.a_sf_swizzled);
     // The workspace, tickets included, is shared with the decode-sized kernel: both leave the tickets zero.
@@ -1053,7 +1105,7 @@ cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* 
     p.tickets = scratch.tickets;
     p.partials = scratch.partials;
     *taken = true;
-    e = launch_with_pdl((g.c_n_major ? 6 : 3) + g.out_dtype, plan, p, stream);
+    e = launch_with_pdl((g.c_n_major ? 6 : 3) + g.out_dtype, plan, &p, stream);
     return e == cudaSuccess ? gemm_scratch_done(scratch, stream) : e;
 }
 

@@ -145,17 +145,40 @@ __device__ __forceinline__ uint32_t swz128(int row, int b) {
                                  ((((b >> 4) ^ (row & 7)) << 4) | (b & 15)));
 }
 
-// Arrives at another CTA's barrier. Nothing that this thread wrote through the generic proxy is handed over by it (stages
-// are written by the bulk copies that its own barrier counted, accumulators are ordered by the tcgen05 fences); the
-// cluster-scope release and acquire cost the pair's issuing loop 1100 clocks a stage.
+// A load of one CTA of a pair into its own shared memory that completes on a barrier of either CTA (an address of
+// cluster_map): the one that issues the MMAs waits for the bytes of both where it would wait for its own.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar,
+                                                 uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+        "[%0], [%1, {%2, %3}], [%4], %5;"
+        :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(cluster_bar), "l"(policy) : "memory");
+}
+
+// Hands tensor memory back to the issuing thread of another CTA: arrival at its barrier, and the wait that belongs to it. The
+// reads are ordered by tcgen05.fence::before_thread_sync ahead of the arrival and ::after_thread_sync behind the wait, which
+// need an order of execution at cluster scope and no more: nothing in memory is handed over. (With release the arrival waits for
+// the results on their way to memory: 10240x5120 with 700 tokens 22.6 us, 21.3 so.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
 }
 
 struct WaitFail {
     bool failed = false;
     __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity) {
         if (!failed && !mbar_wait_bounded(bar, parity, 20000000u)) failed = true;
+        return !failed;
+    }
+    __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {     // for arrivals of another CTA
+        for (uint32_t i = 0; !failed && !mbar_try_wait_cluster(bar, parity); ++i) failed = i >= 20000000u;
         return !failed;
     }
 };

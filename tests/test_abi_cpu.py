@@ -235,3 +235,13 @@ def test_kernels_that_write_operands_let_nothing_in_before_they_end():
     large = code((csrc / "gemm_large.cu").read_text())
     before_wait = large[large.index("int pre = 0;"):]
     assert re.match(r"int pre = 0;\s*if \(!kTma\) \{", before_wait)
+
+
+def test_barriers_between_ctas_name_the_cluster_scope():
+    """An arrival at another CTA's barrier and the wait for it only meet at cluster scope; the default is the CTA."""
+    csrc = REPO / "reset_b200" / "csrc"
+    arrivals = [m for f in csrc.glob("*.cu*") for m in re.findall(r"mbarrier\.arrive[\w.:]*shared::cluster[\w.:]*", f.read_text())
+                if "::one" not in m]
+    assert arrivals and all(re.search(r"\.(relaxed|release)\.cluster\.shared", m) for m in arrivals), arrivals
+    ptx = (csrc / "tcgen05_ptx.cuh").read_text()
+    assert re.search(r"mbarrier\.try_wait\.parity\.(relaxed|acquire)\.cluster\.", ptx)

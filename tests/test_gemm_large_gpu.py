@@ -379,3 +379,33 @@ def test_gemm_directly_behind_the_quantizer_of_its_weight(capi, M, dtype):
         got.append(product())
     for i in range(12):
         assert torch.equal(got[i], want[i % 3]), i
+
+
+@pytest.mark.parametrize("bn", [192, 256])                               # accumulators apart, overlapping
+@pytest.mark.parametrize("row_major", [False, True])
+def test_pairs_hand_stages_and_accumulators_over_in_order(capi, row_major, bn):
+    """Many tiles and ring turns a pair, an odd number of row tiles, two weights in turn: every call gives the bits of the first
+    one with its weight (the sums have one order), and those of the first are within the bound of the exact product."""
+    M, N, K = 1500, 3 * 128 * 31, 2048
+    cases = [_case(M, N, K, seed=s) for s in (1, 5)]
+    _tune(1, bn, 9)
+    x, gs = [c[2].cuda() for c in cases], cases[0][3]
+    if row_major:
+        operands = [(*capi.quant(x[i], gs, swizzled=True), cuda(cases[i][0]), cuda(onv.swizzle_blockscale(cases[i][1]))) for i in (0, 1)]
+        wksp = torch.zeros(1 << 20, dtype=torch.int64, device="cuda")
+
+        def call(i):
+            C = torch.empty((M, N), device="cuda")
+            xc, xsf, w, ws = operands[i]
+            capi.gemm(xc, w, xsf, ws, C, 0.5, wksp, n_major=False)
+            return C
+    else:
+        packed = [capi.pack_weight(cuda(c[0]), cuda(c[1])) for c in cases]
+
+        def call(i):
+            return torch.ops.nvfp4r.linear_packed(x[i], gs, packed[i], N, 0.5, F32, 0)
+    first = [call(0), call(1)]
+    for i in (0, 1):
+        assert rel_l2(first[i].cpu().numpy(), cases[i][4]) <= 1e-5
+    for r in range(30):
+        assert torch.equal(call(r & 1), first[r & 1]), r
