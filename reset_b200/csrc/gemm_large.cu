@@ -897,15 +897,17 @@ bool make_large_plan(int M, int N, int K, bool row_major, int G, LargePlan* plan
     return true;
 }
 
-// A call asks three times (scratch size, its check, launch) and plans once: 0.3 us each.
+// A call asks three times (scratch size, its check, launch) and plans once: 0.3 us each. The device is part of the key: two with
+// as many SMs need not place as many clusters.
 bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
-    struct Last { int M, N, K, G, bn, sk; bool row_major, found; LargePlan plan; };
+    struct Last { int M, N, K, dev, bn, sk; bool row_major, found; LargePlan plan; };
     static thread_local Last last = {};
-    const int G = device_sm_count();
-    if (last.M != M || last.N != N || last.K != K || last.G != G || last.bn != g_large_bn || last.sk != g_large_sk ||
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    if (last.M != M || last.N != N || last.K != K || last.dev != dev || last.bn != g_large_bn || last.sk != g_large_sk ||
         last.row_major != row_major) {
-        last = Last{M, N, K, G, g_large_bn, g_large_sk, row_major, false, {}};
-        last.found = make_large_plan(M, N, K, row_major, G, &last.plan);
+        last = Last{M, N, K, dev, g_large_bn, g_large_sk, row_major, false, {}};
+        last.found = make_large_plan(M, N, K, row_major, device_sm_count(), &last.plan);
     }
     *plan = last.plan;
     return last.found;

@@ -245,3 +245,10 @@ def test_barriers_between_ctas_name_the_cluster_scope():
     assert arrivals and all(re.search(r"\.(relaxed|release)\.cluster\.shared", m) for m in arrivals), arrivals
     ptx = (csrc / "tcgen05_ptx.cuh").read_text()
     assert re.search(r"mbarrier\.try_wait\.parity\.(relaxed|acquire)\.cluster\.", ptx)
+
+
+def test_plans_are_kept_per_device():
+    """A many-token plan depends on how many clusters the device can place, not on its SM count alone."""
+    text = (REPO / "reset_b200" / "csrc" / "gemm_large.cu").read_text()
+    keep = text[text.index("bool plan_large("):]
+    assert re.search(r"last\.dev != dev", keep[:keep.index("\n}\n")])
