@@ -96,7 +96,6 @@ constexpr uint32_t kColSfaL = 416, kColSfbL = 448, kColSfa1 = 464, kColSfb1 = 48
 
 struct alignas(64) LargeParams {
     CUtensorMap map_w, map_x;                        // row-major form: codes; packed form, pairs: weight blocks, token codes
-    CUtensorMap map_xsf;                             // pairs: token scales
     const uint8_t* w;                                // packed weight blocks
     const uint8_t* x;                                // packed token blocks
     const uint8_t* wsf;                              // row-major form: 128x4-tiled scales
@@ -112,10 +111,10 @@ struct alignas(64) LargeParams {
     unsigned* tickets;                               // [tiles], zero before the launch, left zero
 };
 
-struct alignas(64) LargeParamsPairTma : LargeParams {
-    CUtensorMap map_wsf;                             // pairs of the row-major form: weight scales
+struct alignas(64) PairParams : LargeParams {
+    CUtensorMap map_xsf, map_wsf;                    // token scales; row-major form: weight scales
 };
-template <bool kTma, bool kPair> using ParamsOf = std::conditional_t<kTma && kPair, LargeParamsPairTma, LargeParams>;
+template <bool kPair> using ParamsOf = std::conditional_t<kPair, PairParams, LargeParams>;
 
 __device__ int g_large_status = 0;
 
@@ -394,7 +393,7 @@ __device__ __forceinline__ void issue_all(const LargeParams& p, uint32_t ring, u
 
 template <bool kTma, int kDtype, bool kNMajor, bool kPair>
 __global__ void __launch_bounds__(kThreadsL, 2)
-gemm_large_kernel(const __grid_constant__ ParamsOf<kTma, kPair> p) {
+gemm_large_kernel(const __grid_constant__ ParamsOf<kPair> p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     __shared__ __align__(8) uint64_t bars[2 * kMaxStagesL + 4];
@@ -469,29 +468,29 @@ gemm_large_kernel(const __grid_constant__ ParamsOf<kTma, kPair> p) {
         // A pair: all loads of a stage, the peer's too, complete on the issuing CTA's barrier, which expects all of their bytes.
         auto load_a = [&](const Source& o, uint32_t dst, uint32_t bar) {
             const uint32_t bytes = kABytes + b_codes + static_cast<uint32_t>(o.ch) * 2048u;
-            if (kPair) {
+            if constexpr (kPair) {
                 if (rank == 0) mbar_expect_tx(bar, 2 * bytes);
                 const uint32_t there = cluster_map(bar, 0);
-                if constexpr (kTma && kPair) {
+                if (kTma) {
                     tma_load_2d_pair(dst, &p.map_w, o.ax, o.ay, there, policy);
                     tma_load_2d_pair(dst + kACodes, &p.map_wsf, 0, o.ar, there, policy);
                 } else {
                     tma_load_2d_pair(dst, &p.map_w, 0, o.ar, there, policy);
                 }
-                return;
-            }
-            mbar_expect_tx(bar, bytes);
-            if (kTma) {
-                tma_load_2d(dst, &p.map_w, o.ax, o.ay, bar, policy);
-                bulk_g2s(dst + kACodes, o.a, 2048, bar, policy);
             } else {
-                bulk_g2s(dst, o.a, kABytes, bar, policy);
+                mbar_expect_tx(bar, bytes);
+                if (kTma) {
+                    tma_load_2d(dst, &p.map_w, o.ax, o.ay, bar, policy);
+                    bulk_g2s(dst + kACodes, o.a, 2048, bar, policy);
+                } else {
+                    bulk_g2s(dst, o.a, kABytes, bar, policy);
+                }
             }
         };
         auto load_b = [&](const Source& o, uint32_t dst, uint32_t bar) {
-            if (kPair) {
+            if constexpr (kPair) {
                 const uint32_t there = cluster_map(bar, 0);
-                if constexpr (kTma && kPair) {
+                if (kTma) {
                     tma_load_2d_pair(dst, &p.map_x, o.ax, o.by, there, keep);
                     for (int j = 0; j < o.ch; ++j) tma_load_2d_pair(dst + b_codes + j * 2048, &p.map_xsf, 0, o.br + j * (p.k64 / 2), there, keep);
                 } else {
@@ -915,7 +914,7 @@ bool plan_large(int M, int N, int K, bool row_major, LargePlan* plan) {
 
 constexpr int kInstances = 18;
 
-// p: a LargeParamsPairTma where the plan is for pairs and the form row-major.
+// p: PairParams where the plan is for pairs.
 cudaError_t launch_with_pdl(int form, const LargePlan& plan, const LargeParams* p, cudaStream_t stream) {
     // packed operands, then row-major ones with M-major and with N-major output; bf16, fp16, fp32; by one CTA, by a pair
 #define NVFP4R_KERN(...) reinterpret_cast<const void*>(&gemm_large_kernel<__VA_ARGS__>)
@@ -1052,7 +1051,7 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
     LargePlan plan;
     if (!plan_large(g.M, g.N, g.K, false, &plan)) return cudaErrorInvalidConfiguration;
     uint8_t* tokens = static_cast<uint8_t*>(scratch);
-    LargeParams p = {};
+    PairParams p = {};
     fill_common(plan, &p, g.out, g.M, g.N, g.K, g.alpha, false);
     p.w = static_cast<const uint8_t*>(g.packed);
     p.x = tokens;
@@ -1089,7 +1088,7 @@ cudaError_t launch_gemm_large(const TcLinearArgs& g, cudaStream_t stream, bool* 
     LargePlan plan;
     if (g.xb != nullptr || g.M < g_large_min_m || (g.M <= 32 && (tc_tuned() || g.out_dtype == NVFP4R_F32))) return cudaSuccess;
     if (!plan_large(g.M, g.N, g.K, true, &plan)) return cudaSuccess;
-    LargeParamsPairTma p = {};
+    PairParams p = {};
     fill_common(plan, &p, g.out, g.M, g.N, g.K, g.alpha, g.c_n_major);
     if (!code_map(g.w, g.N, g.K, kRows, &p.map_w) || !code_map(g.a_codes, g.M, g.K, plan.pair ? plan.bn / 2 : plan.bn, &p.map_x)) return cudaSuccess;
     if (plan.pair && (!row_map(g.wsf_swizzled, static_cast<int64_t>(g.N / kRows) * p.k64 / 2, 2, &p.map_wsf) ||
