@@ -514,7 +514,9 @@ gemm_large_kernel(const __grid_constant__ ParamsOf<kPair> p) {
         };
         // A packed weight does not depend on the kernel before: the weight half of the first stages is requested ahead of the
         // wait, the token half behind it. The raw operator's weight may be that kernel's output, and what it wrote is only
-        // sure to be visible behind the wait, also where it let this one in at its end. Behind a quantizer it costs nothing.
+        // sure to be visible behind the wait, also where it let this one in at its end. Device us in a CUDA graph, asked for
+        // ahead of the wait / behind it: quant + gemm 4096x12288 128 tokens 14.6 / 14.0, 4096x4096 1 token 8.87 / 8.67;
+        // gemm behind gemm 4864x7168 1 token 8.2 / 8.3, 32 tokens 8.0 / 7.8, 1920x11264 1 token 7.5 / 8.1.
         int pre = 0;
         if (!kTma) {
             Walker wa(p, kPair);
@@ -996,11 +998,13 @@ void fill_common(const LargePlan& plan, LargeParams* p, void* out, int M, int N,
 // choice. Up to 16 tokens the decode kernel makes one pass over the weight as well and needs no second launch; its
 // CTAs each quantize the tokens of their K part, which grows with the tokens, while this path pays a few us for
 // partial sums where the weight has few row tiles and long rows. Measured in CUDA graphs, us, decode kernel / this one:
-//   N >= 6 K       34816x5120: 13 tokens 25.6 / 21.3, 16 tokens 26.4 / 21.5; 12288x2048: 13 tokens 8.2 / 6.4;
-//                  but (N >= 16 K) 24576x1024: 13 tokens 6.1 / 6.8, 17 tokens 8.1 / 6.9
-//   N >= 1.5 K     12288x4096: 17 tokens 15.3 / 10.5; 10240x5120: 17 tokens 15.9 / 11.6; 6144x4096: 17 tokens 10.0 / 9.7
-//   N >= K         4096x4096: 25 tokens 9.9 / 9.4, 32 tokens 11.3 / 9.5
-//   below          4096x12288: 24 tokens 13.2 / 15.7, 32 tokens 15.7 / 15.7; 1280x5120: 32 tokens 9.6 / 11.2
+//   N >= 6 K       34816x5120: 13 tokens 23.1 / 19.4, 16 tokens 25.7 / 19.3; 12288x2048: 13 tokens 8.2 / 5.9;
+//                  but (N >= 16 K) 24576x1024: 13 tokens 6.2 / 6.9, 17 tokens 8.2 / 6.9
+//   N >= 1.5 K     12288x4096: 17 tokens 15.6 / 9.4; 10240x5120: 17 tokens 16.3 / 9.7; 6144x4096: 17 tokens 10.3 / 7.4
+//   N >= K         4096x4096: 25 tokens 10.2 / 7.0, 32 tokens 11.6 / 7.1
+//   below          4096x12288: 17 tokens 12.2 / 10.3, 24 tokens 13.5 / 10.3, 32 tokens 16.2 / 10.3; 1280x5120: 32 tokens 9.9 / 6.9
+// The last two lines were drawn before clusters shared a tile (4096x12288, 24 tokens, 15.7 here) and are kept with the answers
+// of the query: this kernel gains on its own side of them.
 int large_min_m(int N, int K) {
     const int64_t n = N, k = K;
     return n >= 6 * k && n < 16 * k ? 13 : 2 * n >= 3 * k ? 17 : n >= k ? 25 : 33;
@@ -1017,14 +1021,14 @@ bool large_pays(int M, int N, int K) {
     const int G = device_sm_count(), tiles = N / kRows, kblocks = (K + kBK - 1) / kBK;
     // A narrow weight with rows of 31 or 32 K blocks: the longest that ran as whole tiles here before clusters shared
     // them (0.48 us a block), while two launches of the decode kernel give each CTA one block and one token to add up. 33 / 48 / 64
-    // tokens: 640x8192 13.0 / 14.0 / 14.3, here 15.5 / 15.7 / 15.9; 1280x8192 14.3 / 15.5 / 18.6, here 16.0 / 15.9 / 16.2;
-    // 30 blocks, 1024x7680: 14.9 / 16.0 / 17.4, here 14.8 / 14.8 / 15.0; 33, 1792x8320: 17.2 / 18.4 / 22.4, here 16.8.
-    // (With clusters 640x8192 takes 7.7 / 7.8 / 8.2 here. The line stays where callers of the query found it.)
+    // tokens then: 640x8192 13.0 / 14.0 / 14.3, here 15.5 / 15.7 / 15.9; 1280x8192 14.3 / 15.5 / 18.6, here 16.0 / 15.9 / 16.2.
+    // With clusters 640x8192 takes 7.7 / 7.7 / 8.0 here, 1280x8192 8.2 / 8.2 / 8.1 (and beside the line 1024x7680 33 tokens
+    // 14.8 there, 7.8 here, 1792x8320 17.2 and 8.3): the line stays where callers of the query found it.
     if (M <= 64 && kblocks > 30 && kblocks <= 32 && tiles <= (M <= 48 ? 16 : 8)) return false;
     // Up to 16 tokens both kernels are bound by the weight, and here 1 to 1.5 tiles per SM cost two rounds. The line was
     // drawn when a K block took 0.48 us here (24576x4096, 16 tokens 17.4 / 18.5; 20480x2048 9.8 / 10.8; but 24064x2304, where
-    // the decode kernel splits K, 15.3 / 11.5) and is kept with the answers of the query; at 0.24 us a block this kernel
-    // gains on its own side of it: 24576x4096, 16 tokens 18.7 / 14.6, 13 tokens 16.8 / 14.7; 24576x2048 10.6 / 9.9.
+    // the decode kernel splits K, now 14.8 / 9.9) and is kept with the answers of the query; at 0.24 us a block this kernel
+    // gains on its own side of it: 24576x4096, 16 tokens 17.8 / 14.0, 13 tokens 16.2 / 14.0; 24576x2048 10.3 / 9.5; 20480x2048 9.6 / 9.2.
     if (M <= 16 && tiles > G && 2 * tiles < 3 * G) return packed_time_us(M, N, K) > 3.9 + 0.96 * kblocks;
     return true;
 }
@@ -1078,8 +1082,8 @@ cudaError_t launch_linear_large(const PackedLinearArgs& g, void* scratch, cudaSt
 
 // The raw operator on row-major operands, any number of tokens. The decode-sized kernel keeps the tokens of a K part in
 // shared memory and asks for the weight in one 16 KB tensor-map request a stage from a single lane; fp16 N-major output,
-// device us, that kernel / this one: 4864x7168 1 token 21.1 / 7.7, 32 tokens 47.4 / 7.9; 4096x4096 1 token 13.7 / 5.9;
-// 640x1024 1 token 6.1 / 3.3; 1920x11264 1 token 10.6 / 7.2. With fp32 output it stays up to 32 tokens: there
+// device us, that kernel / this one: 4864x7168 1 token 21.1 / 8.3, 32 tokens 47.4 / 7.8; 4096x4096 1 token 13.7 / 6.8;
+// 640x1024 1 token 6.1 / 4.4; 1920x11264 1 token 10.6 / 8.1. With fp32 output it stays up to 32 tokens: there
 // nvfp4r_linear_tc, which quantizes the tokens itself, is bound to give the same bits.
 // *taken stays false (nothing launched) where the workspace does not hold what this path needs or a tensor map cannot be
 // made: the caller's other kernel runs.

@@ -21,16 +21,13 @@
 // to reach the goal.
 //
 // Bound: latency (barriers and dependent passes over shared memory); the traffic is 0.6 MB per row.
-// Measured against 11 to 17 launches over a scratch in device memory, 151936 entries, us a call, before -> after:
-//   top-k 20 top-p 0.95   1 row 57.7 -> 7.4    8 rows 70.9 -> 8.4    32 rows 133 -> 10.1   256 rows 956 -> 90
-//   top-p 0.9             1 row 38.3 -> 35.3   8 rows 49.5 -> 41.4   32 rows 105 -> 55.4   256 rows 700 -> 410
-//   top-k 1000            1 row 37.1 -> 24.1   8 rows 45.1 -> 26.1   32 rows 96 -> 34.8    256 rows 657 -> 268
-// and with phase 3, the masses in 32-bit halves and the draw's logarithms only where they can matter, device us in a CUDA
-// graph with the counters' reset, radix descent -> steps:
-//   top-p 0.9   1 row 31.6 -> 19.2   8 rows 39.4 -> 26.8   32 rows 53.8 -> 38.8     top-k 1000, 8 rows 27.9 -> 22.4
+// Measured, 151936 entries. Top-k 20 top-p 0.95, us a call, 11 to 17 launches over a scratch in device memory -> one launch
+// (and that without phase 2): 1 row 57.7 -> 7.4 (35.1), 8 rows 70.9 -> 8.4 (37.6), 32 rows 133 -> 10.1 (47.2), 256 rows
+// 956 -> 90 (373). Larger sets, device us in a CUDA graph with the counters' reset, radix descent alone -> phase 3, the masses in
+// 32-bit halves and the draw's logarithms only where they can matter:
+//   top-p 0.9   1 row 31.6 -> 19.1   8 rows 39.4 -> 26.7   32 rows 53.8 -> 38.7     top-k 1000, 8 rows 27.9 -> 22.4
 //   top-k 150 top-p 0.8, 8 rows 40.2 -> 28.6
 // of which, 8 rows in clusters of eight, thousand clocks: load 5, histogram 11, its bin 6, list 5, pairs 3, draw 13.
-// (the first line without phase 2: 35.1, 37.6, 47.2, 373)
 //
 //   * 8 CTAs of 512 threads (16 for a few rows of top-p alone, where the device can place them): the largest cluster every
 //     device can place, and at 151936 entries two CTAs
